@@ -377,7 +377,7 @@ int32_t przmg_package_literals_batch(przmg_ctx* ctx, uint64_t d_in, const uint64
  * or a stream that must not meet the device-wide synchronisation of
  * cudaFree).  It allocates nothing: no cudaMalloc/cudaFree, no host staging
  * copy, no context; all scratch is one file-scope __device__ array of about
- * 2.3 MiB per device, so n is limited to PRZMG_NOALLOC_MAX_N symbols.
+ * 2.7 MiB per device, so n is limited to PRZMG_NOALLOC_MAX_N symbols.
  *   n > PRZMG_NOALLOC_MAX_N           -> PRZMG_ERR_EXCEEDS_MAX_BLOCK
  *   out_cap < 1024 + 2 * n            -> PRZMG_ERR_BUFFER_TOO_SMALL
  *   unknown norm, null address, or

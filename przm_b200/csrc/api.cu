@@ -156,6 +156,8 @@ struct przmg_batch {
     DevBuf d_asm_job;     // the same items grouped by input (plain per-input launches)
     DevBuf d_s3, d_s3f;   // P2 and up: per-input Section 3 regions and their S3Frame facts
     DevBuf d_fib;         // P3: per-input fiber regions
+    DevBuf d_seg;         // segments of the long rANS tasks
+    uint32_t seg_cap = 0, seg_cap_m8 = 0;  // segments at most, of Meta8 tasks at most
     // P2 and up: the Mode 12 chains run on a second stream, forked after the
     // distance codes exist and joined before the plan (graph capture keeps
     // the two branches)
@@ -197,7 +199,7 @@ struct przmg_batch {
                          &d_job_lens, &d_hist, &d_tabs, &d_infos, &d_ans, &d_outs, &d_plans, &d_sizes, &d_out, &d_misc,
                          &d_lists, &d_rtiles, &d_rx_toff, &d_rx_list, &d_rx_pred, &d_stage_in,
                          &d_stage_out, &d_stage_offs, &d_up_offs, &d_tile_sched, &d_asm, &d_asm_job,
-                         &d_fitems, &d_ftiles, &d_ftarget, &d_fctl, &d_s3, &d_s3f, &d_fib};
+                         &d_fitems, &d_ftiles, &d_ftarget, &d_fctl, &d_s3, &d_s3f, &d_fib, &d_seg};
         for (DevBuf* b : all) b->release();
         h_offs.release();
     }
@@ -235,7 +237,7 @@ struct Ctx {
     DevBuf d_dist12;  // Mode 12 static weights in EncSym form (4 x 64)
     przmg_batch single;  // reused by the one-input calls
     HostBuf h_in, h_out, h_aux;
-    DevBuf d_scr_in, d_scr_out, d_scr_aux, d_scr_tab;
+    DevBuf d_scr_in, d_scr_out, d_scr_aux, d_scr_tab, d_scr_seg;
     DevBuf d_s3;   // scratch of przmg_package_offsets_batch
     DevBuf d_lit;  // scratch of przmg_package_literals_batch
     // the GPU decoder: static tables, per-frame scratch, jobs, results,
@@ -308,7 +310,7 @@ static int32_t batch_prepare(przmg_batch* b, const uint64_t* sizes, uint32_t njo
     b->max_big_cand = 0;
     b->in_offs.assign(njobs, 0);
     b->out_offs.assign(njobs, 0);
-    uint64_t in = 0, desc = 0, str = 0, ans = 0, out = 0, s3 = 0, fib = 0;
+    uint64_t in = 0, desc = 0, str = 0, ans = 0, out = 0, s3 = 0, fib = 0, segb = 0, segb_m8 = 0;
     uint32_t tile0 = 0;
     for (auto* v : {&b->job_small0, &b->job_rt0, &b->job_big0, &b->job_tile0, &b->job_asm0}) v->assign(njobs + 1, 0);
     for (uint32_t i = 0; i < njobs; i++) {
@@ -345,7 +347,13 @@ static int32_t batch_prepare(przmg_batch* b, const uint64_t* sizes, uint32_t njo
             fib += align16(fib_region_bytes(j));
         }
         j.ans_off = ans;
-        if (profile >= 1) ans += align16(ans_region_bytes(j));
+        if (profile >= 1) {
+            ans += align16(ans_region_bytes(j));
+            // literals, op / meta / var twice, distance codes, fibers of four foliations
+            const uint64_t cmds = 3 * seg_bound(std::min<uint64_t>(j.cmd_cap, n));
+            segb += (profile >= 3 ? 5 : 1) * seg_bound(n) + 2 * cmds + (profile >= 2 ? seg_bound(j.dist_cap) : 0);
+            segb_m8 += cmds;
+        }
         j.out_cap = (uint32_t)std::min<uint64_t>(przmg_frame_bound(n), 0xFFFFFFF0u);
         j.out_off = out;
         b->out_offs[i] = out;
@@ -436,7 +444,10 @@ static int32_t batch_prepare(przmg_batch* b, const uint64_t* sizes, uint32_t njo
     CK(b->d_sizes.ensure((size_t)njobs * 4 + 16));
     CK(b->d_out.ensure(b->out_bytes));
     CK(b->d_misc.ensure(64));
-    CK(b->d_lists.ensure((size_t)2 * kModels * std::max<uint32_t>(njobs, 1) * sizeof(TaskDesc) + 64));
+    b->seg_cap = seg_cap(segb);
+    b->seg_cap_m8 = std::min(seg_cap(segb_m8), b->seg_cap);
+    CK(b->d_lists.ensure((size_t)2 * (kModels * std::max<uint32_t>(njobs, 1) + b->seg_cap) * sizeof(TaskDesc) + 64));
+    CK(b->d_seg.ensure(seg_bytes(b->seg_cap)));
     CK(b->d_up_offs.ensure(8ull * std::max<uint32_t>(njobs, 1) + 64));
     if (b->nbig) {
         CK(b->d_rtiles.ensure(sizeof(RxTile) * std::max<size_t>(b->rtiles.size(), 1)));
@@ -527,6 +538,23 @@ static Range job_range(const przmg_batch* b, uint32_t i) {
     r.maxtiles = std::max<uint32_t>(1, b->jobs[i].ntiles);
     r.max_big_cand = rx_ncand(b->jobs[i].n);
     return r;
+}
+
+// The rANS launches of a task list: the walk and the resolution of its
+// segments (none without segment scratch), the coding, the segments' sums.
+// nb_ad, nb_m8: blocks that hold every adaptive and every Meta8 task;
+// m8_segs: Meta8 tasks may be split.
+static cudaError_t launch_rans(const SegBufs& sb, const TaskDesc* lists, uint32_t list_cap, const uint32_t* counts,
+                               uint32_t nb_ad, uint32_t nb_m8, const EncSym* tabs, const EncSym* meta8,
+                               const uint8_t* ctxlut, TaskOut* outs, cudaStream_t s, bool m8_segs = false) {
+    if (sb.cap) {
+        k_seg_walk<false><<<sb.cap, kWalkThreads, kWalkSmemAd, s>>>(sb, tabs, meta8, ctxlut);
+        if (m8_segs) k_seg_walk<true><<<sb.cap, kWalkThreads, kWalkSmemM8, s>>>(sb, tabs, meta8, ctxlut);
+        k_seg_resolve<<<sb.cap / 2, 128, 0, s>>>(sb, tabs, meta8, ctxlut);
+    }
+    k_rans<<<nb_ad + nb_m8, kRansWarps * 32, kRansSmem, s>>>(lists, list_cap, counts, nb_ad, tabs, meta8, ctxlut, outs, sb);
+    if (sb.cap) k_seg_sums<<<sb.cap / 2, 128, 0, s>>>(sb, outs);
+    return cudaGetLastError();
 }
 
 // ev (optional): kStages + 1 events; ev[0] before the first kernel and
@@ -660,21 +688,20 @@ static int32_t launch_range(przmg_batch* b, cudaStream_t s, int stop_after, cons
                                                       b->d_infos.as<TableInfo>());
             CK(cudaGetLastError());
             CK(mark(6));
-            const uint32_t list_cap = kModels * b->njobs;
+            const uint32_t list_cap = kModels * b->njobs + b->seg_cap;
+            const SegBufs sb = seg_bufs(b->d_seg.p, b->seg_cap, b == &c->single ? 1u : 3u);
             TaskDesc* lists = b->d_lists.as<TaskDesc>();
             uint32_t* counts = reinterpret_cast<uint32_t*>(lists + 2 * list_cap);
             k_task_list<<<1, 1024, 0, s>>>(b->d_jobs.as<Job>(), R.j0, R.nj, b->d_job_lens.as<uint32_t>(),
                                            b->d_s3f.as<S3Frame>(), b->d_streams.as<uint8_t>(), b->d_s3.as<uint8_t>(),
-                                           b->d_fib.as<uint8_t>(), b->d_ans.as<uint8_t>(), lists, list_cap, counts);
+                                           b->d_fib.as<uint8_t>(), b->d_ans.as<uint8_t>(), lists, list_cap, counts, sb);
             CK(cudaGetLastError());
             const uint32_t nad = (b->profile >= 3 ? kModels : b->profile >= 2 ? 5 : 4) * R.nj;  // adaptive tasks at most
-            const uint32_t nb_ad = (nad + 8 * kRansWarps - 1) / (8 * kRansWarps);
-            const uint32_t nb_m8 = (3 * R.nj + 8 * kRansWarps - 1) / (8 * kRansWarps);
-            k_rans<<<nb_ad + nb_m8, kRansWarps * 32, kRansSmem, s>>>(lists, list_cap, counts, nb_ad,
-                                                                    b->d_tabs.as<EncSym>(), c->d_meta8.as<EncSym>(),
-                                                                    c->d_ctxlut.as<uint8_t>(), b->d_outs.as<TaskOut>());
-            CK(cudaGetLastError());
-            launches += 3;
+            const uint32_t nb_ad = (nad + b->seg_cap + 8 * kRansWarps - 1) / (8 * kRansWarps);
+            const uint32_t nb_m8 = (3 * R.nj + b->seg_cap_m8 + 8 * kRansWarps - 1) / (8 * kRansWarps);
+            CK(launch_rans(sb, lists, list_cap, counts, nb_ad, nb_m8, b->d_tabs.as<EncSym>(), c->d_meta8.as<EncSym>(),
+                           c->d_ctxlut.as<uint8_t>(), b->d_outs.as<TaskOut>(), s, b->seg_cap_m8 != 0));
+            launches += 3 + (sb.cap ? 3 + (b->seg_cap_m8 != 0) : 0);
             if (b->profile >= 2) CK(cudaStreamWaitEvent(s, b->ev_join, 0));  // the Mode 12 chains
             CK(mark(7));
         } else {
@@ -774,7 +801,6 @@ static int32_t ctx_setup(Ctx* c) {
     CK(cudaFuncSetAttribute(k_rans, cudaFuncAttributeMaxDynamicSharedMemorySize, kRansSmem));
     CK(cudaFuncSetAttribute(k_front, cudaFuncAttributeMaxDynamicSharedMemorySize, kFrontSmem));
     CK(cudaDeviceGetAttribute(&c->clock_khz, cudaDevAttrClockRate, c->device));
-    CK(cudaFuncSetAttribute(k_stream_rans, cudaFuncAttributeMaxDynamicSharedMemorySize, kRansSmem));
     CK(c->d_meta8.ensure(8 * 256 * sizeof(EncSym)));
     CK(c->d_ctxlut.ensure(256));
     {
@@ -822,7 +848,7 @@ extern "C" int32_t przmg_close(przmg_ctx* h) {
         c->single.drop_graph();
         c->single.release();
         DevBuf* bufs[] = {&c->d_meta8, &c->d_ctxlut, &c->d_dist12, &c->d_scr_in, &c->d_scr_out, &c->d_scr_aux,
-                          &c->d_scr_tab, &c->d_s3, &c->d_lit, &c->d_dstatic, &c->d_dscr, &c->d_djobs,
+                          &c->d_scr_tab, &c->d_scr_seg, &c->d_s3, &c->d_lit, &c->d_dstatic, &c->d_dscr, &c->d_djobs,
                           &c->d_dinfo, &c->d_dtasks, &c->d_dout, &c->d_ddiff};
         for (DevBuf* b : bufs) b->release();
         c->h_in.release();

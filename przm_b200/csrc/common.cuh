@@ -219,14 +219,14 @@ __host__ __device__ inline FibGeom fib_geom(const Job& j, const uint32_t* fl, ui
 }
 
 // Encoding table entry for one symbol of one model:
-//   m   : 32-bit reciprocal so that floor(x_r / f) == umulhi(x_r, m) >> s for
-//         every x_r < 2^24 (Granlund-Montgomery 1994, round-up variant);
-//         f = 2^t uses m = 2^(32-t), s = 0; f = 1 uses m = 2^32-1 (one short)
-//         with the deficit folded into cb.
+//   m   : 32-bit reciprocal so that floor(x / f) == umulhi(x, m) >> s for
+//         every x < 2^31 (Granlund-Montgomery 1994, round-up variant);
+//         f = 2^t uses m = 2^(32-t), s = 0; f = 1 uses m = 2^31, s = -1 mod
+//         32 (a state always gives off a byte then, so the total shift below
+//         is positive).
 //   t1  : 4096 * f, the renormalisation bound (x >= t1 -> emit a byte)
 //   t2  : 256 * t1 saturated to 2^32-1 (x >= t2 -> emit a second byte)
-//   w   : cb | (4096 - f) << 13 | s << 25, cb = cumulative frequency c
-//         (+4095 when f == 1)
+//   w   : c | (4096 - f) << 13 | s << 25, c = cumulative frequency
 struct __align__(16) EncSym {
     uint32_t m, t1, t2, w;
 };

@@ -136,14 +136,14 @@ __global__ void __launch_bounds__(kS3Threads) k_s3_frame(const Job* __restrict__
 // reference would write (low byte first) into em[e..] and advances x.
 // False when they would pass the reference's 2 MiB emission scratch.
 __device__ __forceinline__ bool m12_step(uint32_t& x, uint32_t& e, const EncSym& es, uint8_t* __restrict__ em) {
-    const uint32_t k = (uint32_t)(x >= es.t1) + (uint32_t)(x >= es.t2);
+    const uint32_t k = rans_shift(x, es);
     if (k) {
-        if (e + k > kS3Scratch) return false;
+        if (e + (k >> 3) > kS3Scratch) return false;
         em[e] = (uint8_t)x;
-        if (k == 2) em[e + 1] = (uint8_t)(x >> 8);
-        e += k;
+        if (k == 16) em[e + 1] = (uint8_t)(x >> 8);
+        e += k >> 3;
     }
-    x = rans_next(x, es);
+    x = rans_after(x, es, k);
     return true;
 }
 

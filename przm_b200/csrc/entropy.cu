@@ -7,25 +7,23 @@ namespace pz {
 
 // ---------------------------------------------------------------------------
 // Encoding tables.  The step x' = x + bias + floor(x / f) * (M - f) with the
-// quotient from a multiply-high by a per-symbol reciprocal, and the f = 1
-// case done as a one-short reciprocal with the deficit moved into the bias,
-// is the reciprocal-encoder form of rANS that F. Giesen published with
-// ryg_rans (rans_byte.h, RansEncSymbolInit / RansEncPutSymbol, 2014); the
-// reciprocal itself is Granlund-Montgomery's (PLDI 1994).
+// quotient from a multiply-high by a per-symbol reciprocal is the
+// reciprocal-encoder form of rANS that F. Giesen published with ryg_rans
+// (rans_byte.h, RansEncSymbolInit / RansEncPutSymbol, 2014); the reciprocal
+// itself is Granlund-Montgomery's (PLDI 1994).
 // ---------------------------------------------------------------------------
 __host__ __device__ inline EncSym make_encsym(uint32_t f, uint32_t c) {
     EncSym e;
     if (f == 0) { e.m = 0; e.t1 = 0xFFFFFFFFu; e.t2 = 0xFFFFFFFFu; e.w = 0; return e; }
     uint32_t s = 0;
     while ((2u << s) <= f) s++;  // floor(log2 f)
-    uint32_t cb = c;
-    if (f == 1) { e.m = 0xFFFFFFFFu; s = 0; cb = c + 4095; }
+    if (f == 1) { e.m = 1u << 31; s = 31; }
     else if ((f & (f - 1)) == 0) { e.m = 1u << (32 - s); s = 0; }
     else e.m = (uint32_t)(((1ull << (32 + s)) + f - 1) / f);
     e.t1 = 4096u * f;
     const uint64_t t2 = 256ull * e.t1;
     e.t2 = t2 > 0xFFFFFFFFull ? 0xFFFFFFFFu : (uint32_t)t2;
-    e.w = cb | ((4096u - f) << 13) | (s << 25);
+    e.w = c | ((4096u - f) << 13) | (s << 25);
     return e;
 }
 
@@ -370,16 +368,19 @@ __device__ __forceinline__ LaneIO lane_io(uint8_t* task_base, uint32_t cap, uint
 // again when x >= 2^20 f), and advances x.  The caller keeps the low 16 bits
 // of x from before the step; its first k bytes (low byte first) are what the
 // reference writes.  x < 2^24 throughout, so x >= t2 can only hold for f < 16.
-// The renormalised state is selected first and divided once: computing the
-// three candidates (0, 1 or 2 bytes shifted out) side by side and selecting
-// last keeps the compares off the multiply's chain, but its extra
-// instructions made the kernel slower (7.68 vs 7.45 ms on the 256 x 1 MiB
-// mixed batch).
-__device__ __forceinline__ uint32_t rans_next(uint32_t x, const EncSym& e) {
-    const uint32_t s = e.w >> 25, cf = (e.w >> 13) & 0xFFFu, cb = e.w & 0x1FFFu;
-    const uint32_t xs = x >= e.t2 ? (x >> 16) : (x >= e.t1 ? (x >> 8) : x);
-    return xs + cb + (__umulhi(xs, e.m) >> s) * cf;
+// The quotient of the renormalised state x >> k is that of x shifted k
+// further (floor(floor(x / f) / 2^k) = floor((x >> k) / f)), so the multiply
+// runs beside the compares that give k instead of after them: 36 cycles a
+// round in a one-warp loop over staged entries, against 45 with the state
+// renormalised first and 38 with the three candidates computed side by side.
+__device__ __forceinline__ uint32_t rans_shift(uint32_t x, const EncSym& e) {
+    return x >= e.t2 ? 16u : (x >= e.t1 ? 8u : 0u);
 }
+__device__ __forceinline__ uint32_t rans_after(uint32_t x, const EncSym& e, uint32_t k) {
+    const uint32_t s = e.w >> 25, cf = (e.w >> 13) & 0xFFFu, c = e.w & 0x1FFFu;
+    return (x >> k) + c + __funnelshift_r(__umulhi(x, e.m), 0u, s + k) * cf;
+}
+__device__ __forceinline__ uint32_t rans_next(uint32_t x, const EncSym& e) { return rans_after(x, e, rans_shift(x, e)); }
 __device__ __forceinline__ uint32_t rans_step(uint32_t& x, const EncSym& e) {
     const uint32_t k = (uint32_t)(x >= e.t1) + (uint32_t)(x >= e.t2);
     x = rans_next(x, e);
@@ -461,17 +462,22 @@ __device__ __forceinline__ void ring_read(const uint4* ring, uint32_t t, int32_t
 // are requested (cp.async, no register waits on them) while group g is
 // encoded, the words of group g - 1 are read from the ring one group ahead,
 // and the 16 table entries of group g are fetched before its chain runs.
+// Rounds [lo, hi) only (lo and hi multiples of 16, or hi == kToTop: up to the
+// lane's last round), from state x; io.cum then counts this segment's bytes.
+constexpr uint32_t kToTop = 0xFFFFFFFFu;
 template <bool kMeta8>
-__device__ __forceinline__ void rans_lane(const uint8_t* __restrict__ src, uint32_t n, uint32_t l,
-                                          const EncSym* __restrict__ tab, const uint8_t* __restrict__ ctxlut,
-                                          uint4* ring, LaneIO io, uint32_t* out_state, uint32_t* out_count) {
-    uint32_t x = 65536, cnt = 0;
+__device__ __forceinline__ void rans_lane(const uint8_t* __restrict__ src, uint32_t n, uint32_t l, uint32_t lo,
+                                          uint32_t hi, uint32_t x, const EncSym* __restrict__ tab,
+                                          const uint8_t* __restrict__ ctxlut, uint4* ring, LaneIO io,
+                                          uint32_t* out_state, uint32_t* out_count) {
+    uint32_t cnt = 0;
     uint16_t* raw = reinterpret_cast<uint16_t*>(io.bytes);
     const uint32_t t = threadIdx.x & 31;
     if (n > l) {
-        const uint32_t J = (n - 1 - l) >> 2;
+        const uint32_t J = hi == kToTop ? (n - 1 - l) >> 2 : hi - 1;
         const bool vec = (reinterpret_cast<uintptr_t>(src) & 15) == 0;
-        const int32_t G = vec ? (int32_t)(n >> 6) : 0;
+        const int32_t g0 = (int32_t)(lo >> 4);
+        const int32_t G = vec ? (int32_t)min(n >> 6, hi >> 4) : g0;
         {
             uint32_t acc = 0;
             for (int32_t j = (int32_t)J; j >= 16 * G; j--) {
@@ -489,7 +495,7 @@ __device__ __forceinline__ void rans_lane(const uint8_t* __restrict__ src, uint3
                 if ((j & (kStitchRounds - 1)) == 0) io.cum[j / kStitchRounds] = cnt;
             }
         }
-        if (G > 0) {
+        if (G > g0) {
             const uint4* s4 = reinterpret_cast<const uint4*>(src);
             uint4* r4 = reinterpret_cast<uint4*>(raw);
             const uint32_t sel = 0x4440u | l;               // __byte_perm selector of byte l
@@ -500,7 +506,7 @@ __device__ __forceinline__ void rans_lane(const uint8_t* __restrict__ src, uint3
             ring_wait<kRing - 1>();
             uint4 cur[4];
             ring_read(ring, t, G - 1, cur);
-            for (int32_t g = G - 1; g >= 0; g--) {
+            for (int32_t g = G - 1; g >= g0; g--) {
                 ring_wait<kRing - 2>();  // group g - 1 has landed
                 uint4 nxt[4];
                 ring_read(ring, t, g - 1, nxt);
@@ -600,41 +606,173 @@ __device__ __forceinline__ uint32_t task_model(int t) {
     return t == T_LIT ? 0u : t == T_S3 ? 4u : t >= T_FIB ? (uint32_t)(kFibModel + t - T_FIB) : 1u + (uint32_t)(t - 1) / 2;
 }
 
-// One rANS task as the rANS kernel takes it, resolved by the task list.
+// One rANS task, or one segment of its rounds, as the rANS kernel takes it.
 struct __align__(16) TaskDesc {
     const uint8_t* src;  // the symbols
     uint8_t* base;       // the task's rANS scratch
     uint32_t n, cap;     // symbols; the scratch layout's capacity
-    uint32_t out;        // TaskOut index: frame * T_COUNT + task
-    uint32_t tab;        // adaptive model row: frame * kModels + model
+    uint32_t out;        // TaskOut index
+    uint32_t tab;        // adaptive model row
+    uint32_t lo, hi;     // rounds [lo, hi), hi == kToTop: up to the stream's last
+    uint32_t seg;        // segment index, kNoSeg: a whole task
+    uint32_t m8;         // 1: Meta8 model
 };
+constexpr uint32_t kNoSeg = 0xFFFFFFFFu;
 
-// Task list: every active (frame, task) pair, split by model kind and
-// ordered longest-first (by the bit length of the symbol count) so that the
-// 8 tasks sharing a warp have similar lengths and the long chains start
-// first; each entry is the task's resolved descriptor.  One block.
-__global__ void __launch_bounds__(1024) k_task_list(const Job* __restrict__ jobs, uint32_t j0, uint32_t njobs,
-                                                    const uint32_t* __restrict__ job_lens,
-                                                    const S3Frame* __restrict__ s3f, const uint8_t* __restrict__ streams,
-                                                    const uint8_t* __restrict__ s3base, const uint8_t* __restrict__ fibbase,
-                                                    uint8_t* __restrict__ ans, TaskDesc* __restrict__ lists,
-                                                    uint32_t list_cap, uint32_t* __restrict__ counts) {
+// Long tasks are coded as independent segments of rounds.  A lane is one
+// chain of states (x' needs x), but the step with a given symbol is a map of
+// [2^16, 2^24) that keeps the cyclic order of the states, and states that
+// leave the same quotient after renormalisation stay together from then on:
+// walkers started anywhere soon fall onto a few trajectories (of 32 spread
+// over the range about 16 are left after 1000 rounds, 8 after 4000), and the
+// true state falls onto one of them.  So
+//   k_seg_walk     32 states walk the kWarm rounds above a segment and then
+//                  the segment itself; their states at kMarks rounds of the
+//                  segment are kept;
+//   k_seg_resolve  goes through a task's segments from the first coded one
+//                  down: the segment's true first state is looked up among
+//                  the walkers' states there, and that walker's last state is
+//                  the next segment's true first state (equal states, equal
+//                  symbols: the walk is the chain).  A state that is not
+//                  among them (0.2 % of the segments of text, 1.4 % of those
+//                  of uniform bytes) walks on until it is;
+//   k_rans         codes every segment from its true first state;
+//   k_seg_sums     adds the byte counts of the segments above.
+// The bytes are those of one chain from end to end.
+constexpr uint32_t kWalkers = 32;
+constexpr uint32_t kWarm = 4096;     // rounds walked above a segment
+constexpr uint32_t kSegMin = 2048;   // shortest segment, in rounds
+constexpr int kSegSizes = 24;        // lengths: 2048, 3072, 4096, 6144, 8192, ...
+__host__ __device__ constexpr uint32_t seg_len(int i) { return ((i & 1) ? 3 * kSegMin / 2 : kSegMin) << (i >> 1); }
+constexpr uint32_t kMarks = 8;       // 0: the segment's first round; m: 256 << m rounds in; the last: its end
+constexpr uint32_t kSegMax = 1776;   // segments of one call at most: 12 blocks of the walk per SM
+
+struct SplitTask {
+    TaskDesc d;
+    uint32_t seg0, nseg, len, pos;  // pos: of its segments in the task list
+};
+// Device scratch of a call's segments; cap 0: tasks are not split.
+struct SegBufs {
+    uint32_t* ctl;     // [0] split tasks, [1] segments
+    TaskDesc* segs;    // [cap]
+    SplitTask* splits; // [cap / 2]
+    uint32_t* first;   // [cap][4] true first states
+    uint32_t* bytes;   // [cap][4] bytes emitted
+    uint32_t* marks;   // [cap][kMarks][4][kWalkers]
+    uint32_t cap;
+    uint32_t weight;   // of the GPU's time against the call's latency (see cut_cost)
+};
+__host__ __device__ constexpr uint64_t seg_bytes(uint32_t cap) {
+    return 256 + (uint64_t)cap * (sizeof(TaskDesc) + sizeof(SplitTask) / 2 + 16 + 16 + kMarks * 4 * kWalkers * 4) + 64;
+}
+__host__ __device__ inline SegBufs seg_bufs(void* base, uint32_t cap, uint32_t weight = 1) {
+    SegBufs b;
+    uint8_t* p = static_cast<uint8_t*>(base);
+    b.ctl = reinterpret_cast<uint32_t*>(p);
+    p += 256;
+    b.segs = reinterpret_cast<TaskDesc*>(p);
+    p += sizeof(TaskDesc) * (uint64_t)cap;
+    b.splits = reinterpret_cast<SplitTask*>(p);
+    p += sizeof(SplitTask) * (uint64_t)(cap / 2);
+    b.first = reinterpret_cast<uint32_t*>(p);
+    p += 16ull * cap;
+    b.bytes = reinterpret_cast<uint32_t*>(p);
+    p += 16ull * cap;
+    b.marks = reinterpret_cast<uint32_t*>(p);
+    b.cap = cap;
+    b.weight = weight;
+    return b;
+}
+// Segments of a task of n symbols at segment length len: [0, len), [len, 2
+// len), ..., the last up to the stream's end.  1: not split, because it has
+// no more rounds than the call's cut or is hardly longer than a segment.
+__host__ __device__ inline uint32_t seg_count(uint32_t n, uint32_t len, uint32_t cut) {
+    const uint32_t rounds = (n + 3) >> 2;
+    return rounds <= cut || rounds < len + len / 2 ? 1u : (rounds + len - 1) / len;
+}
+// The cut of a call: tasks of more rounds are split.  The longest task left
+// whole takes 26 ns a round; walking the split ones takes the whole GPU 0.05
+// ns a round (SegBufs::weight times: 1 where the call waits for its result,
+// 3 where other batches in flight would use the GPU meanwhile: with ten in
+// flight 256 frames of 1 MiB take 3.1 ms a step whole and 4.2 ms split, with
+// three in flight 64 frames 3.3 and 1.7); and 0.2 ms pass before a segment
+// can be coded.  In units of 0.05 ns.  Below kCutMin rounds the walk and the
+// coding of the shortest segments (kWarm + kSegMin and kSegMin rounds) take
+// as long as the chain itself.
+constexpr uint32_t kCutMin = 2 * (kWarm + kSegMin);
+__host__ __device__ constexpr uint32_t seg_cut(int i) { return ((i & 1) ? 3 * kCutMin / 2 : kCutMin) << (i >> 1); }
+__host__ __device__ inline uint64_t cut_cost(uint64_t longest_whole, uint64_t split_rounds, uint32_t weight) {
+    return 520 * longest_whole + (split_rounds ? weight * split_rounds + 4200000 : 0);
+}
+// Most segments a task of up to n symbols, or several of n in all, can have.
+__host__ __device__ inline uint64_t seg_bound(uint64_t n) {
+    return (n >> 2) + 1 <= kCutMin ? 0 : (n >> 2) / kSegMin + 1;
+}
+inline uint32_t seg_cap(uint64_t bound) { return (uint32_t)(bound < kSegMax ? (bound + 1) & ~1ull : kSegMax); }
+
+// Task list: every active entry of [0, total) (get(e, d) fills the task and
+// says whether it is active), split by model kind and ordered longest-first
+// (by the bit length of the symbol count) so that the 8 tasks sharing a warp
+// have similar lengths and the long chains start first.  The segment length
+// is the shortest with which the tasks above the cut together have at most
+// sb.cap segments.  One block.
+template <class Get>
+__device__ void build_task_list(uint32_t total, Get get, TaskDesc* __restrict__ lists, uint32_t list_cap,
+                                uint32_t* __restrict__ counts, const SegBufs& sb) {
     __shared__ uint32_t s_cnt[2][33];
     __shared__ uint32_t s_pos[2][33];
+    __shared__ uint32_t s_segs[kSegSizes];
+    __shared__ unsigned long long s_rounds[kSegSizes];
+    __shared__ uint32_t s_len, s_nseg, s_nsplit, s_longest, s_cut;
     const uint32_t tid = threadIdx.x;
     if (tid < 66) (&s_cnt[0][0])[tid] = 0;
+    if (tid < kSegSizes) { s_segs[tid] = 0; s_rounds[tid] = 0; }
+    if (tid == 0) s_len = s_nseg = s_nsplit = s_longest = 0;
     __syncthreads();
-    const uint32_t total = njobs * T_COUNT;
+    if (sb.cap) {
+        for (uint32_t e = tid; e < total; e += blockDim.x) {
+            TaskDesc d;
+            if (!get(e, d)) continue;
+            const uint32_t rounds = (d.n + 3) >> 2;
+            int i = -1;  // the highest cut below it
+            while (i + 1 < kSegSizes && rounds > seg_cut(i + 1)) i++;
+            if (i >= 0) atomicAdd(&s_rounds[i], (unsigned long long)rounds);
+            atomicMax(&s_longest, rounds);
+        }
+        __syncthreads();
+        if (tid == 0) {
+            uint64_t best = cut_cost(s_longest, 0, sb.weight), above = 0;
+            s_cut = 0xFFFFFFFFu;
+            for (int i = kSegSizes - 1; i >= 0; i--) {
+                above += s_rounds[i];
+                if (above && cut_cost(seg_cut(i), above, sb.weight) < best) {
+                    best = cut_cost(seg_cut(i), above, sb.weight);
+                    s_cut = seg_cut(i);
+                }
+            }
+        }
+        __syncthreads();
+        for (uint32_t e = tid; e < total && s_cut != 0xFFFFFFFFu; e += blockDim.x) {
+            TaskDesc d;
+            if (!get(e, d)) continue;
+            for (int i = 0; i < kSegSizes; i++) {
+                const uint32_t c = seg_count(d.n, seg_len(i), s_cut);
+                if (c < 2) break;
+                atomicAdd(&s_segs[i], c);
+            }
+        }
+        __syncthreads();
+        if (tid == 0)
+            for (int i = kSegSizes - 1; i >= 0; i--)
+                if (s_segs[i] && s_segs[i] <= sb.cap) s_len = seg_len(i);
+        __syncthreads();
+    }
+    const uint32_t len = s_len, cut = s_cut;
     for (uint32_t e = tid; e < total; e += blockDim.x) {
-        const uint32_t j = j0 + e / T_COUNT;
-        const int t = (int)(e % T_COUNT);
-        const uint32_t* lens = job_lens + (uint64_t)j * S_COUNT;
-        const Job job = jobs[j];
-        const uint32_t nd = task_nd(job, s3f, j, t);
-        const uint32_t* fl = task_fl(job, fibbase);
-        if (!task_active(job, lens, t, nd, fl)) continue;
-        const uint32_t kind = task_is_m8(t) ? 1u : 0u;
-        atomicAdd(&s_cnt[kind][32 - __clz(task_len(lens, t, nd, fl))], 1u);
+        TaskDesc d;
+        if (!get(e, d)) continue;
+        const uint32_t c = len ? seg_count(d.n, len, cut) : 1u;
+        atomicAdd(&s_cnt[d.m8][32 - __clz(c > 1 ? 4 * len : d.n)], c);
     }
     __syncthreads();
     if (tid < 2) {
@@ -644,24 +782,431 @@ __global__ void __launch_bounds__(1024) k_task_list(const Job* __restrict__ jobs
     }
     __syncthreads();
     for (uint32_t e = tid; e < total; e += blockDim.x) {
+        TaskDesc d;
+        if (!get(e, d)) continue;
+        const uint32_t c = len ? seg_count(d.n, len, cut) : 1u;
+        d.lo = 0;
+        d.hi = kToTop;
+        d.seg = kNoSeg;
+        const uint32_t p = atomicAdd(&s_pos[d.m8][32 - __clz(c > 1 ? 4 * len : d.n)], c);
+        if (c == 1) {
+            lists[d.m8 * list_cap + p] = d;
+            continue;
+        }
+        SplitTask st;
+        st.d = d;
+        st.seg0 = atomicAdd(&s_nseg, c);
+        st.nseg = c;
+        st.len = len;
+        st.pos = p;
+        sb.splits[atomicAdd(&s_nsplit, 1u)] = st;
+    }
+    __syncthreads();
+    // the segments of the split tasks, a warp per task
+    for (uint32_t i = tid >> 5; i < s_nsplit; i += blockDim.x >> 5) {
+        const SplitTask st = sb.splits[i];
+        TaskDesc* l = lists + st.d.m8 * list_cap + st.pos;
+        for (uint32_t k = tid & 31; k < st.nseg; k += 32) {
+            TaskDesc d = st.d;
+            d.lo = k * len;
+            d.hi = k + 1 < st.nseg ? d.lo + len : kToTop;
+            d.seg = st.seg0 + k;
+            l[k] = d;
+            sb.segs[d.seg] = d;
+        }
+    }
+    __syncthreads();
+    if (tid == 0 && sb.cap) {
+        sb.ctl[0] = s_nsplit;
+        sb.ctl[1] = s_nseg;
+    }
+}
+
+__global__ void __launch_bounds__(1024) k_task_list(const Job* __restrict__ jobs, uint32_t j0, uint32_t njobs,
+                                                    const uint32_t* __restrict__ job_lens,
+                                                    const S3Frame* __restrict__ s3f, const uint8_t* __restrict__ streams,
+                                                    const uint8_t* __restrict__ s3base, const uint8_t* __restrict__ fibbase,
+                                                    uint8_t* __restrict__ ans, TaskDesc* __restrict__ lists,
+                                                    uint32_t list_cap, uint32_t* __restrict__ counts, SegBufs sb) {
+    auto get = [&](uint32_t e, TaskDesc& d) {
         const uint32_t j = j0 + e / T_COUNT;
         const int t = (int)(e % T_COUNT);
         const uint32_t* lens = job_lens + (uint64_t)j * S_COUNT;
         const Job job = jobs[j];
         const uint32_t nd = task_nd(job, s3f, j, t);
         const uint32_t* fl = task_fl(job, fibbase);
-        if (!task_active(job, lens, t, nd, fl)) continue;
-        const uint32_t kind = task_is_m8(t) ? 1u : 0u;
-        const uint32_t p = atomicAdd(&s_pos[kind][32 - __clz(task_len(lens, t, nd, fl))], 1u);
+        if (!task_active(job, lens, t, nd, fl)) return false;
         const TaskView v = task_view(job, lens, streams, s3base, fibbase, nd, fl, t);
-        TaskDesc d;
         d.src = v.src;
         d.base = ans + job.ans_off + v.ans_off;
         d.n = v.n;
         d.cap = v.cap;
         d.out = j * T_COUNT + (uint32_t)t;
         d.tab = j * kModels + task_model(t);
-        lists[kind * list_cap + p] = d;
+        d.m8 = task_is_m8(t) ? 1u : 0u;
+        return true;
+    };
+    build_task_list(njobs * T_COUNT, get, lists, list_cap, counts, sb);
+}
+
+// A symbol's entry as the walk takes it: {m, t1, c, (4096 - f) << 5 | s} of
+// its EncSym, so that a step unpacks one shift.
+__device__ __forceinline__ uint4 walk_sym(const EncSym& e) {
+    return make_uint4(e.m, e.t1, e.w & 0x1FFFu, (((e.w >> 13) & 0xFFFu) << 5) | (e.w >> 25));
+}
+// The same for the renormalise-first step: for f = 1 a reciprocal that is one
+// short, 2^32 - 1, with the deficit in c.
+__device__ __forceinline__ uint4 walk_sym_first(const uint4& e) {
+    return e.w == (4095u << 5 | 31u) ? make_uint4(0xFFFFFFFFu, e.y, e.z + 4095u, 4095u << 5) : e;
+}
+// rans_next with such an entry (x >= t2 is x >> 8 >= t1), in two forms.
+// Cycles a round, one warp per SM and eight per scheduler: multiply beside
+// the compares 36 and 24 a warp, renormalised first 57 and 17 a warp.  So
+// the first where the chain's latency counts, the second where several warps
+// share a scheduler.
+template <bool kFirst>
+__device__ __forceinline__ uint32_t walk_step(uint32_t x, const uint4& e) {
+    if (kFirst) {
+        if (x >= e.y) x >>= 8;
+        if (x >= e.y) x >>= 8;
+        return x + e.z + __funnelshift_r(__umulhi(x, e.x), 0u, e.w) * (e.w >> 5);
+    }
+    uint32_t k = x >= e.y ? 8u : 0u;
+    if ((x >> 8) >= e.y) k = 16u;
+    return (x >> k) + e.z + __funnelshift_r(__umulhi(x, e.x), 0u, e.w + k) * (e.w >> 5);
+}
+
+constexpr uint32_t kWalkTile = 512;  // rounds staged at a time
+constexpr uint32_t kWalkThreads = 128;
+constexpr uint32_t kWalkStride = kWalkTile + 8;  // u16 table offsets of a lane's rounds
+constexpr uint32_t kWalkStage = 2 * 4 * kWalkStride * 2;
+constexpr uint32_t kWalkSmemAd = 256 * 16 + kWalkStage;
+constexpr uint32_t kWalkSmemM8 = 8 * 256 * 16 + 256 + kWalkStage;
+
+// Rounds [512 k + 4 tid, ... + 4) of the four lanes, those below top, and the
+// byte before them (Meta8).
+struct WalkWords {
+    uint4 w;
+    uint32_t before;
+};
+template <bool kMeta8>
+__device__ __forceinline__ WalkWords walk_load(const uint8_t* __restrict__ src, bool vec, uint32_t k, uint32_t top) {
+    const uint32_t r = kWalkTile * k + 4 * threadIdx.x;
+    WalkWords q;
+    q.w = make_uint4(0, 0, 0, 0);
+    q.before = 0;
+    if (vec && r + 4 <= top) {
+        q.w = __ldg(reinterpret_cast<const uint4*>(src + 4ull * r));
+    } else {
+        uint32_t v[4] = {0, 0, 0, 0};
+#pragma unroll
+        for (uint32_t i = 0; i < 4; i++)
+            if (r + i < top) {
+                const uint8_t* p = src + 4ull * (r + i);
+                v[i] = (uint32_t)p[0] | ((uint32_t)p[1] << 8) | ((uint32_t)p[2] << 16) | ((uint32_t)p[3] << 24);
+            }
+        q.w = make_uint4(v[0], v[1], v[2], v[3]);
+    }
+    if (kMeta8 && r > 0 && r < top) q.before = src[4ull * r - 1];
+    return q;
+}
+// Their table offsets (16 bytes an entry) into the stage, lane by lane.
+template <bool kMeta8>
+__device__ __forceinline__ void walk_put(uint16_t* __restrict__ st, const WalkWords& q, const uint8_t* __restrict__ lut) {
+    const uint32_t w[4] = {q.w.x, q.w.y, q.w.z, q.w.w};
+#pragma unroll
+    for (uint32_t l = 0; l < 4; l++) {
+        uint2 o;
+        if (kMeta8) {
+            uint32_t v[4];
+#pragma unroll
+            for (uint32_t i = 0; i < 4; i++) {
+                const uint32_t prev = l ? (w[i] >> (8 * l - 8)) & 0xFFu : i ? w[i - 1] >> 24 : q.before;
+                v[i] = ((uint32_t)lut[prev] << 12) | (((w[i] >> (8 * l)) & 0xFFu) << 4);
+            }
+            o = make_uint2(v[0] | (v[1] << 16), v[2] | (v[3] << 16));
+        } else {
+            o = make_uint2(((w[0] >> (8 * l)) & 0xFFu) << 4 | (((w[1] >> (8 * l)) & 0xFFu) << 20),
+                           ((w[2] >> (8 * l)) & 0xFFu) << 4 | (((w[3] >> (8 * l)) & 0xFFu) << 20));
+        }
+        *reinterpret_cast<uint2*>(st + l * kWalkStride + 4 * threadIdx.x) = o;
+    }
+}
+
+// Rounds [0, cnt) of a staged lane, the last first, for kN states.  The
+// entries of three rounds are on their way while one steps.
+template <bool kFirst, int kN>
+__device__ __forceinline__ void walk_tile(uint32_t (&xs)[kN], const uint16_t* __restrict__ st, uint32_t cnt,
+                                          const uint8_t* __restrict__ tab) {
+    auto at = [&](uint32_t off) { return *reinterpret_cast<const uint4*>(tab + off); };
+    auto step = [&](const uint4& e) {
+#pragma unroll
+        for (int i = 0; i < kN; i++) xs[i] = walk_step<kFirst>(xs[i], e);
+    };
+    for (; cnt & 7; cnt--) step(at(st[cnt - 1]));
+    const uint4* s8 = reinterpret_cast<const uint4*>(st);
+    int32_t g = (int32_t)(cnt >> 3) - 1;
+    if (g < 0) return;
+    uint4 o = s8[g];
+    uint4 a = at(o.w >> 16), b = at(o.w & 0xFFFFu), c = at(o.z >> 16), d;
+    for (; g >= 0; g--) {
+        const uint4 n = s8[max(g - 1, 0)];
+        d = at(o.z & 0xFFFFu);
+        step(a);
+        a = at(o.y >> 16);
+        step(b);
+        b = at(o.y & 0xFFFFu);
+        step(c);
+        c = at(o.x >> 16);
+        step(d);
+        d = at(o.x & 0xFFFFu);
+        step(a);
+        a = at(n.w >> 16);
+        step(b);
+        b = at(n.w & 0xFFFFu);
+        step(c);
+        c = at(n.z >> 16);
+        step(d);
+        o = n;
+    }
+}
+
+// Equal neighbours of a ring of kN states (lanes of one aligned group of kN)
+// share a slot: the number of slots (0: one state in all) and this lane's.
+template <int kN>
+__device__ __forceinline__ uint32_t walk_slots(uint32_t x, uint32_t& slot, bool& lead, uint32_t& last) {
+    const uint32_t lane = threadIdx.x & 31, base = lane & ~(uint32_t)(kN - 1), k = lane & (kN - 1);
+    const uint32_t prev = __shfl_sync(0xFFFFFFFFu, x, base + ((k + kN - 1) & (kN - 1)));
+    lead = x != prev;
+    uint32_t m = __ballot_sync(0xFFFFFFFFu, lead) >> base;
+    if (kN < 32) m &= (1u << (kN & 31)) - 1u;
+    const uint32_t c = __popc(m);
+    slot = c ? (__popc(m & (0xFFFFFFFFu >> (31 - k))) + c - 1) % c : 0u;
+    last = __shfl_sync(0xFFFFFFFFu, x, base + (m ? 31 - __clz(m) : 0));
+    return c;
+}
+
+// The distinct states of 64 in ring order (two a lane) when they are at most
+// 32, else every second one.
+__device__ __forceinline__ uint32_t walk_halve(const uint32_t (&xs)[2], uint32_t* __restrict__ s_w) {
+    const uint32_t lane = threadIdx.x & 31;
+    const uint32_t prev = __shfl_sync(0xFFFFFFFFu, xs[1], (lane + 31) & 31);
+    const bool la = xs[0] != prev, lb = xs[1] != xs[0];
+    const uint32_t a = __ballot_sync(0xFFFFFFFFu, la), b = __ballot_sync(0xFFFFFFFFu, lb);
+    const uint32_t c = __popc(a) + __popc(b), lt = (1u << lane) - 1u;
+    if (c > 32 || c == 0) return xs[0];
+    const uint32_t at = __popc(a & lt) + __popc(b & lt);
+    if (la) s_w[at] = xs[0];
+    if (lb) s_w[at + la] = xs[1];
+    __syncwarp();
+    const uint32_t x = s_w[min(lane, c - 1)];
+    __syncwarp();
+    return x;
+}
+
+// The walkers of one segment: block b, segment b, warp l its lane l, all
+// states at the same round, so a round's table entry is one broadcast load.
+// Once no lane has more than 16 distinct states left warps 0 and 1 go on with
+// two lanes each, at eight warp 0 with all four; the others then only stage
+// symbols.
+template <bool kMeta8>
+__global__ void __launch_bounds__(kWalkThreads, kMeta8 ? 4 : 12) k_seg_walk(SegBufs sb, const EncSym* __restrict__ tabs,
+                                                                           const EncSym* __restrict__ meta8,
+                                                                           const uint8_t* __restrict__ ctxlut) {
+    extern __shared__ __align__(16) uint8_t smem_w[];
+    __shared__ uint32_t s_x[2][64], s_cnt[2][4], s_t[64], s_map[64], s_w[4][32];
+    const uint32_t nseg = sb.ctl[1];
+    if (blockIdx.x >= nseg) return;
+    const TaskDesc d = sb.segs[blockIdx.x];
+    if ((d.m8 != 0) != kMeta8) return;
+    const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    uint4* tab = reinterpret_cast<uint4*>(smem_w);
+    constexpr uint32_t kTab = (kMeta8 ? 8u : 1u) * 256;
+    uint8_t* lut = smem_w + kTab * 16;
+    uint16_t* stage = reinterpret_cast<uint16_t*>(smem_w + kTab * 16 + (kMeta8 ? 256 : 0));
+    const EncSym* gt = kMeta8 ? meta8 : tabs + (uint64_t)d.tab * 256;
+    // the form with the short chain once at most two of its warps share a scheduler
+    auto latency = [&](uint32_t mode) { return nseg * (4u >> mode) <= 2u * 4 * 148; };
+    uint32_t mode = 0;  // mode 0, 1, 2: 32, 16, 8 states of a lane
+    bool first_form = !latency(mode);
+    for (uint32_t i = tid; i < kTab; i += kWalkThreads) {
+        const uint4 e = walk_sym(gt[i]);
+        tab[i] = first_form ? walk_sym_first(e) : e;
+    }
+    if (kMeta8) for (uint32_t i = tid; i < 256; i += kWalkThreads) lut[i] = ctxlut[i];
+    const bool vec = (reinterpret_cast<uintptr_t>(d.src) & 15) == 0;
+    // from the stream's end when that is within the warm-up: the chain itself
+    const uint32_t rounds = d.n >> 2;
+    const bool from_end = d.hi == kToTop || d.hi + kWarm > rounds;
+    const uint32_t top = from_end ? rounds : d.hi + kWarm;
+    const uint32_t hi = d.hi == kToTop ? 0xFFFFFFFFu : d.hi;
+    const int32_t k0 = (int32_t)(d.lo / kWalkTile);
+    int32_t k = (int32_t)(top / kWalkTile);  // the first tile may hold no round: its mark is due all the same
+    WalkWords nx = walk_load<kMeta8>(d.src, vec, k, top);
+    __syncthreads();
+    walk_put<kMeta8>(stage + (k & 1) * 4 * kWalkStride, nx, lut);
+    // 64 states spread evenly over the logarithm of the range, eight to a
+    // doubling, two neighbours a thread; the first tile leaves about 25 of them
+    const uint32_t q4 = lane & 3, up = lane >> 2;
+    uint32_t xs[2] = {(q4 == 0 ? 65536u : q4 == 1 ? 77936u : q4 == 2 ? 92682u : 110218u) << up,
+                      (q4 == 0 ? 71468u : q4 == 1 ? 84990u : q4 == 2 ? 101070u : 120194u) << up};
+    uint32_t x = from_end ? 65536u : xs[0];
+    bool two = !from_end;
+    if (from_end && 4 * rounds + warp < d.n) {  // the stream's incomplete last round
+        const uint32_t i = 4 * rounds + warp;
+        uint32_t ti = d.src[i];
+        if (kMeta8) ti |= (i ? (uint32_t)lut[d.src[i - 1]] : 0u) << 8;
+        x = first_form ? walk_step<true>(x, tab[ti]) : walk_step<false>(x, tab[ti]);
+    }
+    uint32_t* marks = sb.marks + (uint64_t)blockIdx.x * kMarks * 4 * kWalkers + tid;
+    uint32_t slot = 0, l = warp;
+    __syncthreads();
+    for (; k >= k0; k--) {
+        const uint32_t r0 = kWalkTile * k, b = k & 1;
+        if (k > k0) nx = walk_load<kMeta8>(d.src, vec, k - 1, top);
+        const bool active = warp < (4u >> mode);
+        if (active && top > r0) {
+            const uint16_t* st = stage + (b * 4 + l) * kWalkStride;
+            const uint32_t cnt = min(kWalkTile, top - r0);
+            if (two) {
+                if (first_form) walk_tile<true, 2>(xs, st, cnt, smem_w);
+                else walk_tile<false, 2>(xs, st, cnt, smem_w);
+                x = walk_halve(xs, s_w[warp]);
+                two = false;
+            } else {
+                uint32_t x1[1] = {x};
+                if (first_form) walk_tile<true, 1>(x1, st, cnt, smem_w);
+                else walk_tile<false, 1>(x1, st, cnt, smem_w);
+                x = x1[0];
+            }
+        }
+        if (k > k0) walk_put<kMeta8>(stage + (b ^ 1) * 4 * kWalkStride, nx, lut);
+        uint32_t ns = 0, last = 0;
+        bool lead = false;
+        if (mode == 0) {
+            const uint32_t c = walk_slots<32>(x, ns, lead, last);
+            if (lane == 0) s_cnt[b][warp] = c;
+        } else if (active) {
+            s_x[b][tid] = x;
+            if (mode == 1) {
+                const uint32_t c = walk_slots<16>(x, ns, lead, last);
+                if ((lane & 15) == 0) s_cnt[b][tid >> 4] = c;
+            }
+        }
+        __syncthreads();
+        // the states at the segment's marks
+        uint32_t mark = kMarks;
+        if (r0 == d.lo) mark = kMarks - 1;
+        else if (r0 == hi) mark = 0;
+        else if (r0 < hi && hi != 0xFFFFFFFFu) {
+            const uint32_t in = hi - r0;
+            if ((in & (in - 1)) == 0 && in < (256u << (kMarks - 1))) mark = 31 - __clz(in >> 8);
+        }
+        if (mark < kMarks)
+            marks[mark * 4 * kWalkers] = mode == 0 ? x : mode == 1 ? s_x[b][warp * 16 + slot] : s_x[b][warp * 8 + slot];
+        // fewer warps when few enough states are left in every lane
+        const uint32_t most = max(max(s_cnt[b][0], s_cnt[b][1]), max(s_cnt[b][2], s_cnt[b][3]));
+        if (mode == 0 && most <= 16) {
+            const uint32_t c = max(s_cnt[b][warp], 1u);
+            if (lane >= c && lane < 16) s_t[warp * 16 + lane] = last;
+            if (lead || (s_cnt[b][warp] == 0 && lane == 0)) s_t[warp * 16 + ns] = x;
+            slot = ns;
+            __syncthreads();
+            mode = 1;
+            l = 2 * warp + (lane >> 4);
+            if (warp < 2) x = s_t[tid];
+        } else if (mode == 1 && most <= 8) {
+            if (active) {
+                const uint32_t c = max(s_cnt[b][l], 1u), i = lane & 15;
+                if (i >= c && i < 8) s_t[l * 8 + i] = last;
+                if (lead || (s_cnt[b][l] == 0 && i == 0)) s_t[l * 8 + ns] = x;
+                s_map[tid] = ns;
+            }
+            __syncthreads();
+            slot = s_map[warp * 16 + slot];
+            mode = 2;
+            l = lane >> 3;
+            if (warp == 0) x = s_t[lane];
+        }
+        if (first_form && latency(mode)) {
+            first_form = false;
+            __syncthreads();
+            for (uint32_t i = tid; i < kTab; i += kWalkThreads) tab[i] = walk_sym(gt[i]);
+            __syncthreads();
+        }
+    }
+}
+
+// Rounds [lo, hi) of lane l from the last down with one state in all lanes of
+// the warp (a segment whose first state no walker had): 32 rounds at a time,
+// lane i bringing the entry of the i-th, the next 32 on their way meanwhile.
+template <bool kMeta8>
+__device__ uint32_t walk_rounds(uint32_t x, const uint8_t* __restrict__ src, uint32_t lo, uint32_t hi, uint32_t l,
+                                const EncSym* __restrict__ tab, const uint8_t* __restrict__ ctxlut,
+                                uint4 (*__restrict__ s_e)[32]) {
+    const uint32_t lane = threadIdx.x & 31;
+    auto entry = [&](uint32_t r) {
+        uint32_t ti = 0;
+        if (lane < r - lo) {
+            const uint32_t i = 4 * (r - 1 - lane) + l;
+            ti = src[i];
+            if (kMeta8) ti |= (i ? (uint32_t)ctxlut[src[i - 1]] : 0u) << 8;
+        }
+        return walk_sym(tab[ti]);
+    };
+    uint4 nx = entry(hi);
+    uint32_t b = 0;
+    for (uint32_t r = hi; r > lo; r -= 32, b ^= 1) {  // hi - lo is a multiple of 32
+        s_e[b][lane] = nx;
+        __syncwarp();
+        if (r - lo > 32) nx = entry(r - 32);
+#pragma unroll 8
+        for (uint32_t q = 0; q < 32; q++) x = walk_step<false>(x, s_e[b][q]);
+    }
+    return x;
+}
+
+// The true first state of every segment of a split task: block b, task b,
+// warp l its lane l.  Per segment two coalesced loads (those of eight
+// segments at a time, so that their latency is paid once), a vote and a
+// shuffle.
+__global__ void __launch_bounds__(128) k_seg_resolve(SegBufs sb, const EncSym* __restrict__ tabs,
+                                                     const EncSym* __restrict__ meta8,
+                                                     const uint8_t* __restrict__ ctxlut) {
+    __shared__ uint4 s_e[4][2][32];
+    if (blockIdx.x >= sb.ctl[0]) return;
+    const SplitTask st = sb.splits[blockIdx.x];
+    const uint32_t l = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t* mk = sb.marks + threadIdx.x;
+    auto at = [&](uint32_t seg, uint32_t mark) { return mk[((uint64_t)(st.seg0 + seg) * kMarks + mark) * 4 * kWalkers]; };
+    uint32_t* first = sb.first + 4 * (uint64_t)st.seg0 + l;
+    if (lane == 0) first[4 * (st.nseg - 1)] = 65536u;
+    uint32_t x = at(st.nseg - 1, kMarks - 1);  // the last segment's walkers are the chain itself
+    for (int32_t c = (int32_t)st.nseg - 2; c >= 0; c -= 8) {
+        uint32_t s[8], e[8];
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+            s[i] = c >= i ? at(c - i, 0) : 0u;
+            e[i] = c >= i ? at(c - i, kMarks - 1) : 0u;
+        }
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+            const int32_t seg = c - i;
+            if (seg < 0) break;
+            if (lane == 0) first[4 * seg] = x;
+            uint32_t hit = __ballot_sync(0xFFFFFFFFu, s[i] == x);
+            uint32_t r = (uint32_t)(seg + 1) * st.len;
+            for (uint32_t m = 1; !hit && m < kMarks; m++) {
+                const uint32_t to = m + 1 < kMarks ? (256u << m) : st.len;  // rounds into the segment
+                if (m + 1 < kMarks && to >= st.len) continue;
+                const uint32_t lo = (uint32_t)(seg + 1) * st.len - to;
+                x = st.d.m8 ? walk_rounds<true>(x, st.d.src, lo, r, l, meta8, ctxlut, s_e[l])
+                            : walk_rounds<false>(x, st.d.src, lo, r, l, tabs + (uint64_t)st.d.tab * 256, nullptr, s_e[l]);
+                r = lo;
+                if (m + 1 < kMarks) hit = __ballot_sync(0xFFFFFFFFu, at(seg, m) == x);
+            }
+            if (hit) x = __shfl_sync(0xFFFFFFFFu, e[i], __ffs(hit) - 1);
+        }
     }
 }
 
@@ -674,12 +1219,13 @@ constexpr uint32_t kRansTabBytes = 8 * 256 * sizeof(EncSym);          // 8 model
 constexpr uint32_t kRansSmem = kRansWarps * (kRansTabBytes + kRingBytesPerWarp);  // tables, rings
 
 // Blocks [0, nb_ad) run adaptive-model tasks, the rest Meta8 tasks; each
-// warp takes 8 consecutive tasks of its list (4 lanes per task).
+// warp takes 8 consecutive tasks (or segments) of its list (4 lanes per task).
 __global__ void __launch_bounds__(kRansWarps * 32) k_rans(const TaskDesc* __restrict__ lists, uint32_t list_cap,
                                                           const uint32_t* __restrict__ counts, uint32_t nb_ad,
                                                           const EncSym* __restrict__ tabs,
                                                           const EncSym* __restrict__ meta8,
-                                                          const uint8_t* __restrict__ ctxlut, TaskOut* __restrict__ outs) {
+                                                          const uint8_t* __restrict__ ctxlut, TaskOut* __restrict__ outs,
+                                                          SegBufs sb) {
     extern __shared__ __align__(16) uint8_t smem_r[];
     __shared__ uint8_t s_lut[256];
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -687,6 +1233,7 @@ __global__ void __launch_bounds__(kRansWarps * 32) k_rans(const TaskDesc* __rest
     const uint32_t nlist = counts[m8 ? 1 : 0];
     const TaskDesc* dl = lists + (m8 ? list_cap : 0);
     const uint32_t wg = (m8 ? blockIdx.x - nb_ad : blockIdx.x) * kRansWarps + warp;  // warp index in its list
+    if (kRansWarps == 1 && wg * 8 >= nlist) return;
     EncSym* wtab = reinterpret_cast<EncSym*>(smem_r + warp * kRansTabBytes);
     uint4* wring = reinterpret_cast<uint4*>(smem_r + kRansWarps * kRansTabBytes + warp * kRingBytesPerWarp);
     if (m8) {
@@ -709,8 +1256,45 @@ __global__ void __launch_bounds__(kRansWarps * 32) k_rans(const TaskDesc* __rest
     const TaskDesc d = dl[ti];
     LaneIO io = lane_io(d.base, d.cap, l);
     TaskOut* o = outs + d.out;
-    if (m8) rans_lane<true>(d.src, d.n, l, wtab, s_lut, wring, io, &o->state[l], &o->count[l]);
-    else rans_lane<false>(d.src, d.n, l, wtab + slot * 256, nullptr, wring, io, &o->state[l], &o->count[l]);
+    uint32_t x0 = 65536;
+    uint32_t *px = &o->state[l], *pc = &o->count[l];
+    if (d.seg != kNoSeg) {
+        x0 = sb.first[4 * d.seg + l];
+        pc = &sb.bytes[4 * d.seg + l];
+        if (d.lo) px = &sb.first[4 * d.seg + l];  // the task's last state is its lowest segment's
+    }
+    if (m8) rans_lane<true>(d.src, d.n, l, d.lo, d.hi, x0, wtab, s_lut, wring, io, px, pc);
+    else rans_lane<false>(d.src, d.n, l, d.lo, d.hi, x0, wtab + slot * 256, nullptr, wring, io, px, pc);
+}
+
+// Byte counts of a split task from its segments': the lane's total, and
+// every running count (io.cum) raised by the segments above its own.  Block
+// b, task b; warp l, lane l; 32 segments at a time from the top.
+__global__ void __launch_bounds__(128) k_seg_sums(SegBufs sb, TaskOut* __restrict__ outs) {
+    if (blockIdx.x >= sb.ctl[0]) return;
+    const SplitTask st = sb.splits[blockIdx.x];
+    const uint32_t l = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    uint32_t* cum = lane_io(st.d.base, st.d.cap, l).cum;
+    const uint32_t last = (st.d.n - 1 - l) >> 2;  // the lane's last round
+    uint32_t above = 0;
+    for (int32_t c0 = (int32_t)st.nseg - 1; c0 >= 0; c0 -= 32) {
+        const int32_t c = c0 - (int32_t)lane;
+        const uint32_t v = c >= 0 ? sb.bytes[4 * (st.seg0 + c) + l] : 0u;
+        uint32_t sum = v;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, sum, o);
+            if (lane >= (uint32_t)o) sum += y;
+        }
+        const uint32_t before = above + sum - v;
+        if (c >= 0 && before) {
+            const uint32_t lo = (uint32_t)c * st.len, hi = c + 1 < (int32_t)st.nseg ? lo + st.len : last + 1;
+            for (uint32_t r = (lo + kStitchRounds - 1) / kStitchRounds * kStitchRounds; r < hi; r += kStitchRounds)
+                cum[r / kStitchRounds] += before;
+        }
+        above += __shfl_sync(0xFFFFFFFFu, sum, 31);
+    }
+    if (lane == 0) outs[st.d.out].count[l] = above;
 }
 
 // ---------------------------------------------------------------------------

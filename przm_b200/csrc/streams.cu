@@ -62,9 +62,25 @@ __global__ void __launch_bounds__(256) k_stream_hist(const STask* __restrict__ t
     for (uint32_t ti = blockIdx.y; ti < ntasks; ti += gridDim.y) stream_hist_task(tasks[ti], ti, s_h, counts);
 }
 
-// One warp per task: normalise and build the encoding table + matrix.
+__device__ __forceinline__ bool stream_desc(const STask& t, uint32_t ti, TaskDesc& d) {
+    d.src = reinterpret_cast<const uint8_t*>(t.src);
+    d.base = reinterpret_cast<uint8_t*>(t.scr);
+    d.n = t.n;
+    d.cap = t.cap;
+    d.out = d.tab = ti;
+    d.lo = 0;
+    d.hi = kToTop;
+    d.seg = kNoSeg;
+    d.m8 = 0;
+    return t.n != 0;
+}
+
+// One warp per task: normalise and build the encoding table + matrix.  list
+// (optional): the tasks as they come as the rANS kernel's list, for calls
+// with no task long enough to split (a launch of its own costs them 5 us).
 __global__ void k_stream_norm(const STask* __restrict__ tasks, uint32_t ntasks, const uint32_t* __restrict__ counts,
-                              EncSym* __restrict__ tabs, TableInfo* __restrict__ infos) {
+                              EncSym* __restrict__ tabs, TableInfo* __restrict__ infos, TaskDesc* __restrict__ list,
+                              uint32_t* __restrict__ list_n) {
     __shared__ uint32_t s_cnt[256];
     __shared__ uint16_t s_freq[256];
     __shared__ GoRem s_rem[256];
@@ -72,6 +88,10 @@ __global__ void k_stream_norm(const STask* __restrict__ tasks, uint32_t ntasks, 
     const uint32_t ti = blockIdx.x;
     if (ti >= ntasks) return;
     const STask t = tasks[ti];
+    if (list && lane == 0) {
+        stream_desc(t, ti, list[ti]);
+        if (ti == 0) list_n[0] = ntasks;
+    }
     if (t.norm == 2 || t.n == 0) return;
     for (uint32_t s = lane; s < 256; s += 32) s_cnt[s] = counts[(uint64_t)ti * 256 + s];
     __syncwarp();
@@ -80,32 +100,20 @@ __global__ void k_stream_norm(const STask* __restrict__ tasks, uint32_t ntasks, 
     warp_build_table(s_freq, tabs + (uint64_t)ti * 256, infos + ti, lane);
 }
 
-// One warp per 8 tasks (4 lanes each), tables and rings in shared memory.
-__global__ void __launch_bounds__(kRansWarps * 32) k_stream_rans(const STask* __restrict__ tasks, uint32_t ntasks,
-                                                                 const EncSym* __restrict__ tabs,
-                                                                 TaskOut* __restrict__ outs) {
-    extern __shared__ __align__(16) uint8_t smem_s[];
-    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const uint32_t wg = blockIdx.x * kRansWarps + warp;
-    EncSym* wtab = reinterpret_cast<EncSym*>(smem_s + warp * kRansTabBytes);
-    uint4* wring = reinterpret_cast<uint4*>(smem_s + kRansWarps * kRansTabBytes + warp * kRingBytesPerWarp);
-    for (uint32_t k = 0; k < 8; k++) {
-        const uint32_t tk = wg * 8 + k;
-        if (tk >= ntasks) break;
-        for (uint32_t i = lane; i < 256; i += 32) wtab[k * 256 + i] = tabs[(uint64_t)tk * 256 + i];
-    }
-    __syncwarp();
-    const uint32_t ti = wg * 8 + (lane >> 2), l = lane & 3;
-    if (ti >= ntasks) return;
-    const STask t = tasks[ti];
-    if (t.n == 0) return;
-    LaneIO io = lane_io(reinterpret_cast<uint8_t*>(t.scr), t.cap, l);
-    rans_lane<false>(reinterpret_cast<const uint8_t*>(t.src), t.n, l, wtab + (lane >> 2) * 256, nullptr, wring, io,
-                     &outs[ti].state[l], &outs[ti].count[l]);
+// The streams with symbols as the rANS kernel's task list (lists[list_cap],
+// counts[0]; no Meta8 tasks).
+__global__ void __launch_bounds__(1024) k_stream_list(const STask* __restrict__ tasks, uint32_t ntasks,
+                                                      TaskDesc* __restrict__ lists, uint32_t list_cap,
+                                                      uint32_t* __restrict__ counts, SegBufs sb) {
+    auto get = [&](uint32_t e, TaskDesc& d) { return stream_desc(tasks[e], e, d); };
+    build_task_list(ntasks, get, lists, list_cap, counts, sb);
 }
 
 constexpr int kStitchThreads = 256;
+static_assert(16 * kStitchThreads == kStitchRounds, "a block takes whole stitch passes");
 
+// Block (x, y): stitch passes y, y + gridDim.y, ... of task x, each at the
+// offset the rANS lanes recorded; block (x, 0) writes the container's head.
 __global__ void __launch_bounds__(kStitchThreads) k_stream_stitch(const STask* __restrict__ tasks, uint32_t ntasks,
                                                                   const TableInfo* __restrict__ infos,
                                                                   const TaskOut* __restrict__ outs,
@@ -113,11 +121,15 @@ __global__ void __launch_bounds__(kStitchThreads) k_stream_stitch(const STask* _
     const uint32_t ti = blockIdx.x;
     if (ti >= ntasks) return;
     const STask t = tasks[ti];
-    if (t.n == 0) { if (threadIdx.x == 0) out_lens[ti] = 0; return; }
+    if (t.n == 0) { if (threadIdx.x == 0 && blockIdx.y == 0) out_lens[ti] = 0; return; }
     uint8_t* dst = reinterpret_cast<uint8_t*>(t.dst);
     const TableInfo* info = infos + ti;
     const TaskOut o = outs[ti];
     const uint32_t h = 8 + info->mat_len;
+    const uint8_t* scr = reinterpret_cast<const uint8_t*>(t.scr);
+    for (uint32_t r0 = blockIdx.y * kStitchRounds; r0 < (t.n + 3) / 4; r0 += gridDim.y * kStitchRounds)
+        stitch_pass<kStitchThreads>(scr, t.cap, t.n, r0, dst + h + 16 + stitch_offset(scr, t.cap, t.n, o, r0));
+    if (blockIdx.y) return;
     if (threadIdx.x == 0) {
         dst[0] = 'V'; dst[1] = 'A'; dst[2] = 0x01; dst[3] = (uint8_t)t.flags;
         for (int k = 0; k < 4; k++) dst[4 + k] = (uint8_t)(t.n >> (8 * k));
@@ -126,7 +138,6 @@ __global__ void __launch_bounds__(kStitchThreads) k_stream_stitch(const STask* _
         out_lens[ti] = h + 16 + o.count[0] + o.count[1] + o.count[2] + o.count[3];
     }
     for (uint32_t i = threadIdx.x; i < info->mat_len; i += kStitchThreads) dst[8 + i] = info->mat[i];
-    block_stitch<kStitchThreads>(reinterpret_cast<const uint8_t*>(t.scr), t.cap, t.n, dst + h + 16);
 }
 
 // PackStreamFlat (przm_ans.cu:202-234): 0x00 | LE32 n | payload.
