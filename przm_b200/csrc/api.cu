@@ -25,6 +25,7 @@
 #include "fibers.cu"
 #include "frame.cu"
 #include "decode.cu"
+#include "exec.cu"
 #include "match.cu"
 #include "tokenize.cu"
 #include "front.cu"

@@ -23,10 +23,14 @@
 //   k_dec_sheaf    two warps per sheaf frame: the literals re-interleaved
 //                  from their four fibers by the class of the bytes before
 //                  each (the order of the fibers is serial by the format).
-//   k_dec_exec     one warp per frame: the command walk, every lane running
-//                  the same scalar parse, literal and match copies split over
-//                  the lanes (a match closer than its length repeats with
-//                  period d, so byte i comes from source byte i mod d).
+//   k_dec_exec     (exec.cu) one block per frame: 512 commands at a time,
+//                  the output made in tiles;
+//   k_dec_exec_serial  one warp per frame that uses opcodes of the
+//                  reference's CPU compressor: the command walk, every lane
+//                  running the same scalar parse, literal and match copies
+//                  split over the lanes (a match closer than its length
+//                  repeats with period d, so byte i comes from source byte
+//                  i mod d).
 //
 // Frames this decoder does not take (an external dictionary, the base64
 // normalisation flag, delta-masked matches, the nibble-plane literal form,
@@ -79,6 +83,7 @@ struct DecInfo {
     uint32_t s3_prefix;  // 1: distance-prefix container, varints rebuilt into DB_OFFS
     uint32_t nd, extra_len, s3_orig;
     uint32_t sheaf, sheaf_mode;
+    uint32_t serial;     // left to k_dec_exec_serial
     uint32_t fl[4];
     uint64_t cmd, meta, var, off, lit, codes, extra;
     uint64_t fib[4];
@@ -1241,25 +1246,54 @@ __device__ __forceinline__ void warp_copy_match(uint8_t* dst, uint8_t* ring, uin
     __syncwarp();
 }
 
+// The joined stream left after the walk, demultiplexed without executing
+// (demux_commands, przm_dec.c:605-623): it must fill the joined length and
+// use up the three substreams.  Returns the DecErr.
+__device__ uint32_t exec_rest(CmdReader& R) {
+    while (R.cp < R.cl && R.j < R.jlim) {
+        const uint32_t op = R.c[R.cp++];
+        R.j++;
+        uint32_t t;
+        bool ok = true;
+        if (op < 0x80 || (op >= 0xF3 && op <= 0xFA)) {
+        } else if (op < 0xC0) {
+            if ((op & 15) == 15) ok = R.skip_leb();
+        } else if (op <= 0xC3 || op == 0xE9) {
+            ok = R.meta(t) && ((t & 15) != 15 || R.skip_leb());
+        } else if (op <= 0xCD || (op >= 0xD0 && op <= 0xD7)) {
+            ok = R.meta(t);
+        } else if (op == 0xCE) {
+            uint32_t t2;
+            ok = R.meta(t) && R.meta(t2) && (((t >> 3) & 7) != 7 || R.skip_leb()) && ((t & 7) != 7 || R.skip_leb());
+        } else if (op == 0xCF || (op >= 0xEA && op <= 0xEF)) {
+            ok = R.meta(t) && R.skip_leb();
+        } else if (op <= 0xE8) {
+            ok = R.meta(t) && (t != 255 || R.skip_leb());
+        } else if (op == 0xF0 || op == 0xF1) {
+            ok = R.skip_leb();
+        } else {
+            ok = false;
+        }
+        if (!ok) return D_CORRUPT;
+    }
+    return R.j != R.jlim || R.cp != R.cl || R.mp != R.ml || R.vp != R.vl ? D_CORRUPT : D_OK;
+}
+
 // The command walk of frame blockIdx.x (stage_execute_commands,
-// przm_dec.c:1285-1525; decompress.go:380-672): one warp, every lane
-// parsing the same commands; the opcodes of the tokenizer (fused repeat
+// przm_dec.c:1285-1525; decompress.go:380-672) where k_dec_exec left it to
+// this kernel: one warp, every lane parsing the same commands; the opcodes of the tokenizer (fused repeat
 // < 0x80, fused explicit 0x80-0xBF, long repeat 0xC0-0xC3, literal runs
 // 0xF0 / 0xF3-0xFA, byte runs 0xF1) and the plain-distance matches
 // (brackets 0xC4-0xCD, the difference lattice 0xCE, strides 0xD0-0xD7).
-__global__ void __launch_bounds__(32) k_dec_exec(const uint8_t* __restrict__ src, const DecJob* __restrict__ jobs,
-                                                 DecInfo* __restrict__ infos, uint8_t* __restrict__ out) {
+__global__ void __launch_bounds__(32) k_dec_exec_serial(const DecJob* __restrict__ jobs, DecInfo* __restrict__ infos,
+                                                        uint8_t* __restrict__ out) {
     const uint32_t f = blockIdx.x, lane = threadIdx.x;
     const DecInfo I = infos[f];
-    if (I.err || I.u_size == 0) return;
+    if (I.err || !I.serial) return;
     const DecJob jb = jobs[f];
     uint8_t* dst = out + jb.out_off;
     const uint32_t u = I.u_size;
     __shared__ __align__(16) uint8_t ring[kExecRing];
-    if (I.stored) {
-        warp_copy_lits(dst, ring, 0, src + jb.src_off + 8, u);
-        return;
-    }
     CmdReader R;
     R.c = reinterpret_cast<const uint8_t*>(I.cmd);
     R.m = reinterpret_cast<const uint8_t*>(I.meta);
@@ -1359,38 +1393,7 @@ __global__ void __launch_bounds__(32) k_dec_exec(const uint8_t* __restrict__ src
         dp += lmatch;
     }
     if (!err && dp != u) err = D_CORRUPT;
-    if (!err && R.split) {
-        // the rest of the joined stream, demultiplexed without executing
-        // (demux_commands, przm_dec.c:605-623): it must fill the joined
-        // length and use up the three substreams
-        while (!err && R.cp < R.cl && R.j < R.jlim) {
-            uint32_t op = R.c[R.cp++];
-            R.j++;
-            uint32_t t;
-            bool ok = true;
-            if (op < 0x80 || (op >= 0xF3 && op <= 0xFA)) {
-            } else if (op < 0xC0) {
-                if ((op & 15) == 15) ok = R.skip_leb();
-            } else if (op <= 0xC3 || op == 0xE9) {
-                ok = R.meta(t) && ((t & 15) != 15 || R.skip_leb());
-            } else if (op <= 0xCD || (op >= 0xD0 && op <= 0xD7)) {
-                ok = R.meta(t);
-            } else if (op == 0xCE) {
-                uint32_t t2;
-                ok = R.meta(t) && R.meta(t2) && (((t >> 3) & 7) != 7 || R.skip_leb()) && ((t & 7) != 7 || R.skip_leb());
-            } else if (op == 0xCF || (op >= 0xEA && op <= 0xEF)) {
-                ok = R.meta(t) && R.skip_leb();
-            } else if (op <= 0xE8) {
-                ok = R.meta(t) && (t != 255 || R.skip_leb());
-            } else if (op == 0xF0 || op == 0xF1) {
-                ok = R.skip_leb();
-            } else {
-                ok = false;
-            }
-            if (!ok) err = D_CORRUPT;
-        }
-        if (!err && (R.j != R.jlim || R.cp != R.cl || R.mp != R.ml || R.vp != R.vl)) err = D_CORRUPT;
-    }
+    if (!err && R.split) err = exec_rest(R);
     if (err && lane == 0) dec_fail(infos, f, err);
 }
 

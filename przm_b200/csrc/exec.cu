@@ -1,0 +1,471 @@
+// exec.cu -- the decoder's command execution (stage_execute_commands,
+// przm_dec.c:1285-1525; decompress.go:380-672), one block per frame.
+//
+// The reference walks the commands one after another; only two things in that
+// walk are serial: the repeat distances and the bytes a match copies from
+// output written just before.  Here 512 commands are taken at a time, a
+// thread each.  Where a command's operand bytes, literals and output start are
+// sums over the commands before it; the repeat distances before it are a scan
+// of maps on four distances (each command moves one to the front or pushes a
+// new one); the first command that ends the walk or fails decides, as in the
+// walk.  The output is then made 4096 bytes at a time: every byte finds its
+// command, literals and matches from before the tile load their byte, and the
+// others point at a byte of the tile and follow the pointers, which jump
+// twice as far each time.
+//
+// Takes the opcodes of the tokenizer: fused repeat (< 0x80), fused explicit
+// (0x80-0xBF), long repeat (0xC0-0xC3), literal runs (0xF0, 0xF3-0xFA), byte
+// runs (0xF1).  A frame that reaches another known opcode is left to
+// k_dec_exec_serial.
+//
+// Measured on 128 mixed frames of 1 MiB: 26.0 ms with one warp walking each
+// frame.
+#include "common.cuh"
+
+namespace pz {
+
+constexpr uint32_t kExThreads = 512;
+constexpr uint32_t kExTile = 4096, kExPer = kExTile / kExThreads;
+constexpr uint32_t kExWindow = 4 * kExThreads;  // bytes that hold a chunk's varints, at most four each
+constexpr uint32_t kExFlat = 6 * kExThreads;    // a flat command's bytes: opcode, token, varint
+constexpr uint32_t kExCap = 1u << 26;           // sums of lengths saturate here, above every frame's size
+
+// how the walk ends at a command
+enum ExecEvent : uint32_t { EV_BEFORE = 0, EV_AFTER = 1, EV_CORRUPT = 2, EV_UNSUPPORTED = 3, EV_SERIAL = 4, EV_NONE = 15 };
+
+struct ExecShared {
+    uint32_t start[kExThreads + 1];  // a command's first output byte
+    uint32_t lend[kExThreads];       // the end of its literals
+    uint32_t lsrc[kExThreads];       // where they start in the literal stream
+    uint32_t dist[kExThreads];       // its match's distance; 0: a run of literal lsrc
+    uint16_t vend[kExThreads], oend[kExThreads];  // ends of the chunk's varints in their windows
+    __align__(16) uint16_t w[kExTile];            // a tile's bytes: 0x8000 | byte, or a place in the tile
+    uint32_t warp[32], warp2[32];
+    uint32_t rep[kExThreads / 32][4];
+    uint16_t pos[kExThreads + 1];  // flat: where the chunk's commands start
+    uint32_t npos;
+    __align__(16) uint8_t flat[kExFlat + 16];
+    uint32_t event;
+    uint32_t st[12];  // the reader's state after the chunk, or at the end of the walk
+};
+
+// Two sums at once over the block, each saturating at kExCap: the sums before
+// this thread in a and b, the totals in ta and tb.
+__device__ __forceinline__ void exec_scan2(uint32_t& a, uint32_t& b, uint32_t& ta, uint32_t& tb, ExecShared& S) {
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    uint32_t x = min(a, kExCap), y = min(b, kExCap);
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t p = __shfl_up_sync(0xFFFFFFFFu, x, o), q = __shfl_up_sync(0xFFFFFFFFu, y, o);
+        if (lane >= (uint32_t)o) {
+            x = min(x + p, kExCap);
+            y = min(y + q, kExCap);
+        }
+    }
+    if (lane == 31) {
+        S.warp[warp] = x;
+        S.warp2[warp] = y;
+    }
+    const uint32_t ex = __shfl_up_sync(0xFFFFFFFFu, x, 1), ey = __shfl_up_sync(0xFFFFFFFFu, y, 1);
+    __syncthreads();
+    uint32_t bx = 0, by = 0;
+    ta = tb = 0;
+#pragma unroll
+    for (uint32_t w = 0; w < kExThreads / 32; w++) {
+        if (w == warp) {
+            bx = ta;
+            by = tb;
+        }
+        ta = min(ta + S.warp[w], kExCap);
+        tb = min(tb + S.warp2[w], kExCap);
+    }
+    a = min(bx + (lane ? ex : 0u), kExCap);
+    b = min(by + (lane ? ey : 0u), kExCap);
+    __syncthreads();
+}
+
+// A map of the four repeat distances: entry i a distance, or kRepFrom | j, the
+// j-th before.
+constexpr uint32_t kRepFrom = 0x80000000u;
+struct RepMap {
+    uint32_t e[4];
+};
+__device__ __forceinline__ uint32_t rep_of(const RepMap& a, uint32_t v) {
+    const uint32_t j = v & 3u;
+    const uint32_t s = j == 0 ? a.e[0] : j == 1 ? a.e[1] : j == 2 ? a.e[2] : a.e[3];
+    return (v & kRepFrom) ? s : v;
+}
+__device__ __forceinline__ RepMap rep_then(const RepMap& a, const RepMap& b) {  // a, then b
+    RepMap r;
+#pragma unroll
+    for (int i = 0; i < 4; i++) r.e[i] = rep_of(a, b.e[i]);
+    return r;
+}
+__device__ __forceinline__ RepMap rep_identity() {
+    return RepMap{{kRepFrom | 0u, kRepFrom | 1u, kRepFrom | 2u, kRepFrom | 3u}};
+}
+
+// Varint of len (1-4) bytes at p.
+__device__ __forceinline__ uint32_t exec_varint(const uint8_t* p, uint32_t len) {
+    uint32_t r = 0;
+    for (uint32_t i = 0; i < len; i++) r |= (uint32_t)(p[i] & 0x7Fu) << (7 * i);
+    return r;
+}
+
+// Ends of the varints in the 2048 bytes of s[at, n) (bit masks of this
+// thread's four bytes that end one).
+__device__ __forceinline__ uint32_t exec_ends(const uint8_t* s, uint32_t at, uint32_t n) {
+    uint32_t m = 0;
+#pragma unroll
+    for (uint32_t i = 0; i < 4; i++) {
+        const uint32_t p = at + 4 * threadIdx.x + i;
+        if (p < n && s[p] < 0x80u) m |= 1u << i;
+    }
+    return m;
+}
+__device__ __forceinline__ void exec_put_ends(uint16_t* ends, uint32_t m, uint32_t k) {
+#pragma unroll
+    for (uint32_t i = 0; i < 4; i++)
+        if ((m >> i) & 1u) {
+            if (k < kExThreads) ends[k] = (uint16_t)(4 * threadIdx.x + i + 1);
+            k++;
+        }
+}
+
+// Output bytes [dp, end) of the E commands in S.
+__device__ void exec_copy(ExecShared& S, uint8_t* dst, const uint8_t* __restrict__ lit, uint32_t dp, uint32_t end,
+                          uint32_t E) {
+    const uint32_t tid = threadIdx.x;
+    // tiles begin on 8-byte boundaries of the address
+    for (int32_t tb = (int32_t)dp - (int32_t)((reinterpret_cast<uintptr_t>(dst) + dp) & 7u); tb < (int32_t)end;
+         tb += kExTile) {
+        const int32_t lo = max(tb, (int32_t)dp), hi = min(tb + (int32_t)kExTile, (int32_t)end);
+        const int32_t p0 = tb + (int32_t)(kExPer * tid);
+        uint32_t v[kExPer];
+        uint32_t open = 0;  // own bytes that still point into the tile
+        if (p0 < hi && p0 + (int32_t)kExPer > lo) {
+            const uint32_t pf = (uint32_t)max(p0, lo);
+            uint32_t a = 0, b = E;  // the last command that starts at or before pf
+            while (b - a > 1) {
+                const uint32_t m = (a + b) / 2;
+                if (S.start[m] <= pf) a = m;
+                else b = m;
+            }
+            uint32_t c = a, cs = S.start[c], cn = S.start[c + 1], le = S.lend[c], ls = S.lsrc[c], d = S.dist[c];
+#pragma unroll
+            for (uint32_t i = 0; i < kExPer; i++) {
+                const int32_t p = p0 + (int32_t)i;
+                v[i] = 0x8000u;
+                if (p < lo || p >= hi) continue;
+                while ((uint32_t)p >= cn) {
+                    c++;
+                    cs = cn;
+                    cn = S.start[c + 1];
+                    le = S.lend[c];
+                    ls = S.lsrc[c];
+                    d = S.dist[c];
+                }
+                if ((uint32_t)p < le) {
+                    v[i] = 0x8000u | lit[ls + ((uint32_t)p - cs)];
+                } else if (d == 0) {
+                    v[i] = 0x8000u | lit[ls];
+                } else {
+                    uint32_t o = (uint32_t)p - le;
+                    if (o >= d) o %= d;  // a match closer than its length repeats
+                    const int32_t s = (int32_t)(le - d + o);
+                    if (s < lo) {
+                        v[i] = 0x8000u | dst[s];
+                    } else {
+                        v[i] = (uint32_t)(s - tb);
+                        open |= 1u << i;
+                    }
+                }
+            }
+            *reinterpret_cast<uint4*>(&S.w[kExPer * tid]) =
+                make_uint4(v[0] | (v[1] << 16), v[2] | (v[3] << 16), v[4] | (v[5] << 16), v[6] | (v[7] << 16));
+        }
+        // follow the pointers: a byte's word is its value or a place before it,
+        // whichever of a writer's words is read
+        volatile uint16_t* w = S.w;
+        while (__syncthreads_or(open)) {
+#pragma unroll
+            for (uint32_t i = 0; i < kExPer; i++)
+                if ((open >> i) & 1u) {
+                    v[i] = w[v[i]];
+                    w[kExPer * tid + i] = (uint16_t)v[i];
+                    if (v[i] & 0x8000u) open &= ~(1u << i);
+                }
+        }
+        if (p0 >= lo && p0 + (int32_t)kExPer <= hi) {
+            uint2 o = make_uint2(0, 0);
+#pragma unroll
+            for (uint32_t i = 0; i < 4; i++) {
+                o.x |= (v[i] & 0xFFu) << (8 * i);
+                o.y |= (v[4 + i] & 0xFFu) << (8 * i);
+            }
+            *reinterpret_cast<uint2*>(dst + p0) = o;
+        } else if (p0 < hi && p0 + (int32_t)kExPer > lo) {
+#pragma unroll
+            for (uint32_t i = 0; i < kExPer; i++)
+                if (p0 + (int32_t)i >= lo && p0 + (int32_t)i < hi) dst[p0 + (int32_t)i] = (uint8_t)v[i];
+        }
+        __syncthreads();  // the tile is read by the ones after it
+    }
+}
+
+__global__ void __launch_bounds__(kExThreads) k_dec_exec(const uint8_t* __restrict__ src, const DecJob* __restrict__ jobs,
+                                                         DecInfo* __restrict__ infos, uint8_t* __restrict__ out) {
+    __shared__ ExecShared S;
+    const uint32_t f = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const DecInfo I = infos[f];
+    if (I.err || I.u_size == 0) return;
+    const DecJob jb = jobs[f];
+    uint8_t* dst = out + jb.out_off;
+    const uint32_t u = I.u_size;
+    if (I.stored) {
+        const uint8_t* s = src + jb.src_off + 8;
+        for (uint32_t i = tid; i < u; i += kExThreads) dst[i] = s[i];
+        return;
+    }
+    const uint8_t* cs = reinterpret_cast<const uint8_t*>(I.cmd);
+    const uint8_t* ms = reinterpret_cast<const uint8_t*>(I.meta);
+    const uint8_t* vs = reinterpret_cast<const uint8_t*>(I.var);
+    const uint8_t* lit = reinterpret_cast<const uint8_t*>(I.lit);
+    const uint8_t* offs = reinterpret_cast<const uint8_t*>(I.off);
+    const uint32_t cl = I.cmd_len, ml = I.meta_len, vl = I.var_len, ll = I.lit_len, ol = I.off_len, bmin = I.bmin;
+    const bool split = I.cmd_mode == 1;
+    const uint32_t jlim = split ? I.cmd_orig : cl;
+    uint32_t cp = 0, mp = 0, vp = 0, j = 0, lp = 0, dp = 0, op0 = 0;
+    RepMap reps;
+    if ((I.flags & 0x01) && I.stride > 1) reps = RepMap{{1, I.stride, 2 * I.stride, 3 * I.stride}};
+    else reps = RepMap{{1, 4, 8, 16}};
+    for (;;) {
+        // the chunk's commands: the next 512 opcodes, or in a flat stream the
+        // commands that one thread finds in its next bytes
+        uint32_t n = min(kExThreads, cl - cp), at = cp + tid;
+        if (!split) {
+            for (uint32_t i = tid; i < kExFlat && cp + i < cl; i += kExThreads) S.flat[i] = cs[cp + i];
+            __syncthreads();
+            if (tid == 0) {
+                const uint32_t have = min(kExFlat, cl - cp);
+                uint32_t p = 0, k = 0;
+                while (k < kExThreads && p < have) {
+                    const uint32_t op = S.flat[p];
+                    S.pos[k++] = (uint16_t)p;
+                    p++;
+                    bool var = false;
+                    if (op < 0x80u || (op >= 0xF3u && op <= 0xFAu)) {
+                    } else if (op < 0xC0u) {
+                        var = (op & 15u) == 15u;
+                    } else if (op <= 0xC3u) {
+                        var = p < have && (S.flat[p] & 15u) == 15u;
+                        p++;
+                    } else if (op == 0xF0u || op == 0xF1u) {
+                        var = true;
+                    } else {
+                        break;  // ends the walk or leaves it to the serial kernel
+                    }
+                    for (uint32_t i = 0; var && i < 4; i++) var = p < have && (S.flat[p++] & 0x80u);
+                }
+                S.npos = k;
+                S.pos[k] = (uint16_t)p;
+            }
+            __syncthreads();
+            n = S.npos;
+            if (tid < n) at = cp + S.pos[tid];
+        }
+        uint32_t ev = EV_NONE, op = 0, m = 0, isvar = 0, isexp = 0, kind = 0, k = 0, llit = 0, lmatch = 0;
+        bool bad = false;
+        if (tid < n) {
+            op = cs[at];
+            if (op < 0x80u) {
+                llit = (op >> 4) & 7u; lmatch = ((op >> 2) & 3u) + bmin; k = op & 3u; kind = 1;
+            } else if (op < 0xC0u) {
+                llit = (op >> 4) & 3u; lmatch = (op & 15u) + bmin; kind = 3; isexp = 1; isvar = (op & 15u) == 15u;
+            } else if (op <= 0xC3u) {
+                m = 1; k = op & 3u; kind = 1;
+            } else if (op == 0xF0u || op == 0xF1u) {
+                isvar = 1; kind = op == 0xF0u ? 0 : 4;
+            } else if (op >= 0xF3u && op <= 0xFAu) {
+                llit = op - 0xF2u;
+            } else {
+                ev = op == 0xF2u || op >= 0xFBu ? EV_CORRUPT
+                     : op <= 0xCEu || (op >= 0xD0u && op <= 0xD7u) ? EV_SERIAL : EV_UNSUPPORTED;
+            }
+        }
+        // operands: tokens, then the varints that the opcodes and tokens ask for
+        uint32_t tot;
+        const uint32_t s1 = block_exclusive_scan<kExThreads>(m | (isexp << 16), S.warp, tot);
+        const uint32_t mi = s1 & 0xFFFFu, ei = s1 >> 16, nexp = tot >> 16;
+        const uint32_t mt = split ? mp + mi : at + 1;
+        if (m) {
+            uint32_t tok = 0;
+            if (mt < (split ? ml : cl)) tok = (split ? ms : cs)[mt];
+            else bad = true;
+            llit = tok >> 4; lmatch = (tok & 15u) + bmin; isvar = (tok & 15u) == 15u && !bad;
+        }
+        const uint32_t em = exec_ends(offs, op0, ol), vm = split ? exec_ends(vs, vp, vl) : 0u;
+        const uint32_t s2 = block_exclusive_scan<kExThreads>(__popc(vm) | (__popc(em) << 16), S.warp, tot);
+        const uint32_t nv = tot & 0xFFFFu, ne = tot >> 16;
+        exec_put_ends(S.vend, vm, s2 & 0xFFFFu);
+        exec_put_ends(S.oend, em, s2 >> 16);
+        const uint32_t vi = block_exclusive_scan<kExThreads>(isvar, S.warp, tot);  // (its barriers publish the ends)
+        uint32_t vlen = 0, vbefore = 0, vval = 0;
+        if (split) {
+            if (vi) vbefore = S.vend[vi - 1];
+            if (isvar) {
+                vlen = vi < nv ? (uint32_t)S.vend[vi] - vbefore : 5u;
+                if (vlen > 4) bad = true;
+                else vval = exec_varint(vs + vp + vbefore, vlen);
+            }
+        } else if (isvar) {
+            const uint32_t p = at + 1 + m;
+            vlen = 5;
+            for (uint32_t i = 0; i < 4; i++)
+                if (p + i < cl && cs[p + i] < 0x80u) { vlen = i + 1; break; }
+            if (vlen > 4) bad = true;
+            else vval = exec_varint(cs + p, vlen);
+        }
+        if (vval > kDecMaxBlock) bad = true;
+        if (isvar && !bad) {
+            if (kind == 0) llit = vval;
+            else if (kind == 4) lmatch = vval;
+            else lmatch += vval;
+        }
+        const uint32_t ji = split ? j + tid + mi + vbefore : at;
+        if (ji + 1 + m + vlen > jlim) bad = true;
+        bool badoff = false;
+        uint32_t d = 0;
+        if (isexp) {
+            const uint32_t b = ei ? S.oend[ei - 1] : 0u, len = ei < ne ? (uint32_t)S.oend[ei] - b : 5u;
+            if (len > 4) badoff = true;
+            else d = exec_varint(offs + op0 + b, len);
+            if (d > kDecMaxBlock) badoff = true;
+        }
+        // literals and output before the command
+        uint32_t li = llit + (kind == 4), oi = llit + (kind ? lmatch : 0u), tl, to;
+        if (tid >= n) li = oi = 0;
+        exec_scan2(li, oi, tl, to, S);
+        li += lp;
+        oi += dp;
+        // the repeat distances before it
+        RepMap own = rep_identity();
+        if (kind == 1) {
+            own.e[0] = kRepFrom | k;
+            if (k >= 1) own.e[1] = kRepFrom | 0u;
+            if (k >= 2) own.e[2] = kRepFrom | 1u;
+            if (k >= 3) own.e[3] = kRepFrom | 2u;
+        } else if (kind == 3) {
+            own = RepMap{{d, kRepFrom | 0u, kRepFrom | 1u, kRepFrom | 2u}};
+        }
+        RepMap inc = own;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            RepMap a;
+#pragma unroll
+            for (int i = 0; i < 4; i++) a.e[i] = __shfl_up_sync(0xFFFFFFFFu, inc.e[i], o);
+            if (lane >= (uint32_t)o) inc = rep_then(a, inc);
+        }
+        if (lane == 31) {
+#pragma unroll
+            for (int i = 0; i < 4; i++) S.rep[warp][i] = inc.e[i];
+        }
+        RepMap before;
+#pragma unroll
+        for (int i = 0; i < 4; i++) before.e[i] = __shfl_up_sync(0xFFFFFFFFu, inc.e[i], 1);
+        if (lane == 0) before = rep_identity();
+        if (tid == 0) S.event = 0xFFFFFFFFu;
+        __syncthreads();
+        RepMap base = reps, all = reps;
+        for (uint32_t w = 0; w < kExThreads / 32; w++) {
+            if (w == warp) base = all;
+            all = rep_then(all, RepMap{{S.rep[w][0], S.rep[w][1], S.rep[w][2], S.rep[w][3]}});
+        }
+        if (kind == 1) d = rep_of(base, rep_of(before, kRepFrom | k));
+        // how the walk fares at this command
+        if (tid > n) {
+            ev = EV_NONE;
+        } else if (tid == n) {
+            ev = EV_BEFORE;  // the commands end here (a full chunk has no such thread)
+        } else if (oi >= u || ji >= jlim) {
+            ev = EV_BEFORE;
+        } else if (ev != EV_NONE) {
+        } else if (bad) {
+            ev = EV_CORRUPT;
+        } else if (kind == 4) {
+            if (li >= ll || oi + lmatch > u) ev = EV_CORRUPT;
+        } else if (li + llit > ll || oi + llit > u) {
+            ev = EV_CORRUPT;
+        } else if (kind) {
+            const uint32_t b = oi + llit;
+            if (b == u) ev = EV_AFTER;
+            else if (badoff || d == 0 || d > b || b + lmatch > u) ev = EV_CORRUPT;
+        }
+        if (ev != EV_NONE) atomicMin(&S.event, (tid << 4) | ev);
+        __syncthreads();
+        const uint32_t first = S.event, e = first == 0xFFFFFFFFu ? n : first >> 4, type = first == 0xFFFFFFFFu ? (uint32_t)EV_NONE : first & 15u;
+        if (type == EV_SERIAL) {
+            if (tid == 0) infos[f].serial = 1;
+            return;
+        }
+        if (type == EV_CORRUPT || type == EV_UNSUPPORTED) {
+            if (tid == 0) dec_fail(infos, f, type == EV_CORRUPT ? D_CORRUPT : D_UNSUPPORTED);
+            return;
+        }
+        const uint32_t E = type == EV_AFTER ? e + 1 : e;
+        if (tid < E) {
+            S.start[tid] = oi;
+            S.lend[tid] = kind == 4 ? oi : oi + llit;
+            S.lsrc[tid] = li;
+            S.dist[tid] = kind == 4 ? 0u : d;
+        }
+        // the state at the walk's end, or after the chunk
+        if (type == EV_NONE ? tid == n - 1 : tid == e) {
+            const bool past = type != EV_BEFORE;
+            S.st[0] = split ? cp + tid + past : 0u;
+            S.st[1] = mp + mi + (past ? m : 0u);
+            S.st[2] = vp + vbefore + (past ? vlen : 0u);
+            S.st[3] = ji + (past ? 1 + m + vlen : 0u);
+            S.st[4] = li + (past ? llit + (kind == 4) : 0u);
+            S.st[5] = type == EV_NONE ? oi + llit + (kind ? lmatch : 0u) : type == EV_AFTER ? oi + llit : oi;
+            S.start[E] = S.st[5];
+        }
+        __syncthreads();
+        const uint32_t end = S.st[5];
+        exec_copy(S, dst, lit, dp, end, E);
+        if (type != EV_NONE) {
+            if (tid == 0) {
+                uint32_t err = end == u ? D_OK : D_CORRUPT;
+                if (!err && split) {
+                    CmdReader R;
+                    R.c = cs;
+                    R.m = ms;
+                    R.v = vs;
+                    R.cl = cl;
+                    R.ml = ml;
+                    R.vl = vl;
+                    R.cp = S.st[0];
+                    R.mp = S.st[1];
+                    R.vp = S.st[2];
+                    R.j = S.st[3];
+                    R.jlim = jlim;
+                    R.split = true;
+                    err = exec_rest(R);
+                }
+                if (err) dec_fail(infos, f, err);
+            }
+            return;
+        }
+        mp = S.st[1];
+        vp = S.st[2];
+        j = S.st[3];
+        lp = S.st[4];
+        dp = end;
+        cp = split ? S.st[0] : cp + S.pos[n];
+        op0 += nexp ? S.oend[nexp - 1] : 0u;
+        reps = all;
+        __syncthreads();  // the next chunk rewrites the shared state
+    }
+}
+
+}  // namespace pz
