@@ -519,158 +519,22 @@ __global__ void __launch_bounds__(32) k_dec_static(const DecTask* __restrict__ t
     if (!ok) dec_fail(infos, t.frame, D_CORRUPT);
 }
 
-// Decode-table entry of slot j of symbol s (frequency f): s | j << 8 |
-// (f - 1) << 20, so x' = f (x >> 12) + j is ((e >> 20) + 1) (x >> 12) +
-// ((e >> 8) & 0xFFF) (the rANS decode step, przm_dec.c:187-199).
-__host__ __device__ inline uint32_t dec_entry(uint32_t f, uint32_t j, uint32_t s) { return ((f - 1) << 20) | (j << 8) | s; }
+// Decode-table entry of slot j of symbol s (frequency f): f - 1 | s << 12 |
+// j << 20, so x' = f (x >> 12) + j is (e & 0xFFF) u + ((e >> 20) + u) with u =
+// x >> 12 (the rANS decode step, przm_dec.c:187-199).
+__host__ __device__ inline uint32_t dec_entry(uint32_t f, uint32_t j, uint32_t s) { return (f - 1) | (s << 12) | (j << 20); }
 __device__ __forceinline__ uint32_t dec_next(uint32_t x, uint32_t e) {
-    return ((e >> 20) + 1) * (x >> 12) + ((e >> 8) & 0xFFFu);
+    const uint32_t u = x >> 12;
+    return (e & 0xFFFu) * u + ((e >> 20) + u);
 }
+__device__ __forceinline__ uint32_t dec_sym(uint32_t e) { return (e >> 12) & 0xFFu; }
 
-// One round of an adaptive body on lanes 0-3 (lane l: state l, stream
-// pointer p in every lane): the lane's symbol (returned with its table
-// entry) and its state renormalised.  The round's eight stream bytes come
-// from three aligned words (below p + 12; the caller keeps p + 16 <= the
-// stream's length).  A state needs 0, 1 or 2 bytes (x < 2^16, x < 2^8
-// after the step, the reference's loop); two ballots of those tests give
-// every lane all four counts, hence its offset o (the bytes of the lanes
-// before it) and the pointer's advance.  One byte permute puts bytes o,
-// o + 1 in the low half of y, a second shifts them into x.
-__device__ __forceinline__ uint32_t dec_round(const uint32_t* tab, uintptr_t sa, uint32_t lt, uint32_t& x,
-                                              uint32_t& p) {
-    const uint32_t* w = reinterpret_cast<const uint32_t*>((sa + p) & ~uintptr_t(3));
-    const uint32_t sh = 8u * (uint32_t)((sa + p) & 3u);
-    const uint32_t w0 = w[0], w1 = w[1], w2 = w[2];
-    const uint32_t lo = __funnelshift_r(w0, w1, sh), hi = __funnelshift_r(w1, w2, sh);
-    const uint32_t e = tab[x & 4095];
-    x = dec_next(x, e);
-    const bool r1 = x < 65536u, r2 = x < 256u;
-    const uint32_t b1 = __ballot_sync(0xFu, r1), b2 = __ballot_sync(0xFu, r2);
-    const uint32_t o = __popc(b1 & lt) + __popc(b2 & lt);
-    const uint32_t y = __byte_perm(lo, hi, 17u * o + 16u);  // byte 0: stream byte o, byte 1: byte o + 1
-    x = __byte_perm(x, y, r2 ? 0x1045u : (r1 ? 0x2104u : 0x3210u));  // (x << 16 | o, o + 1), (x << 8 | o), x
-    p += __popc(b1) + __popc(b2);
-    return e;
-}
-
-// One adaptive body per warp (task slot blockIdx.x; other kinds return at
-// once), for batches whose bodies all fit on the SMs at once: the warp builds
-// a 4096-entry table (s | j << 8 | (f - 1) << 20 per slot, one shared load
-// per step), lanes 0-3 run the body's four states.  Its rounds are the
-// shortest of the two adaptive kernels; k_dec_adaptive trades them for eight
-// bodies per warp when there are many.
-constexpr uint32_t kDecAdaptive1Smem = 4096 * 4 + 256 * 2;
-__global__ void __launch_bounds__(32) k_dec_adaptive1(const DecTask* __restrict__ tasks, DecInfo* __restrict__ infos) {
-    extern __shared__ __align__(16) uint8_t smem_d[];
-    uint32_t* tab = reinterpret_cast<uint32_t*>(smem_d);
-    uint16_t* freq = reinterpret_cast<uint16_t*>(smem_d + 4096 * 4);
-    const DecTask t = tasks[blockIdx.x];
-    const uint32_t lane = threadIdx.x;
-    if (t.kind != DT_ADAPTIVE || t.n == 0) return;
-    const uint8_t* s = reinterpret_cast<const uint8_t*>(t.src);
-    uint8_t* dst = reinterpret_cast<uint8_t*>(t.dst);
-    const uint32_t n = t.n, slen = t.slen;
-    for (uint32_t i = lane; i < 256; i += 32) freq[i] = 0;
-    __syncwarp();
-    uint32_t p = 0;
-    if (lane == 0) p = dec_matrix(s, slen, freq);
-    p = __shfl_sync(0xFFFFFFFFu, p, 0);
-    if (p == 0 || p + 16 > slen) {
-        if (lane == 0) dec_fail(infos, t.frame, D_CORRUPT);
-        return;
-    }
-    __syncwarp();
-    // decode table: lane l takes symbols 8l .. 8l + 7
-    uint32_t f8[8], loc = 0;
-#pragma unroll
-    for (int k = 0; k < 8; k++) { f8[k] = freq[lane * 8 + k]; loc += f8[k]; }
-    uint32_t x = loc;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, x, o);
-        if (lane >= (uint32_t)o) x += y;
-    }
-    uint32_t c = x - loc;
-    for (int k = 0; k < 8; k++) {
-        for (uint32_t j = 0; j < f8[k]; j++) tab[c + j] = dec_entry(f8[k], j, lane * 8 + k);
-        c += f8[k];
-    }
-    __syncwarp();
-    if (lane >= 4) return;
-    // lane l holds state l (the state of symbols l, l + 4, ...)
-    uint32_t xl = drd32(s + p + 4 * lane);
-    p += 16;
-    uint32_t i = 0;
-    bool ok = true;
-    if (__all_sync(0xFu, xl >= 65536u)) {
-        // Rounds of four symbols, one per lane: each lane's byte count
-        // comes from its own state; two ballots give every lane all four,
-        // hence its offset in the round's 8 bytes and the stream's
-        // advance, so only the stream position links one round to the
-        // next.
-        const uintptr_t sa = reinterpret_cast<uintptr_t>(s);
-        const uint32_t lt = (1u << lane) - 1u;
-        uint8_t* dl = dst + lane;
-        for (; i + 8 <= n && p + 24 <= slen; i += 8) {  // two rounds per trip
-            dl[i] = (uint8_t)dec_round(tab, sa, lt, xl, p);
-            dl[i + 4] = (uint8_t)dec_round(tab, sa, lt, xl, p);
-        }
-        for (; i + 4 <= n && p + 16 <= slen; i += 4) dl[i] = (uint8_t)dec_round(tab, sa, lt, xl, p);
-    }
-    uint32_t x0 = __shfl_sync(0xFu, xl, 0), x1 = __shfl_sync(0xFu, xl, 1), x2 = __shfl_sync(0xFu, xl, 2),
-             x3 = __shfl_sync(0xFu, xl, 3);
-    if (lane != 0) return;
-    // the rest (the stream's last 16 bytes, or initial states below 2^16)
-    // byte by byte
-    ByteWin bw;
-    bw.init(s, slen, p);
-    bw.prefetch();
-    for (; i + 4 <= n && ok; i += 4) {  // vans_run_4x_loop, przm_dec.c:201-255
-        bw.step();
-        const uint32_t e0 = tab[x0 & 4095], e1 = tab[x1 & 4095], e2 = tab[x2 & 4095], e3 = tab[x3 & 4095];
-        x0 = dec_next(x0, e0);
-        x1 = dec_next(x1, e1);
-        x2 = dec_next(x2, e2);
-        x3 = dec_next(x3, e3);
-        ok = bw.renorm(x0) && bw.renorm(x1) && bw.renorm(x2) && bw.renorm(x3);
-        dst[i] = (uint8_t)e0;
-        dst[i + 1] = (uint8_t)e1;
-        dst[i + 2] = (uint8_t)e2;
-        dst[i + 3] = (uint8_t)e3;
-    }
-    uint32_t xs[4] = {x0, x1, x2, x3};
-    for (; i < n && ok; i++) {
-        bw.step();
-        const uint32_t e = tab[xs[i & 3] & 4095];
-        dst[i] = (uint8_t)e;
-        xs[i & 3] = dec_next(xs[i & 3], e);
-        ok = bw.renorm(xs[i & 3]);
-    }
-    if (!ok) dec_fail(infos, t.frame, D_CORRUPT);
-}
-
-// Adaptive bodies, eight per warp: lane group g (lanes 4g .. 4g + 3) of
-// block b decodes task list[8 b + g], lane 4g + l holding state l.  The warp
-// builds the eight models one after another (per model the symbol of every
-// slot and (f - 1) << 20 | cumulative frequency per symbol, 5 KiB), then all
-// groups run their rounds together, so one warp instruction advances eight
-// chains; the list is sorted by length (k_dec_lists), so a warp's chains
-// end close together.
-constexpr uint32_t kDecGroups = 8;
-// Batches of up to this many frames decode their adaptive bodies one per
-// warp (k_dec_adaptive1): at 13 such warps per SM their bodies all run at
-// once.  Measured on 1 MiB frames: 128 frames 29.4 ms one per warp against
-// 67 ms eight per warp; 2560 frames 89 ms (whole decode) eight per warp
-// against 97 ms.
-constexpr uint32_t kDecOneWarpFrames = 512;
-constexpr uint32_t kDecModel = 4096 + 256 * 4;
-constexpr uint32_t kDecAdaptiveSmem = kDecGroups * kDecModel + 256 * 2 + kDecGroups * 4;
-
-// The decoded state after symbol slot x & 4095 with model word g = (f - 1)
-// << 20 | cumulative frequency: f (x >> 12) + (x & 4095) - cum (the rANS
-// decode step, przm_dec.c:187-199).
-__device__ __forceinline__ uint32_t dec_step(uint32_t x, uint32_t g) {
-    return ((g >> 20) + 1) * (x >> 12) + (x & 4095u) - (g & 0xFFFFFu);
+// Byte permute with the whole selector (the intrinsic drops bit 3 of its
+// nibbles, which replicates a byte's sign).
+__device__ __forceinline__ uint32_t dec_pick(uint32_t a, uint32_t b, uint32_t sel) {
+    uint32_t d;
+    asm("prmt.b32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(sel));
+    return d;
 }
 
 // The adaptive tasks of the slots, longest first by bit length of their
@@ -699,6 +563,198 @@ __global__ void __launch_bounds__(1024) k_dec_lists(const DecTask* __restrict__ 
         const DecTask t = tasks[i];
         if (t.kind == DT_ADAPTIVE && t.n) list[4 + atomicAdd(&s_off[31 - __clz(t.n)], 1u)] = i;
     }
+}
+
+// One adaptive body per warp (entry blockIdx.x of the list, longest first: the
+// long bodies then start on different SMs; taken by task slot, those of 128
+// frames shared 37 SMs), for batches whose bodies all fit on the SMs at once;
+// k_dec_adaptive takes eight bodies per warp when there are many.  The body's four states
+// are held by eight lanes each (a branch around 28 idle lanes would cost each
+// vote a convergence check), which run up to 64 rounds of four symbols at a
+// time; then the lanes turn the rounds' slots into symbols, write them, and
+// put the next stream bytes into the ring (their loads in flight since the
+// rounds before).  A state needs 0, 1 or 2 bytes (x < 2^16, x < 2^8 after the
+// step, the reference's loop), in the order of the states.  Two ballots of
+// those tests give every lane the counts; its offset in the round's eight
+// bytes is looked up with a byte permute of a nibble of the ballot, which is
+// a third of a population count's latency.  Bound by the chain of a round: 94
+// cycles by the instructions' latencies (table load 25, step 12, compare and
+// vote 17, byte selection 28, address 8), 100 in a one-warp loop, against 177
+// there with the stream read from global memory, a symbol stored each round
+// and population counts (27.4 ms for 128 mixed frames of 1 MiB).  Tried in
+// that loop: thresholds for the votes beside the table entry (8 bytes an
+// entry) 124, all offsets of a state tried on eight lanes and the right one
+// shuffled in 178, the four states in one thread 215.
+constexpr uint32_t kDecRing = 2048, kDecRounds = 64;
+struct Dec1Shared {
+    uint32_t tab[4096];
+    uint32_t ring[kDecRing / 4 + 4];  // stream bytes by position mod kDecRing, the first 16 again at the end
+    uint16_t slot[4 * kDecRounds];    // 4 x the slots of the rounds' symbols
+    uint16_t freq[256];
+};
+// R rounds (kFull: kDecRounds of them, unrolled) from ring position q, state x
+// of this lane; returns the position after them.
+template <bool kFull>
+__device__ __forceinline__ uint32_t dec1_rounds(Dec1Shared& S, uint32_t& x, uint32_t q, uint32_t R) {
+    const uint32_t l = threadIdx.x & 3u, below = ((1u << l) - 1u) << 4;
+    const uint8_t* ring = reinterpret_cast<const uint8_t*>(S.ring);
+    uint16_t* so = S.slot + l;
+#pragma unroll(kFull ? 8 : 1)
+    for (uint32_t r = 0; r < (kFull ? kDecRounds : R); r++) {
+        const uint32_t* w = reinterpret_cast<const uint32_t*>(ring + (q & (kDecRing - 4)));
+        const uint32_t w0 = w[0], w1 = w[1], w2 = w[2], sh = 8u * q;
+        const uint32_t lo = __funnelshift_r(w0, w1, sh), hi = __funnelshift_r(w1, w2, sh);
+        const uint32_t at = (x << 2) & 0x3FFCu;
+        const uint32_t e = *reinterpret_cast<const uint32_t*>(reinterpret_cast<const uint8_t*>(S.tab) + at);
+        x = dec_next(x, e);
+        const bool r1 = x < 65536u, r2 = x < 256u;
+        const uint32_t b1 = __ballot_sync(0xFFFFFFFFu, r1), b2 = __ballot_sync(0xFFFFFFFFu, r2);
+        so[4 * r] = (uint16_t)at;  // the eight lanes of a state alike
+        // 17 times the states below that take a byte, and a second one, in
+        // the second byte: the offset in its two nibbles
+        const uint32_t o = dec_pick(0x22111100u, 0x33222211u, b1 & below) +
+                           dec_pick(0x22111100u, 0x33222211u, b2 & below) + 0x0100u;
+        const uint32_t y = dec_pick(lo, hi, o);  // top bytes: stream bytes o, o + 1
+        x = __funnelshift_l(y, x, r2 ? 16u : (r1 ? 8u : 0u));
+        q += (uint32_t)(__popc(b1) + __popc(b2)) >> 3;
+    }
+    return q;
+}
+
+__global__ void __launch_bounds__(32) k_dec_adaptive1(const DecTask* __restrict__ tasks, const uint32_t* __restrict__ list,
+                                                      DecInfo* __restrict__ infos) {
+    __shared__ __align__(16) Dec1Shared S;
+    if (blockIdx.x >= list[0]) return;
+    const DecTask t = tasks[list[4 + blockIdx.x]];
+    const uint32_t lane = threadIdx.x;
+    const uint8_t* s = reinterpret_cast<const uint8_t*>(t.src);
+    uint8_t* dst = reinterpret_cast<uint8_t*>(t.dst);
+    const uint32_t n = t.n, slen = t.slen;
+    for (uint32_t i = lane; i < 256; i += 32) S.freq[i] = 0;
+    __syncwarp();
+    uint32_t p = 0;
+    if (lane == 0) p = dec_matrix(s, slen, S.freq);
+    p = __shfl_sync(0xFFFFFFFFu, p, 0);
+    if (p == 0 || p + 16 > slen) {
+        if (lane == 0) dec_fail(infos, t.frame, D_CORRUPT);
+        return;
+    }
+    __syncwarp();
+    // decode table: lane l takes symbols 8l .. 8l + 7
+    uint32_t f8[8], loc = 0;
+#pragma unroll
+    for (int k = 0; k < 8; k++) { f8[k] = S.freq[lane * 8 + k]; loc += f8[k]; }
+    uint32_t x = loc;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, x, o);
+        if (lane >= (uint32_t)o) x += y;
+    }
+    uint32_t c = x - loc;
+    for (int k = 0; k < 8; k++) {
+        for (uint32_t j = 0; j < f8[k]; j++) S.tab[c + j] = dec_entry(f8[k], j, lane * 8 + k);
+        c += f8[k];
+    }
+    const uint32_t l = lane & 3;
+    x = drd32(s + p + 4 * l);  // lanes l, l + 4, ...: state l (of symbols l, l + 4, ...)
+    p += 16;
+    uint32_t i = 0;
+    if (__all_sync(0xFFFFFFFFu, x >= 65536u)) {
+        // ring position q of stream byte p: p + a, a the stream's place in its 16-byte unit
+        const uint32_t a = (uint32_t)(reinterpret_cast<uintptr_t>(s) & 15u);
+        const uint8_t* s16 = s - a;
+        uint32_t loaded = (p + a) & ~15u;
+        auto fetch = [&](uint32_t at) {  // 16-byte units that hold stream bytes
+            const uint32_t q = at + 16 * lane;
+            return q < slen + a ? *reinterpret_cast<const uint4*>(s16 + q) : make_uint4(0, 0, 0, 0);
+        };
+        uint4 nx = fetch(loaded);
+        while (i + 4 <= n && p + 16 <= slen) {
+            while (loaded < p + a + 8 * kDecRounds + 16) {
+                const uint32_t q = (loaded + 16 * lane) & (kDecRing - 1);
+                *reinterpret_cast<uint4*>(&S.ring[q / 4]) = nx;
+                if (q == 0) *reinterpret_cast<uint4*>(&S.ring[kDecRing / 4]) = nx;
+                loaded += 512;
+                nx = fetch(loaded);
+            }
+            __syncwarp();
+            // a round takes at most eight bytes and starts 16 before the stream's end
+            const uint32_t R = min(min(kDecRounds, (n - i) / 4), (slen - 16 - p) / 8 + 1);
+            p = (R == kDecRounds ? dec1_rounds<true>(S, x, p + a, R) : dec1_rounds<false>(S, x, p + a, R)) - a;
+            __syncwarp();
+            // symbols 8 lane .. 8 lane + 7 of the R rounds
+            const uint4 q8 = reinterpret_cast<const uint4*>(S.slot)[lane];
+            const uint32_t qs[4] = {q8.x, q8.y, q8.z, q8.w};
+            uint32_t o2[2] = {0, 0};
+#pragma unroll
+            for (int k = 0; k < 8; k++) {
+                const uint32_t at = (qs[k >> 1] >> (16 * (k & 1))) & 0x3FFCu;
+                o2[k >> 2] |= dec_sym(S.tab[at >> 2]) << (8 * (k & 3));
+            }
+            uint8_t* d8 = dst + i + 8 * lane;
+            const uint32_t have = 4 * R > 8 * lane ? min(8u, 4 * R - 8 * lane) : 0u;
+            if (have == 8 && (reinterpret_cast<uintptr_t>(d8) & 7u) == 0) {
+                *reinterpret_cast<uint2*>(d8) = make_uint2(o2[0], o2[1]);
+            } else {
+                for (uint32_t k = 0; k < have; k++) d8[k] = (uint8_t)(o2[k >> 2] >> (8 * (k & 3)));
+            }
+            i += 4 * R;
+            __syncwarp();
+        }
+    }
+    uint32_t xs[4];
+#pragma unroll
+    for (int k = 0; k < 4; k++) xs[k] = __shfl_sync(0xFFFFFFFFu, x, k);
+    if (lane != 0) return;
+    // the rest (the stream's last 16 bytes, or initial states below 2^16)
+    // byte by byte, with bytes taken after every four symbols
+    // (vans_run_4x_loop, przm_dec.c:201-255), then after each
+    bool ok = true;
+    ByteWin bw;
+    bw.init(s, slen, p);
+    bw.prefetch();
+    for (; i + 4 <= n && ok; i += 4) {
+        bw.step();
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            const uint32_t e = S.tab[xs[k] & 4095];
+            dst[i + k] = (uint8_t)dec_sym(e);
+            xs[k] = dec_next(xs[k], e);
+        }
+        ok = bw.renorm(xs[0]) && bw.renorm(xs[1]) && bw.renorm(xs[2]) && bw.renorm(xs[3]);
+    }
+    for (int k = 0; i < n && ok; i++, k++) {
+        bw.step();
+        const uint32_t x0 = k == 0 ? xs[0] : k == 1 ? xs[1] : xs[2], e = S.tab[x0 & 4095];
+        dst[i] = (uint8_t)dec_sym(e);
+        uint32_t xn = dec_next(x0, e);
+        ok = bw.renorm(xn);
+    }
+    if (!ok) dec_fail(infos, t.frame, D_CORRUPT);
+}
+
+// Adaptive bodies, eight per warp: lane group g (lanes 4g .. 4g + 3) of
+// block b decodes task list[8 b + g], lane 4g + l holding state l.  The warp
+// builds the eight models one after another (per model the symbol of every
+// slot and (f - 1) << 20 | cumulative frequency per symbol, 5 KiB), then all
+// groups run their rounds together, so one warp instruction advances eight
+// chains; the list is sorted by length (k_dec_lists), so a warp's chains
+// end close together.
+constexpr uint32_t kDecGroups = 8;
+// Batches of up to this many frames decode their adaptive bodies one per
+// warp (k_dec_adaptive1): at 13 such warps per SM their bodies all run at
+// once.  Measured on 1 MiB frames: 128 frames 29.4 ms one per warp against
+// 67 ms eight per warp; 2560 frames 89 ms (whole decode) eight per warp
+// against 97 ms.
+constexpr uint32_t kDecOneWarpFrames = 512;
+constexpr uint32_t kDecModel = 4096 + 256 * 4;
+constexpr uint32_t kDecAdaptiveSmem = kDecGroups * kDecModel + 256 * 2 + kDecGroups * 4;
+
+// The decoded state after symbol slot x & 4095 with model word g = (f - 1)
+// << 20 | cumulative frequency: f (x >> 12) + (x & 4095) - cum (the rANS
+// decode step, przm_dec.c:187-199).
+__device__ __forceinline__ uint32_t dec_step(uint32_t x, uint32_t g) {
+    return ((g >> 20) + 1) * (x >> 12) + (x & 4095u) - (g & 0xFFFFFu);
 }
 
 __global__ void __launch_bounds__(32) k_dec_adaptive(const DecTask* __restrict__ tasks, const uint32_t* __restrict__ list,
@@ -936,14 +992,9 @@ struct ShShared {
     uint32_t done, bad;
     ClassLut lut;
 };
-// Byte permute with the sign-replicating selectors (bit 3 of a nibble), and
-// the selector of the f-th 16-bit field of two registers, zero-extended as
-// every field is below 2^15.
-__device__ __forceinline__ uint32_t sh_pick(uint32_t a, uint32_t b, uint32_t sel) {
-    uint32_t d;
-    asm("prmt.b32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(sel));
-    return d;
-}
+// Selector of the f-th 16-bit field of two registers, zero-extended: the
+// upper bytes replicate the field's sign (bit 3 of a nibble), and every field
+// is below 2^15.
 __device__ __forceinline__ uint32_t sh_sel(uint32_t f) { return 0x9910u + 0x2222u * f; }
 
 // Positions [at, at + 256) of fiber k into the rings (positions past its
@@ -1072,7 +1123,7 @@ __global__ void __launch_bounds__(64) k_dec_sheaf(DecInfo* __restrict__ infos) {
                 const uint8_t* pi = reinterpret_cast<const uint8_t*>(S.info);
 #pragma unroll 8
                 for (uint32_t v = 0; v < kShVisits; v++) {
-                    const uint32_t at = sh_pick(C0, C1, sel);
+                    const uint32_t at = dec_pick(C0, C1, sel);
                     sel = *reinterpret_cast<const uint16_t*>(ps + at);
                     const uint32_t in = *reinterpret_cast<const uint16_t*>(pi + at), c = in & 0xFFu;
                     const uint32_t t = (2 * c) << (16 * (f & 1u));

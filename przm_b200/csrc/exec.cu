@@ -41,7 +41,8 @@ struct ExecShared {
     uint16_t vend[kExThreads], oend[kExThreads];  // ends of the chunk's varints in their windows
     __align__(16) uint16_t w[kExTile];            // a tile's bytes: 0x8000 | byte, or a place in the tile
     uint32_t warp[32], warp2[32];
-    uint32_t rep[kExThreads / 32][4];
+    uint32_t rep[kExThreads / 32 + 1][4];
+    uint32_t vwin[kExThreads], owin[kExThreads];  // the bytes of the chunk's varints
     uint16_t pos[kExThreads + 1];  // flat: where the chunk's commands start
     uint32_t npos;
     __align__(16) uint8_t flat[kExFlat + 16];
@@ -108,20 +109,26 @@ __device__ __forceinline__ RepMap rep_identity() {
 // Varint of len (1-4) bytes at p.
 __device__ __forceinline__ uint32_t exec_varint(const uint8_t* p, uint32_t len) {
     uint32_t r = 0;
-    for (uint32_t i = 0; i < len; i++) r |= (uint32_t)(p[i] & 0x7Fu) << (7 * i);
+#pragma unroll
+    for (uint32_t i = 0; i < 4; i++)
+        if (i < len) r |= (uint32_t)(p[i] & 0x7Fu) << (7 * i);
     return r;
 }
 
-// Ends of the varints in the 2048 bytes of s[at, n) (bit masks of this
-// thread's four bytes that end one).
-__device__ __forceinline__ uint32_t exec_ends(const uint8_t* s, uint32_t at, uint32_t n) {
-    uint32_t m = 0;
-#pragma unroll
-    for (uint32_t i = 0; i < 4; i++) {
-        const uint32_t p = at + 4 * threadIdx.x + i;
-        if (p < n && s[p] < 0x80u) m |= 1u << i;
+// Bytes [at + 4 tid, ...+ 4) of s[0, n), 0x80 past its end, into win: which of
+// them end a varint.
+__device__ __forceinline__ uint32_t exec_window(const uint8_t* s, uint32_t at, uint32_t n, uint32_t* win) {
+    const uint32_t p = at + 4 * threadIdx.x;
+    uint32_t w = 0x80808080u, m = 0;
+    if (p + 4 <= n) {
+        w = (uint32_t)s[p] | ((uint32_t)s[p + 1] << 8) | ((uint32_t)s[p + 2] << 16) | ((uint32_t)s[p + 3] << 24);
+    } else {
+        for (uint32_t i = 0; p + i < n; i++) w ^= (0x80u ^ s[p + i]) << (8 * i);
     }
-    return m;
+    win[threadIdx.x] = w;
+#pragma unroll
+    for (uint32_t i = 0; i < 4; i++) m |= ((w >> (8 * i + 7)) & 1u) << i;
+    return m ^ 15u;
 }
 __device__ __forceinline__ void exec_put_ends(uint16_t* ends, uint32_t m, uint32_t k) {
 #pragma unroll
@@ -141,9 +148,10 @@ __device__ void exec_copy(ExecShared& S, uint8_t* dst, const uint8_t* __restrict
          tb += kExTile) {
         const int32_t lo = max(tb, (int32_t)dp), hi = min(tb + (int32_t)kExTile, (int32_t)end);
         const int32_t p0 = tb + (int32_t)(kExPer * tid);
+        const bool any = p0 < hi && p0 + (int32_t)kExPer > lo;
         uint32_t v[kExPer];
         uint32_t open = 0;  // own bytes that still point into the tile
-        if (p0 < hi && p0 + (int32_t)kExPer > lo) {
+        if (any) {
             const uint32_t pf = (uint32_t)max(p0, lo);
             uint32_t a = 0, b = E;  // the last command that starts at or before pf
             while (b - a > 1) {
@@ -152,34 +160,67 @@ __device__ void exec_copy(ExecShared& S, uint8_t* dst, const uint8_t* __restrict
                 else b = m;
             }
             uint32_t c = a, cs = S.start[c], cn = S.start[c + 1], le = S.lend[c], ls = S.lsrc[c], d = S.dist[c];
+            const uint32_t pl = (uint32_t)p0 + kExPer - 1;  // (when all the bytes are this tile's)
+            const bool whole = p0 >= lo && p0 + (int32_t)kExPer <= hi && pl < cn;
+            const uint8_t* from = nullptr;  // eight bytes in a row, literals or from before the tile
+            if (whole && pl < le) from = lit + ls + ((uint32_t)p0 - cs);
+            else if (whole && (uint32_t)p0 >= le && pl - le < d && (int32_t)(pl - d) < lo) from = dst + ((uint32_t)p0 - d);
+            if (from) {
+                const uint32_t* q = reinterpret_cast<const uint32_t*>(reinterpret_cast<uintptr_t>(from) & ~uintptr_t(3));
+                const uint32_t sh = 8u * (uint32_t)(reinterpret_cast<uintptr_t>(from) & 3u);
+                const uint32_t r0 = q[0], r1 = q[1], r2 = sh ? q[2] : 0u;  // words that hold one of them
+                const uint32_t x0 = __funnelshift_r(r0, r1, sh), x1 = __funnelshift_r(r1, r2, sh);
 #pragma unroll
-            for (uint32_t i = 0; i < kExPer; i++) {
-                const int32_t p = p0 + (int32_t)i;
-                v[i] = 0x8000u;
-                if (p < lo || p >= hi) continue;
-                while ((uint32_t)p >= cn) {
-                    c++;
-                    cs = cn;
-                    cn = S.start[c + 1];
-                    le = S.lend[c];
-                    ls = S.lsrc[c];
-                    d = S.dist[c];
-                }
-                if ((uint32_t)p < le) {
-                    v[i] = 0x8000u | lit[ls + ((uint32_t)p - cs)];
-                } else if (d == 0) {
-                    v[i] = 0x8000u | lit[ls];
-                } else {
-                    uint32_t o = (uint32_t)p - le;
-                    if (o >= d) o %= d;  // a match closer than its length repeats
-                    const int32_t s = (int32_t)(le - d + o);
-                    if (s < lo) {
-                        v[i] = 0x8000u | dst[s];
+                for (uint32_t i = 0; i < kExPer; i++)
+                    v[i] = 0x8000u | (((i < 4 ? x0 : x1) >> (8 * (i & 3))) & 0xFFu);
+            } else {
+                // every byte's place first (a match closer than its length
+                // repeats: mo counts modulo d), then the loads side by side
+                const uint8_t* at[kExPer];
+                uint32_t load = 0, mo = 0;
+                auto enter = [&](uint32_t p) {  // byte p of command c
+                    mo = p > le ? p - le : 0u;
+                    if (mo >= d && d) mo %= d;
+                };
+                enter(pf);
+#pragma unroll
+                for (uint32_t i = 0; i < kExPer; i++) {
+                    const int32_t p = p0 + (int32_t)i;
+                    v[i] = 0x8000u;
+                    at[i] = dst;
+                    if (p < lo || p >= hi) continue;
+                    if ((uint32_t)p >= cn) {
+                        do {
+                            c++;
+                            cn = S.start[c + 1];
+                        } while ((uint32_t)p >= cn);
+                        cs = S.start[c];
+                        le = S.lend[c];
+                        ls = S.lsrc[c];
+                        d = S.dist[c];
+                        enter((uint32_t)p);
+                    }
+                    if ((uint32_t)p < le) {
+                        at[i] = lit + (ls + ((uint32_t)p - cs));
+                        load |= 1u << i;
+                    } else if (d == 0) {
+                        at[i] = lit + ls;
+                        load |= 1u << i;
                     } else {
-                        v[i] = (uint32_t)(s - tb);
-                        open |= 1u << i;
+                        const int32_t s = (int32_t)(le - d + mo);
+                        mo = mo + 1 == d ? 0u : mo + 1;
+                        at[i] = dst + s;
+                        if (s < lo) {
+                            load |= 1u << i;
+                        } else {
+                            v[i] = (uint32_t)(s - tb);
+                            open |= 1u << i;
+                        }
                     }
                 }
+#pragma unroll
+                for (uint32_t i = 0; i < kExPer; i++)
+                    if ((load >> i) & 1u) v[i] = 0x8000u | *at[i];
             }
             *reinterpret_cast<uint4*>(&S.w[kExPer * tid]) =
                 make_uint4(v[0] | (v[1] << 16), v[2] | (v[3] << 16), v[4] | (v[5] << 16), v[6] | (v[7] << 16));
@@ -196,18 +237,21 @@ __device__ void exec_copy(ExecShared& S, uint8_t* dst, const uint8_t* __restrict
                     if (v[i] & 0x8000u) open &= ~(1u << i);
                 }
         }
-        if (p0 >= lo && p0 + (int32_t)kExPer <= hi) {
+        if (any) {
             uint2 o = make_uint2(0, 0);
 #pragma unroll
             for (uint32_t i = 0; i < 4; i++) {
                 o.x |= (v[i] & 0xFFu) << (8 * i);
                 o.y |= (v[4 + i] & 0xFFu) << (8 * i);
             }
-            *reinterpret_cast<uint2*>(dst + p0) = o;
-        } else if (p0 < hi && p0 + (int32_t)kExPer > lo) {
+            if (p0 >= lo && p0 + (int32_t)kExPer <= hi) {
+                *reinterpret_cast<uint2*>(dst + p0) = o;
+            } else {
 #pragma unroll
-            for (uint32_t i = 0; i < kExPer; i++)
-                if (p0 + (int32_t)i >= lo && p0 + (int32_t)i < hi) dst[p0 + (int32_t)i] = (uint8_t)v[i];
+                for (uint32_t i = 0; i < kExPer; i++)
+                    if (p0 + (int32_t)i >= lo && p0 + (int32_t)i < hi)
+                        dst[p0 + (int32_t)i] = (uint8_t)((i < 4 ? o.x : o.y) >> (8 * (i & 3)));
+            }
         }
         __syncthreads();  // the tile is read by the ones after it
     }
@@ -304,7 +348,7 @@ __global__ void __launch_bounds__(kExThreads) k_dec_exec(const uint8_t* __restri
             else bad = true;
             llit = tok >> 4; lmatch = (tok & 15u) + bmin; isvar = (tok & 15u) == 15u && !bad;
         }
-        const uint32_t em = exec_ends(offs, op0, ol), vm = split ? exec_ends(vs, vp, vl) : 0u;
+        const uint32_t em = exec_window(offs, op0, ol, S.owin), vm = split ? exec_window(vs, vp, vl, S.vwin) : 0u;
         const uint32_t s2 = block_exclusive_scan<kExThreads>(__popc(vm) | (__popc(em) << 16), S.warp, tot);
         const uint32_t nv = tot & 0xFFFFu, ne = tot >> 16;
         exec_put_ends(S.vend, vm, s2 & 0xFFFFu);
@@ -316,7 +360,7 @@ __global__ void __launch_bounds__(kExThreads) k_dec_exec(const uint8_t* __restri
             if (isvar) {
                 vlen = vi < nv ? (uint32_t)S.vend[vi] - vbefore : 5u;
                 if (vlen > 4) bad = true;
-                else vval = exec_varint(vs + vp + vbefore, vlen);
+                else vval = exec_varint(reinterpret_cast<const uint8_t*>(S.vwin) + vbefore, vlen);
             }
         } else if (isvar) {
             const uint32_t p = at + 1 + m;
@@ -339,7 +383,7 @@ __global__ void __launch_bounds__(kExThreads) k_dec_exec(const uint8_t* __restri
         if (isexp) {
             const uint32_t b = ei ? S.oend[ei - 1] : 0u, len = ei < ne ? (uint32_t)S.oend[ei] - b : 5u;
             if (len > 4) badoff = true;
-            else d = exec_varint(offs + op0 + b, len);
+            else d = exec_varint(reinterpret_cast<const uint8_t*>(S.owin) + b, len);
             if (d > kDecMaxBlock) badoff = true;
         }
         // literals and output before the command
@@ -376,11 +420,24 @@ __global__ void __launch_bounds__(kExThreads) k_dec_exec(const uint8_t* __restri
         if (lane == 0) before = rep_identity();
         if (tid == 0) S.event = 0xFFFFFFFFu;
         __syncthreads();
-        RepMap base = reps, all = reps;
-        for (uint32_t w = 0; w < kExThreads / 32; w++) {
-            if (w == warp) base = all;
-            all = rep_then(all, RepMap{{S.rep[w][0], S.rep[w][1], S.rep[w][2], S.rep[w][3]}});
+        if (warp == 0) {  // the maps of the warps before each, from the distances before the chunk
+            constexpr uint32_t kW = kExThreads / 32;
+            RepMap a;
+            for (int i = 0; i < 4; i++) a.e[i] = lane == 0 || lane > kW ? reps.e[i] : S.rep[lane - 1][i];
+#pragma unroll
+            for (int o = 1; o <= (int)kW; o <<= 1) {
+                RepMap b;
+                for (int i = 0; i < 4; i++) b.e[i] = __shfl_up_sync(0xFFFFFFFFu, a.e[i], o);
+                if (lane >= (uint32_t)o) a = rep_then(b, a);
+            }
+            __syncwarp();
+            if (lane <= kW)
+                for (int i = 0; i < 4; i++) S.rep[lane][i] = a.e[i];
         }
+        __syncthreads();
+        const RepMap base = RepMap{{S.rep[warp][0], S.rep[warp][1], S.rep[warp][2], S.rep[warp][3]}};
+        const RepMap all = RepMap{{S.rep[kExThreads / 32][0], S.rep[kExThreads / 32][1], S.rep[kExThreads / 32][2],
+                                   S.rep[kExThreads / 32][3]}};
         if (kind == 1) d = rep_of(base, rep_of(before, kRepFrom | k));
         // how the walk fares at this command
         if (tid > n) {
