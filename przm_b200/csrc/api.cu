@@ -638,8 +638,12 @@ static int32_t launch_range(przmg_batch* b, cudaStream_t s, int stop_after, cons
         uint32_t* tile_w = b->d_tile_sched.as<uint32_t>() + R.tile0;
         uint32_t* tile_order = b->d_tile_sched.as<uint32_t>() + b->tiles.size() + R.tile0;
         const TokTile* tiles = b->d_tiles.as<TokTile>() + R.tile0;
-        k_tile_weight<<<std::min<uint32_t>(nt, 16u * c->sms), 256, 0, s>>>(b->d_jobs.as<Job>(), tiles, nt,
-                                                                          b->d_desc.as<uint32_t>(), tile_w);
+        // gather blocks per frame: two per SM in all, eight tiles each at least
+        const uint32_t parts = std::max<uint32_t>(1, std::min<uint32_t>(2u * c->sms / std::max<uint32_t>(R.nj, 1),
+                                                                        R.maxtiles / 8));
+        k_tile_weight<<<std::min<uint32_t>(nt, 16u * c->sms), 256, 0, s>>>(
+            b->d_jobs.as<Job>(), tiles, nt, b->d_desc.as<uint32_t>(), tile_w,
+            b->d_hist.as<uint32_t>() + (size_t)R.j0 * 1024, parts > 1 ? R.nj * 1024 : 0u);
         CK(cudaGetLastError());
         k_tile_order<<<1, 1024, 0, s>>>(tile_w, nt, tile_order);
         CK(cudaGetLastError());
@@ -648,7 +652,7 @@ static int32_t launch_range(przmg_batch* b, cudaStream_t s, int stop_after, cons
             b->d_slots.as<uint8_t>(), b->d_tile_lens.as<uint32_t>(), b->err_word());
         CK(cudaGetLastError());
         CK(mark(3));
-        k_gather<<<std::min<uint32_t>(R.nj, 16u * c->sms), kGatherThreads, (R.maxtiles + 1) * 4, s>>>(
+        k_gather<<<dim3(std::min<uint32_t>(R.nj, 16u * c->sms), parts), kGatherThreads, (R.maxtiles + 1) * 4, s>>>(
             b->d_jobs.as<Job>(), R.j0, R.nj, b->d_slots.as<uint8_t>(), b->d_tile_lens.as<uint32_t>(),
             b->d_streams.as<uint8_t>(), b->d_job_lens.as<uint32_t>(), b->d_hist.as<uint32_t>(), b->err_word());
         CK(cudaGetLastError());

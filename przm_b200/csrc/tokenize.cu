@@ -98,13 +98,18 @@ __device__ uint32_t warp_match_end(const uint8_t* src, uint32_t a, uint32_t b, u
 // Tokenizer, in two phases per tile (one warp per 32 KiB tile).
 //
 // Walk.  The greedy parse is serial: each decision fixes where the next one
-// starts.  It runs over a shared window of kTokWin match descriptors
-// (radix frames: 8-aligned candidates; small frames: every position), with
-// two shared bitmaps of the window -- non-zero descriptors, and positions
-// whose 4 bytes are equal (the run-length test) -- and a register summary of
-// the non-empty bitmap words.  Finding the next descriptor is a warp-uniform
-// lookup in those; only run-length scans and the extension of 4095-byte
-// matches read global memory.  Every decision
+// starts.  But where it starts depends on the descriptor alone, not on how the
+// parse came there, so over a shared window of kTokWin match descriptors
+// (radix frames: 8-aligned candidates; small frames: every position) the
+// lanes work out every descriptor's successor side by side, and the walk is a
+// chain of one shared load per decision (about 45 cycles, against 300 for a
+// warp-uniform search of the window's bitmaps at every step).  Descriptors
+// that may become a run-length token or whose match may extend past 4095
+// bytes are settled by the warp when the walk comes to them.  Up to 32
+// decisions at a time then become records, lane by lane; which repeat slot a
+// distance is in is a scan of the lists of the three latest distinct
+// distances.  Measured on 12 KB of records (one tile): 300 us with the
+// search.  Every decision
 // becomes a record in shared memory (16 bytes, the fourth word unused):
 //   r0 = q - tile start | literals before q << 16
 //   r1 = match or run length | kind << 16 | repeat slot << 18
@@ -125,9 +130,34 @@ constexpr uint32_t kLongLit = 128;   // literal runs copied 16 bytes per lane
 struct TokSmem {
     uint32_t desc[kTokWin];
     uint32_t nz[kTokWin / 32];  // non-zero descriptors of the window, word per 32 entries
-    uint32_t eq[kTokWin / 32];  // ... whose 4 bytes are equal
+    uint32_t eq[kTokWin / 32];  // ... where a run of equal bytes may be a run-length token
     uint4 rec[kTokRec];         // records (x, y, z; w unused): one 16-byte store each
+    uint16_t next[kTokWin];     // where the walk goes from an entry: the entry after it, or flags
 };
+// flags of a successor: the entry only passes the walk on to the one after it
+// (a longer match starts there); it is settled by the warp; the walk leaves
+// the window
+constexpr uint32_t kNextPass = 0x1000u, kNextSlow = 0x2000u, kNextOut = 0x4000u;
+
+// The three latest distinct distances, latest first (0: none): those of b,
+// then those of a that are not in b.
+struct RepList {
+    uint32_t r0, r1, r2;
+};
+__device__ __forceinline__ RepList rep_list(const RepList& a, const RepList& b) {
+    const bool k0 = a.r0 && a.r0 != b.r0 && a.r0 != b.r1 && a.r0 != b.r2;
+    const bool k1 = a.r1 && a.r1 != b.r0 && a.r1 != b.r1 && a.r1 != b.r2;
+    const bool k2 = a.r2 && a.r2 != b.r0 && a.r2 != b.r1 && a.r2 != b.r2;
+    const uint32_t x2 = k2 ? a.r2 : 0u;
+    const uint32_t c0 = k0 ? a.r0 : k1 ? a.r1 : x2;
+    const uint32_t c1 = k0 ? (k1 ? a.r1 : x2) : (k1 ? x2 : 0u);
+    const uint32_t c2 = k0 && k1 ? x2 : 0u;
+    RepList r;
+    r.r0 = b.r0 ? b.r0 : c0;
+    r.r1 = b.r1 ? b.r1 : b.r0 ? c0 : c1;
+    r.r2 = b.r2 ? b.r2 : b.r1 ? c0 : b.r0 ? c1 : c2;
+    return r;
+}
 
 __device__ __forceinline__ uint32_t vlen(uint32_t v) { return v < 0x80u ? 1u : v < 0x4000u ? 2u : v < 0x200000u ? 3u : v < 0x10000000u ? 4u : 5u; }
 
@@ -217,6 +247,29 @@ __device__ void warp_copy_hist(uint8_t* __restrict__ d, const uint8_t* s, uint32
     }
 }
 
+// Copies n bytes s -> d with eight lanes (t: 0..7), as warp_copy_hist.
+__device__ __forceinline__ void copy_run8(uint8_t* __restrict__ d, const uint8_t* __restrict__ s, uint32_t n, uint32_t t) {
+    const uint32_t head = min(n, (uint32_t)((16 - (reinterpret_cast<uintptr_t>(d) & 15)) & 15));
+    for (uint32_t i = t; i < head; i += 8) d[i] = s[i];
+    d += head;
+    s += head;
+    n -= head;
+    const uint32_t nv = n / 16;
+    const uint32_t sh = 8 * (uint32_t)(reinterpret_cast<uintptr_t>(s) & 3);
+    const uint32_t* sw = reinterpret_cast<const uint32_t*>(reinterpret_cast<uintptr_t>(s) & ~uintptr_t(3));
+    uint4* d4 = reinterpret_cast<uint4*>(d);
+    uint32_t v = t;
+    for (; v + 24 < nv; v += 32) {
+        uint4 o[4];
+#pragma unroll
+        for (int u = 0; u < 4; u++) o[u] = ld16_shifted<false>(sw, v + 8 * u, sh);
+#pragma unroll
+        for (int u = 0; u < 4; u++) d4[v + 8 * u] = o[u];
+    }
+    for (; v < nv; v += 8) d4[v] = ld16_shifted<false>(sw, v, sh);
+    for (uint32_t i = 16 * nv + t; i < n; i += 8) d[i] = s[i];
+}
+
 // Writes records [0, nrec) of the warp's buffer.
 __device__ void tok_emit(const uint4* rec, uint32_t nrec, const uint8_t* tile_src, TokTileOut& o, uint32_t lane) {
     for (uint32_t g = 0; g < nrec; g += 32) {
@@ -302,9 +355,11 @@ __device__ void tok_emit(const uint4* rec, uint32_t nrec, const uint8_t* tile_sr
                 if (kind == 0) put_varint(o.base + slot_base(S_OFF) + off[S_OFF], r2);
             }
         }
-        // literal runs of these records: runs of kLongLit bytes or more one at a
-        // time with the warp's 16-byte copy, the shorter ones all lanes over
-        // their concatenated bytes, four bytes per lane in flight
+        // literal runs of these records: runs of kLongLit bytes or more with
+        // 16-byte copies, four at a time by eight lanes each (one at a time by
+        // the warp, each waits for its loads: 23 000 cycles for 32 runs of 200
+        // bytes), the shorter ones all lanes over their concatenated bytes,
+        // four bytes per lane in flight
         {
             const uint32_t cl = c[S_LIT];
             const bool lng = cl >= kLongLit;
@@ -341,10 +396,14 @@ __device__ void tok_emit(const uint4* rec, uint32_t nrec, const uint8_t* tile_sr
             }
             uint32_t lm = __ballot_sync(0xFFFFFFFFu, lng);
             while (lm) {
-                const uint32_t j = __ffs(lm) - 1;
-                lm &= lm - 1;
-                warp_copy_hist<false>(dl + __shfl_sync(0xFFFFFFFFu, dx, j), tile_src + __shfl_sync(0xFFFFFFFFu, from, j),
-                               __shfl_sync(0xFFFFFFFFu, cl, j), nullptr, lane);
+                // lanes 8 g .. 8 g + 7 take the g-th run left
+                uint32_t m = lm;
+                for (uint32_t g = 0; g < (lane >> 3); g++) m &= m - 1;
+                const uint32_t j = m ? __ffs(m) - 1 : 0;
+                const uint32_t run = __shfl_sync(0xFFFFFFFFu, cl, j), at = __shfl_sync(0xFFFFFFFFu, dx, j),
+                               src_at = __shfl_sync(0xFFFFFFFFu, from, j);
+                if (m) copy_run8(dl + at, tile_src + src_at, run, lane & 7);
+                for (uint32_t g = 0; g < 4; g++) lm &= lm - 1;
             }
         }
 #pragma unroll
@@ -373,9 +432,57 @@ __device__ void tokenize_tile(const uint8_t* __restrict__ in, const Job* __restr
         o.base = slots + S * kSlotStride;
         for (int s = 0; s < S_COUNT; s++) o.len[s] = 0;
         o.ok = true;
-        int rep0 = tt.tile == 0 ? 1 : -1, rep1 = tt.tile == 0 ? 4 : -1, rep2 = tt.tile == 0 ? 8 : -1;
+        RepList reps = tt.tile == 0 ? RepList{1, 4, 8} : RepList{0, 0, 0};
         uint32_t pos = start, litStart = start, nrec = 0;
         uint32_t wb = 0xFFFFFFFFu, wsum = 0;  // window base entry; bit k: word k of the window has a descriptor
+        // decisions not yet records: lane i has the i-th one's window entry,
+        // its length where the warp settled it (else 0) and whether it is a run
+        uint32_t cnt = 0, my = 0, my_len = 0;
+        bool my_run = false;
+        auto pos_of = [&](uint32_t ent) { return radix ? 8 * ent : ent; };
+        auto flush = [&]() {
+            const bool v = lane < cnt;
+            const uint32_t qd = sm.desc[my], q = pos_of(wb + my);
+            const uint32_t len = my_len ? my_len : min(qd >> 20, end - q), d = qd & 0xFFFFFu;
+            uint32_t from = __shfl_up_sync(0xFFFFFFFFu, q + len, 1);
+            if (lane == 0) from = litStart;
+            RepList inc = v && !my_run ? RepList{d, 0, 0} : RepList{0, 0, 0};
+#pragma unroll
+            for (int sft = 1; sft < 32; sft <<= 1) {
+                RepList a;
+                a.r0 = __shfl_up_sync(0xFFFFFFFFu, inc.r0, sft);
+                a.r1 = __shfl_up_sync(0xFFFFFFFFu, inc.r1, sft);
+                a.r2 = __shfl_up_sync(0xFFFFFFFFu, inc.r2, sft);
+                if (lane >= (uint32_t)sft) inc = rep_list(a, inc);
+            }
+            inc = rep_list(reps, inc);
+            RepList before;
+            before.r0 = __shfl_up_sync(0xFFFFFFFFu, inc.r0, 1);
+            before.r1 = __shfl_up_sync(0xFFFFFFFFu, inc.r1, 1);
+            before.r2 = __shfl_up_sync(0xFFFFFFFFu, inc.r2, 1);
+            if (lane == 0) before = reps;
+            if (v) {
+                const int k = d == before.r0 ? 0 : d == before.r1 ? 1 : d == before.r2 ? 2 : -1;
+                sm.rec[nrec + lane] =
+                    my_run ? make_uint4((q - start) | ((q - from) << 16), len | (2u << 16), 0u, 0u)
+                           : make_uint4((q - start) | ((q - from) << 16),
+                                        len | ((k >= 0 ? 1u : 0u) << 16) | ((uint32_t)(k >= 0 ? k : 0) << 18), d, 0u);
+            }
+            reps.r0 = __shfl_sync(0xFFFFFFFFu, inc.r0, 31);
+            reps.r1 = __shfl_sync(0xFFFFFFFFu, inc.r1, 31);
+            reps.r2 = __shfl_sync(0xFFFFFFFFu, inc.r2, 31);
+            litStart = __shfl_sync(0xFFFFFFFFu, q + len, cnt - 1);
+            nrec += cnt;
+            cnt = 0;
+            my = my_len = 0;
+            my_run = false;
+            if (nrec > kTokRec - 32) {
+                __syncwarp();
+                tok_emit(sm.rec, nrec, src + start, o, lane);
+                nrec = 0;
+                __syncwarp();
+            }
+        };
         auto refill = [&](uint32_t base) {
             // entries [base, base + kTokWin): descriptors to shared memory, one
             // bitmap word per lane.  Every load instruction of the warp reads
@@ -427,34 +534,91 @@ __device__ void tokenize_tile(const uint8_t* __restrict__ in, const Job* __restr
                     bool ea = false, eb = false;
                     if (base + 2 * u < e_hi) {  // bytes below 8 e_hi + 8 <= n + 8
                         const uint4 v = __ldg(s4 + u);
-                        ea = v.x == 0x01010101u * (v.x & 0xFFu);
-                        eb = v.z == 0x01010101u * (v.z & 0xFFu);
+                        ea = v.x == v.y && v.x == 0x01010101u * (v.x & 0xFFu);
+                        eb = v.z == v.w && v.z == 0x01010101u * (v.z & 0xFFu);
                     }
                     const uint32_t ba = __ballot_sync(0xFFFFFFFFu, ea), bb = __ballot_sync(0xFFFFFFFFu, eb);
                     if ((lane >> 1) == i) { capa = ba; capb = bb; }
                 }
                 const uint32_t s16 = 16 * (lane & 1);
                 eq = spread16((capa >> s16) & 0xFFFFu) | (spread16((capb >> s16) & 0xFFFFu) << 1);
-            } else if (nz) {
+            } else {
                 // positions base + 32 lane .. + 31 (32-aligned, inputs are 16-aligned
-                // and padded by 64 bytes past n)
-                const uint4* s4 = reinterpret_cast<const uint4*>(src + base + 32 * lane);
-                const uint4 a = __ldg(s4), b = __ldg(s4 + 1), c = __ldg(s4 + 2);
-                const uint32_t w[12] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w, c.x, c.y, c.z, c.w};
+                // and padded by 64 bytes past n): the runs of twelve equal bytes,
+                // nine neighbours whose four bytes are equal
+                if (base + 32 * lane < e_hi) {
+                    const uint4* s4 = reinterpret_cast<const uint4*>(src + base + 32 * lane);
+                    const uint4 a = __ldg(s4), b = __ldg(s4 + 1), c = __ldg(s4 + 2);
+                    const uint32_t w[12] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w, c.x, c.y, c.z, c.w};
 #pragma unroll
-                for (uint32_t k = 0; k < 32; k++) {
-                    const uint32_t x = (k & 3) ? __funnelshift_r(w[k >> 2], w[(k >> 2) + 1], 8 * (k & 3)) : w[k >> 2];
-                    eq |= (x == 0x01010101u * (x & 0xFFu) ? 1u : 0u) << k;
+                    for (uint32_t k = 0; k < 32; k++) {
+                        const uint32_t x = (k & 3) ? __funnelshift_r(w[k >> 2], w[(k >> 2) + 1], 8 * (k & 3)) : w[k >> 2];
+                        eq |= (x == 0x01010101u * (x & 0xFFu) ? 1u : 0u) << k;
+                    }
                 }
+                uint32_t hi = __shfl_down_sync(0xFFFFFFFFu, eq, 1);
+                if (lane == 31) hi = 0xFFFFFFFFu;  // (not looked at: kept as candidates)
+                const uint64_t m0 = (uint64_t)eq | ((uint64_t)hi << 32), m1 = m0 & (m0 >> 1), m2 = m1 & (m1 >> 2);
+                eq = (uint32_t)(m2 & (m2 >> 4) & (m0 >> 8));
             }
             sm.nz[lane] = nz;
             sm.eq[lane] = eq & nz;
+            __syncwarp();
+            // every descriptor's successor: 128 neighbours at a time, four a
+            // lane, step by step so that their shared loads overlap
+            for (uint32_t i0 = 0; i0 < 32; i0 += 4) {
+                if (((wsum >> i0) & 15u) == 0) continue;
+                uint32_t qd[4], nd[4], eqw[4], to[4], f[4], w[4];
+                bool pass[4], none = false;
+#pragma unroll
+                for (int u = 0; u < 4; u++) {
+                    const uint32_t rel = 32 * (i0 + u) + lane;
+                    qd[u] = sm.desc[rel];
+                    nd[u] = radix ? 0u : sm.desc[min(rel + 1, kTokWin - 1)];
+                    eqw[u] = sm.eq[i0 + u];
+                }
+                if (!radix && i0 == 28 && lane == 31 && base + kTokWin < e_hi) nd[3] = ld_stage<kC>(dj + base + kTokWin);
+#pragma unroll
+                for (int u = 0; u < 4; u++) {
+                    const uint32_t q = pos_of(base + 32 * (i0 + u) + lane), len = qd[u] >> 20;
+                    const uint32_t mLen = min(len, end - q), t = q + mLen;
+                    // lookahead (przm_tokenizer.cuh:196-216): radix frames have
+                    // no descriptor at q + 1
+                    pass[u] = !radix && q + 1 < end && (nd[u] >> 20) > len + 1;
+                    f[u] = (q + 12 <= end && ((eqw[u] >> lane) & 1u)) || mLen >= kMaxLen32 ? kNextSlow : 0u;
+                    to[u] = min((radix ? (t + 7) >> 3 : t) - base, kTokWin);  // entries from there on
+                    w[u] = to[u] < kTokWin ? sm.nz[to[u] >> 5] & (0xFFFFFFFFu << (to[u] & 31)) : 0u;
+                    none |= w[u] == 0;
+                }
+                if (none) {  // the next non-empty word
+#pragma unroll
+                    for (int u = 0; u < 4; u++)
+                        if (w[u] == 0) {
+                            const uint32_t l = to[u] >> 5, rest = l < 31 ? wsum & (0xFFFFFFFEu << l) : 0u;
+                            const uint32_t k = rest ? __ffs(rest) - 1 : 0u;
+                            if (rest) {
+                                w[u] = sm.nz[k];
+                                to[u] = 32 * k;
+                            }
+                        }
+                }
+#pragma unroll
+                for (int u = 0; u < 4; u++) {
+                    const uint32_t rel = 32 * (i0 + u) + lane;
+                    f[u] |= w[u] ? (to[u] & ~31u) + __ffs(w[u]) - 1 : kNextOut;
+                    if (pass[u]) f[u] = kNextPass | (rel + 1 < kTokWin ? rel + 1 : kNextOut);
+                    if (qd[u]) sm.next[rel] = (uint16_t)f[u];
+                }
+            }
             __syncwarp();
         };
         while (pos < end && o.ok) {
             const uint32_t e0 = radix ? (pos + 7) >> 3 : pos;
             if (e0 >= e_hi) break;
-            if (wb == 0xFFFFFFFFu || e0 >= wb + kTokWin || e0 < wb) refill(e0 & ~31u);
+            if (wb == 0xFFFFFFFFu || e0 >= wb + kTokWin || e0 < wb) {
+                if (cnt) flush();
+                refill(e0 & ~31u);
+            }
             // next descriptor at or after e0: the rest of e0's word, else the
             // first non-empty word after it (warp-uniform, no shuffles)
             const uint32_t rel = e0 - wb;
@@ -471,65 +635,71 @@ __device__ void tokenize_tile(const uint8_t* __restrict__ in, const Job* __restr
                 l = __ffs(rest) - 1;
                 wl = sm.nz[l];
             }
-            const uint32_t eql = sm.eq[l];
-            const uint32_t bit = __ffs(wl) - 1;
-            const uint32_t ent = wb + 32 * l + bit;
-            const uint32_t q = radix ? 8 * ent : ent;
-            if (q >= end) break;
-            const uint32_t qd = sm.desc[ent - wb];
-            uint32_t mLen = qd >> 20;
-            const uint32_t d = qd & 0xFFFFFu;
-            // lookahead (przm_tokenizer.cuh:196-216): radix frames have no
-            // descriptor at q + 1
-            if (!radix && q + 1 < end) {
-                const uint32_t nd = ent + 1 - wb < kTokWin ? sm.desc[ent + 1 - wb] : ld_stage<kC>(dj + ent + 1);
-                if (nd != 0 && (nd >> 20) > mLen + 1) { pos = q + 1; continue; }
-            }
-            // run-length token (:218-286)
-            if (q + 12 <= end && ((eql >> bit) & 1u)) {
-                const uint8_t b0 = src[q];
-                const uint32_t lim = q + min(end - q, 65535u);
-                const uint32_t r = warp_run_end(src, q + 4, lim, b0, lane) - q;
-                if (r >= 12 && r >= mLen) {
-                    if (lane == 0) sm.rec[nrec] = make_uint4((q - start) | ((q - litStart) << 16), r | (2u << 16), 0u, 0u);
-                    nrec++;
-                    pos = q + r;
-                    litStart = pos;
-                    if (nrec == kTokRec) { __syncwarp(); tok_emit(sm.rec, nrec, src + start, o, lane); nrec = 0; __syncwarp(); }
+            uint32_t e = 32 * l + __ffs(wl) - 1, nx;
+            // the chain: decisions until one leaves the window or is settled here
+            for (;;) {
+                // four links at a time while nothing has to be settled
+                while (cnt <= 28) {
+                    const uint32_t n0 = sm.next[e], e1 = n0 & (kTokWin - 1), n1 = sm.next[e1], e2 = n1 & (kTokWin - 1);
+                    const uint32_t n2 = sm.next[e2], e3 = n2 & (kTokWin - 1), n3 = sm.next[e3];
+                    if ((n0 | n1 | n2 | n3) & (kNextSlow | kNextOut)) break;
+                    const bool d0 = !(n0 & kNextPass), d1 = !(n1 & kNextPass), d2 = !(n2 & kNextPass), d3 = !(n3 & kNextPass);
+                    const uint32_t i = lane - cnt, i1 = d0, i2 = i1 + d1, i3 = i2 + d2;
+                    if (i == 0 && d0) my = e;
+                    if (i == i1 && d1) my = e1;
+                    if (i == i2 && d2) my = e2;
+                    if (i == i3 && d3) my = e3;
+                    cnt += i3 + d3;
+                    e = n3 & (kTokWin - 1);
+                }
+                nx = sm.next[e];
+                if (nx & kNextPass) {
+                    if (nx & kNextOut) break;
+                    e = nx & (kTokWin - 1);
                     continue;
                 }
+                if (cnt == 32) flush();
+                if (lane == cnt) my = e;
+                cnt++;
+                if (nx & (kNextSlow | kNextOut)) break;
+                e = nx & (kTokWin - 1);
             }
-            // match (:289-320).  The reference re-checks d <= q, mLen >= 4 and
-            // the first 4 bytes here; every non-zero descriptor of both finders
-            // (k_tile_find, k_rx_verify) already satisfies them.  Both finders
-            // also stop a match at its first mismatch unless it reached 4095
-            // bytes or the end of the data, so the forward extension can only
-            // continue a 4095-byte descriptor.
-            if (q + mLen > end) mLen = end - q;
-            if (mLen >= kMaxLen32) {
-                const uint32_t lim = min(end - q, 65530u);
-                if (mLen < lim && src[q + mLen] == src[q - d + mLen])
-                    mLen = warp_match_end(src, q, q - d, mLen, lim, lane);
+            const uint32_t q = pos_of(wb + e);
+            if (nx & kNextPass) {
+                pos = q + 1;
+                continue;
             }
-            int k = -1;
-            if ((int)d == rep0 && rep0 > 0) k = 0;
-            else if ((int)d == rep1 && rep1 > 0) k = 1;
-            else if ((int)d == rep2 && rep2 > 0) k = 2;
-            if (lane == 0)
-                sm.rec[nrec] = make_uint4((q - start) | ((q - litStart) << 16),
-                                          mLen | ((k >= 0 ? 1u : 0u) << 16) | ((uint32_t)(k >= 0 ? k : 0) << 18), d, 0u);
-            nrec++;
-            if (k < 0) {
-                rep2 = rep1; rep1 = rep0; rep0 = (int)d;
-            } else if (k == 1) {
-                rep1 = rep0; rep0 = (int)d;
-            } else if (k == 2) {
-                rep2 = rep1; rep1 = rep0; rep0 = (int)d;
+            uint32_t mLen = min(sm.desc[e] >> 20, end - q);
+            if (nx & kNextSlow) {
+                // run-length token (:218-286)
+                bool run = false;
+                if (q + 12 <= end && ((sm.eq[e >> 5] >> (e & 31)) & 1u)) {
+                    const uint32_t lim = q + min(end - q, 65535u);
+                    const uint32_t r = warp_run_end(src, q + 4, lim, src[q], lane) - q;
+                    if (r >= 12 && r >= (sm.desc[e] >> 20)) {
+                        run = true;
+                        mLen = r;
+                    }
+                }
+                // match (:289-320).  The reference re-checks d <= q, mLen >= 4
+                // and the first 4 bytes here; every non-zero descriptor of both
+                // finders (k_tile_find, k_rx_verify) already satisfies them.
+                // Both finders also stop a match at its first mismatch unless it
+                // reached 4095 bytes or the end of the data, so the forward
+                // extension can only continue a 4095-byte descriptor.
+                if (!run && mLen >= kMaxLen32) {
+                    const uint32_t d = sm.desc[e] & 0xFFFFFu, lim = min(end - q, 65530u);
+                    if (mLen < lim && src[q + mLen] == src[q - d + mLen])
+                        mLen = warp_match_end(src, q, q - d, mLen, lim, lane);
+                }
+                if (lane == cnt - 1) {
+                    my_len = mLen;
+                    my_run = run;
+                }
             }
             pos = q + mLen;
-            litStart = pos;
-            if (nrec == kTokRec) { __syncwarp(); tok_emit(sm.rec, nrec, src + start, o, lane); nrec = 0; __syncwarp(); }
         }
+        if (cnt) flush();
         if (o.ok && litStart < end) {  // trailing literals (:440-464)
             if (lane == 0) sm.rec[nrec] = make_uint4((end - start) | ((end - litStart) << 16), 3u << 16, 0u, 0u);
             nrec++;
@@ -544,7 +714,7 @@ __device__ void tokenize_tile(const uint8_t* __restrict__ in, const Job* __restr
     }
 }
 
-__global__ void __launch_bounds__(kTokWarps * 32) k_tokenize(const uint8_t* __restrict__ in, const Job* __restrict__ jobs,
+__global__ void __launch_bounds__(kTokWarps * 32, 5) k_tokenize(const uint8_t* __restrict__ in, const Job* __restrict__ jobs,
                                                             const TokTile* __restrict__ tiles, uint32_t ntiles,
                                                             const uint32_t* __restrict__ order,
                                                             const uint32_t* __restrict__ desc, uint8_t* __restrict__ slots,
@@ -567,8 +737,11 @@ __global__ void __launch_bounds__(kTokWarps * 32) k_tokenize(const uint8_t* __re
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(256) k_tile_weight(const Job* __restrict__ jobs, const TokTile* __restrict__ tiles,
                                                      uint32_t ntiles, const uint32_t* __restrict__ desc,
-                                                     uint32_t* __restrict__ weight) {
+                                                     uint32_t* __restrict__ weight, uint32_t* __restrict__ hist,
+                                                     uint32_t hist_words) {
     __shared__ uint32_t s_w[8];
+    // (and clears the histograms that several gather blocks add to)
+    for (uint32_t i = blockIdx.x * 256 + threadIdx.x; i < hist_words; i += gridDim.x * 256) hist[i] = 0;
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     for (uint32_t T = blockIdx.x; T < ntiles; T += gridDim.x) {
         const TokTile tt = tiles[T];
@@ -635,20 +808,23 @@ __global__ void __launch_bounds__(1024) k_tile_order(const uint32_t* __restrict_
 }
 
 // ---------------------------------------------------------------------------
-// Gather: one CTA per frame concatenates its tiles' slots into the frame's
-// contiguous streams (przm_tokenizer.cuh:474-609) and counts the byte
-// histograms of the literal stream and of the three command substreams,
-// privatised per warp in shared memory.
+// Gather: concatenates a frame's tiles' slots into the frame's contiguous
+// streams (przm_tokenizer.cuh:474-609) and counts the byte histograms of the
+// literal stream and of the three command substreams, privatised per warp in
+// shared memory.  One block per frame, or several with a run of its tiles
+// each where the frames alone leave SMs idle (one frame of 4 MiB took 0.30 ms
+// with one block); their counts then meet in the frame's histogram by atomics.
 // ---------------------------------------------------------------------------
 constexpr uint32_t kGatherThreads = 512;
 
-// Frame j by the whole block (any multiple of 128 threads); s_off =
-// ntiles + 1 words, s_hist = [stream][warp group][symbol] counts.
+// Frame j by the whole block (any multiple of 128 threads), or part `part` of
+// `parts` of its tiles (hist then zeroed before); s_off = ntiles + 1 words,
+// s_hist = [stream][warp group][symbol] counts.
 template <bool kC>
 __device__ void gather_item(const Job* __restrict__ jobs, uint32_t j, const uint8_t* slots,
                             const uint32_t* tile_lens, uint8_t* __restrict__ streams,
                             uint32_t* __restrict__ job_lens, uint32_t* __restrict__ hist, uint32_t* __restrict__ err,
-                            uint32_t* s_off, uint32_t (*s_hist)[4][256]) {
+                            uint32_t* s_off, uint32_t (*s_hist)[4][256], uint32_t part = 0, uint32_t parts = 1) {
     const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nthr = blockDim.x;
     {
         const Job job = jobs[j];
@@ -685,17 +861,20 @@ __device__ void gather_item(const Job* __restrict__ jobs, uint32_t j, const uint
             uint8_t* dst = sreg + stream_base(job, s);
             const int hs = s == S_LIT ? 0 : (s == S_OP ? 1 : (s == S_META ? 2 : (s == S_VAR ? 3 : -1)));
             // one warp per tile
-            for (uint32_t t = warp; t < job.ntiles; t += nthr / 32) {
+            const uint32_t t1 = (uint32_t)((uint64_t)job.ntiles * (part + 1) / parts);
+            for (uint32_t t = (uint32_t)((uint64_t)job.ntiles * part / parts) + warp; t < t1; t += nthr / 32) {
                 const uint32_t o = s_off[t], l = s_off[t + 1] - o;
                 const uint8_t* sp = slots + (uint64_t)(job.tile0 + t) * kSlotStride + slot_base(s);
                 warp_copy_hist<kC>(dst + o, sp, l, hs >= 0 ? s_hist[hs][warp & 3] : nullptr, lane);
             }
-            if (tid == 0) job_lens[(uint64_t)j * S_COUNT + s] = total;
+            if (tid == 0 && part == 0) job_lens[(uint64_t)j * S_COUNT + s] = total;
         }
         __syncthreads();
         for (uint32_t i = tid; i < 4 * 256; i += nthr) {
             uint32_t hs = i >> 8, sym = i & 255;
-            hist[(uint64_t)j * 1024 + i] = s_hist[hs][0][sym] + s_hist[hs][1][sym] + s_hist[hs][2][sym] + s_hist[hs][3][sym];
+            const uint32_t c = s_hist[hs][0][sym] + s_hist[hs][1][sym] + s_hist[hs][2][sym] + s_hist[hs][3][sym];
+            if (parts == 1) hist[(uint64_t)j * 1024 + i] = c;
+            else if (c) atomicAdd(&hist[(uint64_t)j * 1024 + i], c);
         }
         __syncthreads();
     }
@@ -710,7 +889,7 @@ __global__ void __launch_bounds__(kGatherThreads) k_gather(const Job* __restrict
     extern __shared__ uint32_t smem_g[];
     __shared__ uint32_t s_hist[4][4][256];
     for (uint32_t jl = blockIdx.x; jl < njobs; jl += gridDim.x)
-        gather_item<false>(jobs, j0 + jl, slots, tile_lens, streams, job_lens, hist, err, smem_g, s_hist);
+        gather_item<false>(jobs, j0 + jl, slots, tile_lens, streams, job_lens, hist, err, smem_g, s_hist, blockIdx.y, gridDim.y);
 }
 
 }  // namespace pz
