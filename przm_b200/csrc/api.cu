@@ -156,6 +156,9 @@ struct przmg_batch {
     DevBuf d_asm;         // assembly work items (frame, part)
     DevBuf d_asm_job;     // the same items grouped by input (plain per-input launches)
     DevBuf d_s3, d_s3f;   // P2 and up: per-input Section 3 regions and their S3Frame facts
+    DevBuf d_m12, d_m12_seg0;  // P2 and up: the Mode 12 chains' segments, each input's first
+    uint64_t m12_segs_total = 0;
+    std::vector<uint32_t> m12_seg0;
     DevBuf d_fib;         // P3: per-input fiber regions
     DevBuf d_seg;         // segments of the long rANS tasks
     uint32_t seg_cap = 0, seg_cap_m8 = 0;  // segments at most, of Meta8 tasks at most
@@ -200,7 +203,7 @@ struct przmg_batch {
                          &d_job_lens, &d_hist, &d_tabs, &d_infos, &d_ans, &d_outs, &d_plans, &d_sizes, &d_out, &d_misc,
                          &d_lists, &d_rtiles, &d_rx_toff, &d_rx_list, &d_rx_pred, &d_stage_in,
                          &d_stage_out, &d_stage_offs, &d_up_offs, &d_tile_sched, &d_asm, &d_asm_job,
-                         &d_fitems, &d_ftiles, &d_ftarget, &d_fctl, &d_s3, &d_s3f, &d_fib, &d_seg};
+                         &d_fitems, &d_ftiles, &d_ftarget, &d_fctl, &d_s3, &d_s3f, &d_m12, &d_m12_seg0, &d_fib, &d_seg};
         for (DevBuf* b : all) b->release();
         h_offs.release();
     }
@@ -311,7 +314,8 @@ static int32_t batch_prepare(przmg_batch* b, const uint64_t* sizes, uint32_t njo
     b->max_big_cand = 0;
     b->in_offs.assign(njobs, 0);
     b->out_offs.assign(njobs, 0);
-    uint64_t in = 0, desc = 0, str = 0, ans = 0, out = 0, s3 = 0, fib = 0, segb = 0, segb_m8 = 0;
+    uint64_t in = 0, desc = 0, str = 0, ans = 0, out = 0, s3 = 0, fib = 0, segb = 0, segb_m8 = 0, m12s = 0;
+    b->m12_seg0.assign(njobs, 0);
     uint32_t tile0 = 0;
     for (auto* v : {&b->job_small0, &b->job_rt0, &b->job_big0, &b->job_tile0, &b->job_asm0}) v->assign(njobs + 1, 0);
     for (uint32_t i = 0; i < njobs; i++) {
@@ -341,6 +345,8 @@ static int32_t batch_prepare(przmg_batch* b, const uint64_t* sizes, uint32_t njo
         if (profile >= 2) {
             j.dist_cap = (uint32_t)(n / 4 + 64);
             j.s3_off = s3;
+            b->m12_seg0[i] = (uint32_t)m12s;
+            m12s += m12_segs(std::min(j.dist_cap, kS3Scratch)) + 1;
             s3 += align16(s3_region_bytes(j));
         }
         if (profile >= 3) {
@@ -434,6 +440,11 @@ static int32_t batch_prepare(przmg_batch* b, const uint64_t* sizes, uint32_t njo
     CK(b->d_s3.ensure(s3 + 64));
     CK(b->d_s3f.ensure(sizeof(S3Frame) * std::max<uint32_t>(njobs, 1)));
     CK(b->d_fib.ensure(fib + 64));
+    b->m12_segs_total = m12s;
+    if (profile >= 2) {
+        CK(b->d_m12.ensure(m12_buf_bytes(m12s)));
+        CK(b->d_m12_seg0.ensure(4ull * std::max<uint32_t>(njobs, 1)));
+    }
     if (profile >= 2 && !b->aux) {
         CK(cudaStreamCreateWithFlags(&b->aux, cudaStreamNonBlocking));
         CK(cudaEventCreateWithFlags(&b->ev_fork, cudaEventDisableTiming));
@@ -477,6 +488,8 @@ static int32_t batch_prepare(przmg_batch* b, const uint64_t* sizes, uint32_t njo
             CK(cudaMemcpyAsync(b->d_ftiles.p, ftiles.data(), sizeof(TokTile) * ftiles.size(), cudaMemcpyHostToDevice, s));
         CK(cudaMemcpyAsync(b->d_ftarget.p, ftarget.data(), 4ull * njobs, cudaMemcpyHostToDevice, s));
     }
+    if (profile >= 2 && njobs)
+        CK(cudaMemcpyAsync(b->d_m12_seg0.p, b->m12_seg0.data(), 4ull * njobs, cudaMemcpyHostToDevice, s));
     CK(cudaMemsetAsync(b->d_sizes.p, 0, (size_t)njobs * 4 + 16, s));
     CK(cudaMemsetAsync(b->d_job_lens.p, 0, (size_t)njobs * S_COUNT * 4 + 16, s));
     // the host-side vectors above must stay alive until the copies ran
@@ -671,15 +684,17 @@ static int32_t launch_range(przmg_batch* b, cudaStream_t s, int stop_after, cons
                                                       b->d_s3f.as<S3Frame>(), b->err_word());
                 CK(cudaGetLastError());
                 launches++;
-                // the Mode 12 chains (one thread per frame, serial by the
-                // format) on the second stream, beside the rANS launch
+                // the Mode 12 chains on the second stream, beside the rANS launch
                 CK(cudaEventRecord(b->ev_fork, s));
                 CK(cudaStreamWaitEvent(b->aux, b->ev_fork, 0));
-                k_s3_chain<<<(R.nj + 31) / 32, 32, 0, b->aux>>>(b->d_jobs.as<Job>(), R.j0, R.nj, b->d_s3.as<uint8_t>(),
-                                                               b->d_s3f.as<S3Frame>(), c->d_dist12.as<EncSym>());
-                CK(cudaGetLastError());
+                uint32_t most = 0;
+                for (uint32_t i = R.j0; i < R.j0 + R.nj; i++) most = std::max(most, b->jobs[i].dist_cap);
+                most = std::min(most, kS3Scratch);
+                const M12Frames mf{b->d_jobs.as<Job>(), b->d_s3.as<uint8_t>(), b->d_s3f.as<S3Frame>(),
+                                   b->d_m12_seg0.as<uint32_t>(), R.j0};
+                CK(launch_m12(mf, R.nj, most, m12_bufs(b->d_m12.p, b->m12_segs_total), c->d_dist12.as<EncSym>(), b->aux));
                 CK(cudaEventRecord(b->ev_join, b->aux));
-                launches++;
+                launches += m12_segs(most) > 1 ? 4 : 2;
             }
             if (b->profile >= 3) {  // Section 4: the literals' four foliations
                 k_frame_fibers<<<dim3(R.nj, 4), kFibThreads, 0, s>>>(b->d_jobs.as<Job>(), R.j0, b->d_job_lens.as<uint32_t>(),

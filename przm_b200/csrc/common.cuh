@@ -117,19 +117,16 @@ struct Job {
 // A P2 job's Section 3 region: the distance codes (dist_cap + 16 bytes),
 // the MSB-first extra-bit stream (3 bytes per distance + 16: at most 18
 // extra bits for distances below 2^20, so at most four bytes are touched
-// per distance), the Mode 12 bytes in emission order (2 per code at most,
-// capped at the reference's 2 MiB scratch, + 16), and the codes' histogram
-// (256 u32).
+// per distance), the Mode 12 chain's records (the layout of a V-ANS task of
+// dist_cap symbols), and the codes' histogram (256 u32).
 constexpr uint32_t kS3Scratch = 2u * 1024 * 1024;  // the reference's 2 MiB distance scratch buffers
 __host__ __device__ inline uint64_t s3_extra_off(const Job& j) { return (j.dist_cap + 16ull + 15) & ~15ull; }
 __host__ __device__ inline uint64_t s3_em_off(const Job& j) { return s3_extra_off(j) + ((3ull * j.dist_cap + 16 + 15) & ~15ull); }
-__host__ __device__ inline uint64_t s3_em_cap(const Job& j) {
-    return 2ull * j.dist_cap < kS3Scratch ? 2ull * j.dist_cap : (uint64_t)kS3Scratch;
-}
-__host__ __device__ inline uint64_t s3_hist_off(const Job& j) { return s3_em_off(j) + ((s3_em_cap(j) + 16 + 15) & ~15ull); }
+__host__ __device__ constexpr uint64_t ans_task_bytes(uint32_t L);
+__host__ __device__ inline uint64_t s3_hist_off(const Job& j) { return s3_em_off(j) + ans_task_bytes(j.dist_cap); }
 __host__ __device__ inline uint64_t s3_region_bytes(const Job& j) { return s3_hist_off(j) + 256 * 4; }
 
-// Per-frame Section 3 facts from k_s3_frame and k_s3_chain.
+// Per-frame Section 3 facts from k_s3_frame and the Mode 12 chain (k_m12_sum).
 struct S3Frame {
     uint32_t nd;     // distances
     uint32_t bits;   // their extra bits

@@ -11,11 +11,9 @@
 //               (DistanceToCode :165-180), ORs the extra bits into a zeroed
 //               MSB-first stream (BitWriter :204-247) at offsets from a
 //               second scan, and counts the codes' histogram;
-//   k_s3_chain  one thread per frame: the Mode 12 chain
-//               (EncodeDistClusteredVans :323-377), one rANS state over the
-//               codes from the last to the first, each coded with the static
-//               weights of its predecessor's class; the emitted bytes are
-//               kept in emission order and reversed by the assembler;
+//   k_m12_*     the Mode 12 chain (EncodeDistClusteredVans :323-377), one
+//               rANS state over the codes from the last to the first, in
+//               segments; its records are stitched by the assembler;
 //   the codes' adaptive V-ANS container (EncodeAdaptiveVANS4x, for 64 codes
 //   or more) is one more task of the frame's rANS launch (model 4, task
 //   T_S3), and k_plan picks the form from the sizes as PackDistancePrefix /
@@ -132,77 +130,280 @@ __global__ void __launch_bounds__(kS3Threads) k_s3_frame(const Job* __restrict__
     }
 }
 
-// One Mode 12 step: the code's entry in registers; emits the bytes the
-// reference would write (low byte first) into em[e..] and advances x.
-// False when they would pass the reference's 2 MiB emission scratch.
-__device__ __forceinline__ bool m12_step(uint32_t& x, uint32_t& e, const EncSym& es, uint8_t* __restrict__ em) {
-    const uint32_t k = rans_shift(x, es);
-    if (k) {
-        if (e + (k >> 3) > kS3Scratch) return false;
-        em[e] = (uint8_t)x;
-        if (k == 16) em[e + 1] = (uint8_t)(x >> 8);
-        e += k >> 3;
-    }
-    x = rans_after(x, es, k);
-    return true;
+// ---------------------------------------------------------------------------
+// Mode 12 (EncodeDistClusteredVans, distance.go:323-377): one rANS state over
+// the codes from the last to the first, each coded with the static weights of
+// its predecessor's class.  Code i goes to round i / 4, lane i mod 4 of a
+// V-ANS task's record layout (one chain instead of four, so the stitch of
+// that layout writes exactly the reversed emission), and long chains are cut
+// into segments found by coalescing walkers, as the V-ANS tasks are (see
+// k_seg_walk): 64 states walk the kM12Warm codes above a segment, at most 32
+// are left of them after 512 codes, and the segment's true first state is one
+// of theirs (in 0 to 0.3 % of the segments it is not and walks on by itself).
+// A warp takes 32 codes at a time: the lanes look up their entries, all lanes
+// run the chain (one state each when walking), the lanes write the records.
+// Measured on 256 sections of 20 000 distances: 1.95 ms with one thread per
+// chain emitting bytes.
+// ---------------------------------------------------------------------------
+constexpr uint32_t kM12Seg = 2048, kM12Warm = 1024;
+constexpr uint32_t kM12Split = 6144;  // codes up to which one warp codes the chain as fast as segments are found
+static_assert(4 * kStitchRounds % kM12Seg == 0, "stitch passes start at segment ends");
+
+struct M12Task {
+    const uint8_t* codes;
+    uint8_t* base;       // record layout of ans_task_bytes(cap), 16-byte aligned
+    uint32_t n, cap;     // n 0: no chain
+    uint32_t seg0;       // its first segment in M12Bufs
+};
+struct M12Bufs {  // per segment: the walkers' states at its first code and after it, its true first state, its bytes, its last state
+    uint32_t *marks, *first, *bytes, *last;
+};
+__host__ __device__ inline uint32_t m12_segs(uint32_t n) { return n > kM12Split ? (n + kM12Seg - 1) / kM12Seg : n ? 1u : 0u; }
+__host__ __device__ inline uint64_t m12_buf_bytes(uint64_t segs) { return 4 * (64 + 3) * segs; }
+__host__ __device__ inline M12Bufs m12_bufs(void* p, uint64_t segs) {
+    M12Bufs b;
+    b.marks = static_cast<uint32_t*>(p);
+    b.first = b.marks + 64 * segs;
+    b.bytes = b.first + segs;
+    b.last = b.bytes + segs;
+    return b;
 }
 
-// The Mode 12 chain over codes[0, nd) (one thread): codes from the last to
-// the first, each with the model of its predecessor's class (s_tab: the
-// 4 x 64 static weights in EncSym form); the emitted bytes go to em in
-// emission order.  Codes are taken eight at a time from aligned words (codes
-// 16-byte aligned), so the table entries of a group load before its
-// dependent steps run.  False where the reference's 2 MiB emission scratch
-// would overflow.
-__device__ bool m12_chain(const uint8_t* __restrict__ codes, uint32_t nd, uint8_t* __restrict__ em,
-                          const EncSym* s_tab, uint32_t& x, uint32_t& e) {
-    x = 65536;
-    e = 0;
-    bool ok = true;
-    const uint32_t full = nd & ~7u;  // codes [0, full) in aligned groups of eight
-    for (uint32_t i = nd; i > full && ok;) {
-        i--;
-        const uint32_t prev = i ? codes[i - 1] : 0u;
-        ok = m12_step(x, e, s_tab[s3_ctx(prev) * 64 + codes[i]], em);
-    }
-    for (int32_t g = (int32_t)(full / 8) - 1; g >= 0 && ok; g--) {
-        const uint2 w = *reinterpret_cast<const uint2*>(codes + 8 * g);
-        const uint32_t below = g ? codes[8 * g - 1] : 0u;
-        uint32_t c[8];
-#pragma unroll
-        for (int r = 0; r < 4; r++) {
-            c[r] = (w.x >> (8 * r)) & 0xFFu;
-            c[r + 4] = (w.y >> (8 * r)) & 0xFFu;
-        }
-        EncSym es[8];
-#pragma unroll
-        for (int r = 0; r < 8; r++) es[r] = s_tab[s3_ctx(r ? c[r - 1] : below) * 64 + c[r]];
-#pragma unroll
-        for (int r = 7; r >= 0; r--)
-            if (ok) ok = m12_step(x, e, es[r], em);
-    }
-    return ok;
-}
-
-// The Mode 12 chains of frames [j0, j0 + njobs), one thread each.  tab12:
-// the 4 x 64 static weights in EncSym form.
-__global__ void __launch_bounds__(32) k_s3_chain(const Job* __restrict__ jobs, uint32_t j0, uint32_t njobs,
-                                                 uint8_t* __restrict__ s3base, S3Frame* __restrict__ s3f,
-                                                 const EncSym* __restrict__ tab12) {
-    __shared__ EncSym s_tab[4 * 64];
-    for (uint32_t i = threadIdx.x; i < 4 * 64; i += 32) s_tab[i] = tab12[i];
+// The static weights as walk entries (4 x 64).
+__device__ __forceinline__ void m12_table(uint4* tab, const EncSym* __restrict__ tab12) {
+    for (uint32_t i = threadIdx.x & 31; i < 4 * 64; i += 32) tab[i] = walk_sym(tab12[i]);
     __syncwarp();
-    const uint32_t jl = blockIdx.x * 32 + threadIdx.x;
-    if (jl >= njobs) return;
-    const uint32_t j = j0 + jl;
-    const Job job = jobs[j];
-    if (job.profile < 2) return;
-    const uint32_t nd = s3f[j].nd;
-    if (nd == 0 || s3f[j].bad || nd > job.dist_cap) return;
-    uint32_t x, e;
-    const bool ok = m12_chain(s3base + job.s3_off, nd, s3base + job.s3_off + s3_em_off(job), s_tab, x, e);
-    s3f[j].m12e = ok ? e : 0xFFFFFFFFu;
-    s3f[j].m12x = x;
+}
+// The entry of code i (any entry where i is not below n).
+__device__ __forceinline__ uint4 m12_entry(const M12Task& t, uint32_t i, const uint4* tab) {
+    uint32_t at = 0;
+    if (i < t.n) at = s3_ctx(i ? t.codes[i - 1] : 0u) * 64 + t.codes[i];
+    return tab[at];
+}
+// Codes [lo, hi) from the last down, kN states a lane (lo a multiple of 32).
+template <int kN>
+__device__ __forceinline__ void m12_walk(uint32_t (&x)[kN], const M12Task& t, uint32_t lo, uint32_t hi, const uint4* tab,
+                                         uint4 (*s_e)[32]) {
+    const uint32_t lane = threadIdx.x & 31;
+    if (hi <= lo) return;
+    uint32_t at = (hi - 1) & ~31u, b = 0;  // blocks of 32 codes, the first perhaps short
+    uint4 nx = m12_entry(t, at + lane, tab);
+    for (uint32_t m = hi - at;; m = 32) {
+        s_e[b][lane] = nx;
+        __syncwarp();
+        if (at > lo) nx = m12_entry(t, at - 32 + lane, tab);
+        if (m == 32) {
+#pragma unroll 8
+            for (int q = 31; q >= 0; q--) {
+                const uint4 e = s_e[b][q];
+#pragma unroll
+                for (int i = 0; i < kN; i++) x[i] = walk_step<false>(x[i], e);
+            }
+        } else {
+            for (int q = (int)m - 1; q >= 0; q--) {
+                const uint4 e = s_e[b][q];
+#pragma unroll
+                for (int i = 0; i < kN; i++) x[i] = walk_step<false>(x[i], e);
+            }
+        }
+        if (at <= lo) break;
+        at -= 32;
+        b ^= 1;
+    }
+    __syncwarp();
+}
+
+// Block (x, y): the walkers of segment x of task y.
+template <class Tasks>
+__global__ void __launch_bounds__(32) k_m12_walk(Tasks tasks, M12Bufs mb, const EncSym* __restrict__ tab12) {
+    __shared__ uint4 s_tab[4 * 64];
+    __shared__ uint4 s_e[2][32];
+    __shared__ uint32_t s_w[32];
+    const M12Task t = tasks.get(blockIdx.y);
+    const uint32_t c = blockIdx.x, segs = m12_segs(t.n), lane = threadIdx.x;
+    if (segs < 2 || c >= segs) return;
+    m12_table(s_tab, tab12);
+    const uint32_t lo = c * kM12Seg, hi = min(lo + kM12Seg, t.n);
+    const bool from_end = hi + kM12Warm >= t.n;
+    uint32_t* marks = mb.marks + 64ull * (t.seg0 + c) + lane;
+    uint32_t x[1];
+    if (from_end) {
+        x[0] = 65536u;
+        m12_walk(x, t, hi, t.n, s_tab, s_e);
+    } else {
+        const uint32_t q4 = lane & 3, up = lane >> 2;
+        uint32_t xs[2] = {(q4 == 0 ? 65536u : q4 == 1 ? 77936u : q4 == 2 ? 92682u : 110218u) << up,
+                          (q4 == 0 ? 71468u : q4 == 1 ? 84990u : q4 == 2 ? 101070u : 120194u) << up};
+        m12_walk(xs, t, hi + kM12Warm - 512, hi + kM12Warm, s_tab, s_e);
+        x[0] = walk_halve(xs, s_w);
+        m12_walk(x, t, hi, hi + kM12Warm - 512, s_tab, s_e);
+    }
+    marks[0] = x[0];
+    m12_walk(x, t, lo, hi, s_tab, s_e);
+    marks[32] = x[0];
+}
+
+// Block b: the true first state of every segment of task b.
+template <class Tasks>
+__global__ void __launch_bounds__(32) k_m12_resolve(Tasks tasks, M12Bufs mb, const EncSym* __restrict__ tab12) {
+    __shared__ uint4 s_tab[4 * 64];
+    __shared__ uint4 s_e[2][32];
+    const M12Task t = tasks.get(blockIdx.x);
+    const uint32_t segs = m12_segs(t.n), lane = threadIdx.x;
+    if (segs < 2) return;
+    m12_table(s_tab, tab12);
+    const uint32_t* mk = mb.marks + 64ull * t.seg0 + lane;
+    uint32_t x[1] = {65536u};
+    uint32_t s = mk[64ull * (segs - 1)], e = mk[64ull * (segs - 1) + 32];
+    for (int32_t c = (int32_t)segs - 1; c >= 0; c--) {
+        const uint32_t sc = s, ec = e;
+        if (c > 0) {
+            s = mk[64ull * (c - 1)];
+            e = mk[64ull * (c - 1) + 32];
+        }
+        if (lane == 0) mb.first[t.seg0 + c] = x[0];
+        const uint32_t hit = __ballot_sync(0xFFFFFFFFu, sc == x[0]);
+        if (hit) x[0] = __shfl_sync(0xFFFFFFFFu, ec, __ffs(hit) - 1);
+        else m12_walk(x, t, c * kM12Seg, min((c + 1) * kM12Seg, t.n), s_tab, s_e);
+    }
+}
+
+// The bits of x at 0, 4, 8, ..., 28 as the even bits of 16.
+__device__ __forceinline__ uint32_t m12_even(uint32_t x) {
+    x &= 0x11111111u;
+    x = (x | (x >> 2)) & 0x05050505u;
+    x = (x | (x >> 4)) & 0x00550055u;
+    return (x | (x >> 8)) & 0x5555u;
+}
+
+// Block (x, y): segment x of task y coded from its true first state.
+template <class Tasks>
+__global__ void __launch_bounds__(32) k_m12_code(Tasks tasks, M12Bufs mb, const EncSym* __restrict__ tab12) {
+    __shared__ uint4 s_tab[4 * 64];
+    __shared__ uint4 s_e[32];
+    __shared__ uint32_t s_x[32];
+    const M12Task t = tasks.get(blockIdx.y);
+    const uint32_t c = blockIdx.x, segs = m12_segs(t.n), lane = threadIdx.x;
+    if (c >= segs) return;
+    m12_table(s_tab, tab12);
+    const uint32_t lo = segs > 1 ? c * kM12Seg : 0u, hi = segs > 1 ? min(lo + kM12Seg, t.n) : t.n;
+    uint32_t x = segs > 1 ? mb.first[t.seg0 + c] : 65536u, bytes = 0;
+    const LaneIO io = lane_io(t.base, t.cap, lane & 3);
+    uint16_t* raw = reinterpret_cast<uint16_t*>(io.bytes);
+    uint16_t* nbw = reinterpret_cast<uint16_t*>(io.nbw);  // eight rounds a half word
+    uint32_t at = (hi - 1) & ~31u;
+    uint4 nx = m12_entry(t, at + lane, s_tab);
+    for (uint32_t m = hi - at;; m = 32) {
+        const uint4 own = nx;
+        s_e[lane] = own;
+        __syncwarp();
+        if (at > lo) nx = m12_entry(t, at - 32 + lane, s_tab);
+        if (m == 32) {
+#pragma unroll 8
+            for (int q = 31; q >= 0; q--) {
+                const uint4 e = s_e[q];
+                s_x[q] = x;
+                x = walk_step<false>(x, e);
+            }
+        } else {
+            for (int q = (int)m - 1; q >= 0; q--) {
+                s_x[q] = x;
+                x = walk_step<false>(x, s_e[q]);
+            }
+        }
+        __syncwarp();
+        const uint32_t v = s_x[lane];
+        const bool in = lane < m;
+        const bool k1 = in && v >= own.y, k2 = in && (v >> 8) >= own.y;
+        if (in) raw[(at + lane) >> 2] = (uint16_t)v;
+        const uint32_t b1 = __ballot_sync(0xFFFFFFFFu, k1), b2 = __ballot_sync(0xFFFFFFFFu, k2);
+        bytes += __popc(b1) + __popc(b2);
+        // count 1: bit 0, count 2: bit 1 of a round's two bits
+        if (lane < 4) nbw[at >> 5] = (uint16_t)(m12_even((b1 & ~b2) >> lane) | (m12_even(b2 >> lane) << 1));
+        if (at <= lo) break;
+        at -= 32;
+        __syncwarp();
+    }
+    if (lane == 0) {
+        mb.bytes[t.seg0 + c] = bytes;
+        mb.last[t.seg0 + c] = x;
+    }
+}
+
+// Warp b of the grid: the totals of task b (bytes, last state) through
+// tasks.put, and the running counts of its record layout, all on lane 0.
+template <class Tasks>
+__global__ void __launch_bounds__(32) k_m12_sum(Tasks tasks, M12Bufs mb) {
+    const M12Task t = tasks.get(blockIdx.x);
+    const uint32_t segs = m12_segs(t.n), lane = threadIdx.x;
+    if (segs == 0) return;
+    constexpr uint32_t kPass = 4 * kStitchRounds / kM12Seg;  // segments of a stitch pass
+    uint32_t above = 0;
+    for (int32_t c0 = (int32_t)segs - 1; c0 >= 0; c0 -= 32) {
+        const int32_t c = c0 - (int32_t)lane;
+        uint32_t sum = c >= 0 ? mb.bytes[t.seg0 + c] : 0u;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, sum, o);
+            if (lane >= (uint32_t)o) sum += y;
+        }
+        if (c >= 0 && c % kPass == 0)
+            for (uint32_t l = 0; l < 4; l++) lane_io(t.base, t.cap, l).cum[c / kPass] = l == 0 ? above + sum : 0u;
+        above += __shfl_sync(0xFFFFFFFFu, sum, 31);
+    }
+    if (lane == 0) tasks.put(blockIdx.x, above, mb.last[t.seg0]);
+}
+
+// Lane totals of a Mode 12 chain's record layout, for stitch_offset.
+__device__ __forceinline__ TaskOut m12_out(uint32_t bytes) {
+    TaskOut o = {};
+    o.count[0] = bytes;
+    return o;
+}
+
+// The Mode 12 chains of frames j0, j0 + 1, ...
+struct M12Frames {
+    const Job* jobs;
+    uint8_t* s3base;
+    S3Frame* s3f;
+    const uint32_t* seg0;
+    uint32_t j0;
+    __device__ M12Task get(uint32_t i) const {
+        const uint32_t j = j0 + i;
+        const Job job = jobs[j];
+        M12Task t = {};
+        if (job.profile < 2) return t;
+        const S3Frame f = s3f[j];
+        t.codes = s3base + job.s3_off;
+        t.base = s3base + job.s3_off + s3_em_off(job);
+        t.cap = job.dist_cap;
+        t.n = f.bad || f.nd > job.dist_cap || f.nd > kS3Scratch ? 0u : f.nd;  // (others take the varint form)
+        t.seg0 = seg0[j];
+        return t;
+    }
+    __device__ void put(uint32_t i, uint32_t bytes, uint32_t state) const {
+        s3f[j0 + i].m12e = bytes > kS3Scratch ? 0xFFFFFFFFu : bytes;
+        s3f[j0 + i].m12x = state;
+    }
+};
+
+// The launches of n tasks with at most max_codes codes each.
+template <class Tasks>
+static cudaError_t launch_m12(const Tasks& tasks, uint32_t n, uint32_t max_codes, const M12Bufs& mb, const EncSym* tab12,
+                              cudaStream_t s) {
+    const uint32_t segs = m12_segs(max_codes);
+    for (uint32_t i0 = 0; i0 < n; i0 += 65535) {  // grid y is at most 65535
+        const uint32_t m = n - i0 < 65535 ? n - i0 : 65535;
+        Tasks part = tasks;
+        part.j0 += i0;
+        if (segs > 1) {
+            k_m12_walk<<<dim3(segs, m), 32, 0, s>>>(part, mb, tab12);
+            k_m12_resolve<<<m, 32, 0, s>>>(part, mb, tab12);
+        }
+        k_m12_code<<<dim3(segs ? segs : 1, m), 32, 0, s>>>(part, mb, tab12);
+        k_m12_sum<<<m, 32, 0, s>>>(part, mb);
+    }
+    return cudaGetLastError();
 }
 
 }  // namespace pz

@@ -436,9 +436,7 @@ __global__ void __launch_bounds__(kAsmThreads, 4) k_assemble(const uint8_t* __re
             const uint8_t* rb = s3base + job.s3_off;
             if (p.s3_code == 0) {  // Mode 12: 0x0C | LE32 state | the emitted bytes reversed
                 if (threadIdx.x == 0) { cs[0] = 0x0C; put32(cs + 1, fr.m12x); }
-                const uint8_t* em = rb + s3_em_off(job);
-                const uint32_t e = fr.m12e;
-                for (uint32_t k = threadIdx.x; k < e; k += blockDim.x) cs[5 + k] = em[e - 1 - k];
+                block_stitch<kAsmThreads>(rb + s3_em_off(job), job.dist_cap, nd, cs + 5);
             } else {
                 write_container(cs, 0x00, nd, infos + (uint64_t)j * kModels + 4, outs[(uint64_t)j * T_COUNT + T_S3],
                                 abase + ans_task_off(job, T_S3), task_cap(job, T_S3));
