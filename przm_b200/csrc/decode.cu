@@ -984,10 +984,11 @@ static_assert(4 * kShRow * 2 < 32768, "a cursor's offset is below 2^15");
 
 struct ShShared {
     uint16_t sel[4][kShRow];   // byte selector of the next fiber's cursor
-    uint16_t info[4][kShRow];  // literals taken, the next fiber << 8
+    uint16_t info[4][kShRow];  // literals taken, the next fiber << 4, its cursor's step << 8 if it is the same fiber
     uint8_t b[4][kShRing];     // the literals
-    uint16_t vis[2][kShVisits];  // visits: fiber, literals << 8
+    uint16_t vis[2][kShVisits];  // the info of the visits
     uint32_t cur[2][4];        // cursors before them
+    uint32_t first[2];         // the first one's fiber
     __align__(16) uint8_t out[kShMost + 32];
     uint32_t done, bad;
     ClassLut lut;
@@ -1017,7 +1018,7 @@ __device__ __forceinline__ void sh_fetch(ShShared& S, const uint8_t* fib, uint32
         const uint32_t c = q + i < len ? (uint32_t)S.lut.c[(v[i >> 2] >> (8 * (i & 3))) & 0xFFu] : k;
         if (c != k) { to = c; n = 0; }
         n++;
-        const uint32_t s = sh_sel(to) & 0xFFFFu, f = n | (to << 8);
+        const uint32_t s = sh_sel(to) & 0xFFFFu, f = n | (to << 4) | (to == k ? n << 9 : 0u);
         if (i & 1) { sel[i >> 1] = s << 16; inf[i >> 1] = f << 16; }
         else { sel[i >> 1] |= s; inf[i >> 1] |= f; }
     }
@@ -1037,7 +1038,9 @@ __device__ __forceinline__ uint32_t sh_place(ShShared& S, uint32_t buf, const ui
                                              uint32_t j, uint32_t n) {
     const uint32_t lane = threadIdx.x & 31, head = j & 15u;
     const uint32_t vv = reinterpret_cast<const uint32_t*>(S.vis[buf])[lane];
-    uint32_t f[2] = {vv & 3u, (vv >> 16) & 3u}, c[2] = {(vv >> 8) & 0xFFu, vv >> 24};
+    // a visit's fiber is the one the visit before it goes to
+    const uint32_t from = __shfl_up_sync(0xFFFFFFFFu, (vv >> 20) & 3u, 1);
+    uint32_t f[2] = {lane ? from : S.first[buf], (vv >> 4) & 3u}, c[2] = {vv & 15u, (vv >> 16) & 15u};
     uint32_t c01 = 0, c23 = 0;
 #pragma unroll
     for (int i = 0; i < 2; i++) {
@@ -1114,6 +1117,7 @@ __global__ void __launch_bounds__(64) k_dec_sheaf(DecInfo* __restrict__ infos) {
         const uint32_t buf = b & 1;
         if (chain) {
             if (lane < 4) S.cur[buf][lane] = lane == 0 ? cur[0] : lane == 1 ? cur[1] : lane == 2 ? cur[2] : cur[3];
+            if (lane == 0) S.first[buf] = f;
             uint32_t start[4];
 #pragma unroll
             for (uint32_t k = 0; k < 4; k++) start[k] = 2 * (k * kShRow + (cur[k] & (kShRing - 1)));
@@ -1121,17 +1125,25 @@ __global__ void __launch_bounds__(64) k_dec_sheaf(DecInfo* __restrict__ infos) {
                 uint32_t C0 = start[0] | (start[1] << 16), C1 = start[2] | (start[3] << 16), sel = sh_sel(f);
                 const uint8_t* ps = reinterpret_cast<const uint8_t*>(S.sel);
                 const uint8_t* pi = reinterpret_cast<const uint8_t*>(S.info);
+                // the cursors' registers lag one visit, so that the next
+                // fiber's is picked as soon as its selector is there; a visit
+                // that stays in its fiber brings the step along
+                uint32_t in = 0, p0 = 0, p1s = 0;
 #pragma unroll 8
                 for (uint32_t v = 0; v < kShVisits; v++) {
-                    const uint32_t at = dec_pick(C0, C1, sel);
+                    const uint32_t at = dec_pick(C0, C1, sel) + (in >> 8);
+                    C0 += p0;
+                    C1 += p1s;
                     sel = *reinterpret_cast<const uint16_t*>(ps + at);
-                    const uint32_t in = *reinterpret_cast<const uint16_t*>(pi + at), c = in & 0xFFu;
-                    const uint32_t t = (2 * c) << (16 * (f & 1u));
-                    if (f < 2) C0 += t;
-                    else C1 += t;
-                    if (lane == 0) S.vis[buf][v] = (uint16_t)(f | (c << 8));
-                    f = in >> 8;
+                    in = *reinterpret_cast<const uint16_t*>(pi + at);
+                    S.vis[buf][v] = (uint16_t)in;  // (all lanes alike)
+                    const uint32_t t = (in & 15u) << (1 + 16 * (f & 1u));
+                    p0 = f < 2 ? t : 0u;
+                    p1s = f < 2 ? 0u : t;
+                    f = (in >> 4) & 3u;
                 }
+                C0 += p0;
+                C1 += p1s;
                 cur[0] += ((C0 & 0xFFFFu) - start[0]) / 2;
                 cur[1] += ((C0 >> 16) - start[1]) / 2;
                 cur[2] += ((C1 & 0xFFFFu) - start[2]) / 2;
@@ -1146,8 +1158,8 @@ __global__ void __launch_bounds__(64) k_dec_sheaf(DecInfo* __restrict__ infos) {
                     cur[1] += f == 1;
                     cur[2] += f == 2;
                     cur[3] += f == 3;
-                    if (lane == 0) S.vis[buf][v] = (uint16_t)(f | (1u << 8));
                     f = class_lut(S.lut, p2, p1, 3);
+                    S.vis[buf][v] = (uint16_t)(1u | (f << 4));
                 }
             }
             total = cur[0] + cur[1] + cur[2] + cur[3];
