@@ -225,17 +225,21 @@ __device__ void warp_normalize_frequencies(const uint32_t* __restrict__ cnt /* s
     if (unique == 0) return;
     const int diff = 4096 - (int)(sum & 0xFFFF);
     if (diff > 0) {
-        // rank among active symbols by (count desc, symbol asc)
-        for (uint32_t s = lane; s < 256; s += 32) {
-            const uint32_t c = cnt[s];
-            if (!c) continue;
-            uint32_t rank = 0;
-            for (uint32_t t = 0; t < 256; t++) {
-                const uint32_t ct = cnt[t];
-                rank += (ct > c || (ct == c && ct != 0 && t < s)) ? 1 : 0;
-            }
-            if (rank < (uint32_t)diff) freq[s] = (uint16_t)(freq[s] + 1);
+        // rank among active symbols by (count desc, symbol asc), a lane's
+        // eight symbols against four counts at a time
+        uint32_t c[8], rank[8];
+#pragma unroll
+        for (uint32_t k = 0; k < 8; k++) { c[k] = cnt[lane + 32 * k]; rank[k] = 0; }
+        for (uint32_t t = 0; t < 256; t += 4) {
+            const uint32_t ct[4] = {cnt[t], cnt[t + 1], cnt[t + 2], cnt[t + 3]};
+#pragma unroll
+            for (uint32_t u = 0; u < 4; u++)
+#pragma unroll
+                for (uint32_t k = 0; k < 8; k++) rank[k] += ct[u] > c[k] || (ct[u] == c[k] && t + u < lane + 32 * k) ? 1 : 0;
         }
+#pragma unroll
+        for (uint32_t k = 0; k < 8; k++)
+            if (c[k] && rank[k] < (uint32_t)diff) freq[lane + 32 * k] = (uint16_t)(freq[lane + 32 * k] + 1);
     } else if (diff < 0 && lane == 0) {
         for (int it = 0; it < -diff; it++)
             for (int s = 255; s >= 0; s--)
@@ -292,11 +296,47 @@ __device__ void warp_build_table(const uint16_t* __restrict__ freq /* smem */, E
     uint32_t c = x - loc;
 #pragma unroll
     for (int k = 0; k < 8; k++) { tab[lane * 8 + k] = make_encsym(f[k], c); c += f[k]; }
-    if (lane == 0) {
-        uint32_t act = 0;
-        for (int s = 0; s < 256; s++) act += freq[s] ? 1 : 0;
-        info->active = act;
-        info->mat_len = serialize_matrix(freq, info->mat);
+    // serialize_matrix by the warp (one lane took 30 us): lane l has half a
+    // row, a row's first half also its two bytes of column mask
+    uint32_t cols = 0, len = 0;
+#pragma unroll
+    for (int k = 0; k < 8; k++)
+        if (f[k]) {
+            cols |= 1u << (8 * (lane & 1) + k);
+            len += f[k] < 128 ? 1 : 2;
+        }
+    const uint32_t act = __popc(cols);
+    cols |= __shfl_xor_sync(0xFFFFFFFFu, cols, 1);
+    const uint32_t present = __ballot_sync(0xFFFFFFFFu, cols != 0);
+    if (cols && (lane & 1) == 0) len += 2;
+    uint32_t at = len, total = act;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, at, o), z = __shfl_up_sync(0xFFFFFFFFu, total, o);
+        if (lane >= (uint32_t)o) {
+            at += y;
+            total += z;
+        }
+    }
+    if (lane == 31) {
+        info->active = total;
+        info->mat_len = 2 + at;
+    }
+    uint8_t* out = info->mat + 2 + at - len;
+    if (lane < 2) {  // the row mask: the even bits of the ballot
+        uint32_t rows = 0;
+        for (int h = 0; h < 8; h++) rows |= ((present >> (2 * (8 * lane + h))) & 1u) << h;
+        info->mat[lane] = (uint8_t)rows;
+    }
+    if (cols && (lane & 1) == 0) {
+        *out++ = (uint8_t)cols;
+        *out++ = (uint8_t)(cols >> 8);
+    }
+#pragma unroll
+    for (int k = 0; k < 8; k++) {
+        if (!f[k]) continue;
+        if (f[k] >= 128) *out++ = (uint8_t)(0x80 | (f[k] >> 8));
+        *out++ = (uint8_t)f[k];
     }
 }
 
