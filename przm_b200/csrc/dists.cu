@@ -218,7 +218,7 @@ template <class Tasks>
 __global__ void __launch_bounds__(32) k_m12_walk(Tasks tasks, M12Bufs mb, const EncSym* __restrict__ tab12) {
     __shared__ uint4 s_tab[4 * 64];
     __shared__ uint4 s_e[2][32];
-    __shared__ uint32_t s_w[32];
+    __shared__ uint32_t s_w[64];
     const M12Task t = tasks.get(blockIdx.y);
     const uint32_t c = blockIdx.x, segs = m12_segs(t.n), lane = threadIdx.x;
     if (segs < 2 || c >= segs) return;
@@ -231,11 +231,9 @@ __global__ void __launch_bounds__(32) k_m12_walk(Tasks tasks, M12Bufs mb, const 
         x[0] = 65536u;
         m12_walk(x, t, hi, t.n, s_tab, s_e);
     } else {
-        const uint32_t q4 = lane & 3, up = lane >> 2;
-        uint32_t xs[2] = {(q4 == 0 ? 65536u : q4 == 1 ? 77936u : q4 == 2 ? 92682u : 110218u) << up,
-                          (q4 == 0 ? 71468u : q4 == 1 ? 84990u : q4 == 2 ? 101070u : 120194u) << up};
+        uint32_t xs[2] = {walk_seed(2 * lane, 8), walk_seed(2 * lane + 1, 8)};
         m12_walk(xs, t, hi + kM12Warm - 512, hi + kM12Warm, s_tab, s_e);
-        x[0] = walk_halve(xs, s_w);
+        walk_pack<2, 1>(xs, x, s_w);
         m12_walk(x, t, hi, hi + kM12Warm - 512, s_tab, s_e);
     }
     marks[0] = x[0];

@@ -1026,22 +1026,46 @@ __device__ __forceinline__ uint32_t walk_slots(uint32_t x, uint32_t& slot, bool&
     return c;
 }
 
-// The distinct states of 64 in ring order (two a lane) when they are at most
-// 32, else every second one.
-__device__ __forceinline__ uint32_t walk_halve(const uint32_t (&xs)[2], uint32_t* __restrict__ s_w) {
+// The distinct ones of 32 kN states in ring order (kN a lane) packed into kM a
+// lane, ring order kept, when they are at most 32 kM; else an even choice of
+// them.  Returns their number.
+template <int kN, int kM>
+__device__ __forceinline__ uint32_t walk_pack(const uint32_t (&xs)[kN], uint32_t (&ys)[kM], uint32_t* __restrict__ s_w) {
     const uint32_t lane = threadIdx.x & 31;
-    const uint32_t prev = __shfl_sync(0xFFFFFFFFu, xs[1], (lane + 31) & 31);
-    const bool la = xs[0] != prev, lb = xs[1] != xs[0];
-    const uint32_t a = __ballot_sync(0xFFFFFFFFu, la), b = __ballot_sync(0xFFFFFFFFu, lb);
-    const uint32_t c = __popc(a) + __popc(b), lt = (1u << lane) - 1u;
-    if (c > 32 || c == 0) return xs[0];
-    const uint32_t at = __popc(a & lt) + __popc(b & lt);
-    if (la) s_w[at] = xs[0];
-    if (lb) s_w[at + la] = xs[1];
+    const uint32_t before = __shfl_sync(0xFFFFFFFFu, xs[kN - 1], (lane + 31) & 31);
+    uint32_t own = 0, lead = 0;
+#pragma unroll
+    for (int i = 0; i < kN; i++) {
+        const bool l = xs[i] != (i ? xs[i - 1] : before);
+        lead |= l ? 1u << i : 0u;
+        own += l;
+    }
+    uint32_t at = own;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, at, o);
+        if (lane >= (uint32_t)o) at += y;
+    }
+    const uint32_t c = max(1u, __shfl_sync(0xFFFFFFFFu, at, 31));
+    at -= own;
+    if (lane == 0) s_w[0] = xs[0];  // (one state in all: no leader)
     __syncwarp();
-    const uint32_t x = s_w[min(lane, c - 1)];
+#pragma unroll
+    for (int i = 0; i < kN; i++)
+        if ((lead >> i) & 1u) s_w[at++] = xs[i];
     __syncwarp();
-    return x;
+#pragma unroll
+    for (int i = 0; i < kM; i++) {
+        const uint32_t k = kM * lane + i;
+        ys[i] = s_w[c <= 32 * kM ? min(k, c - 1) : k * c / (32 * kM)];
+    }
+    __syncwarp();
+    return c;
+}
+// The eighths of a doubling, times 65536: state k of 32 kN spread evenly over
+// the logarithm of [2^16, 2^24).
+__device__ __forceinline__ uint32_t walk_seed(uint32_t k, uint32_t per_doubling) {
+    return (uint32_t)(exp2f((float)(k % per_doubling) / (float)per_doubling) * 65536.0f) << (k / per_doubling);
 }
 
 // The walkers of one segment: block b, segment b, warp l its lane l, all
@@ -1054,7 +1078,7 @@ __global__ void __launch_bounds__(kWalkThreads, kMeta8 ? 4 : 12) k_seg_walk(SegB
                                                                            const EncSym* __restrict__ meta8,
                                                                            const uint8_t* __restrict__ ctxlut) {
     extern __shared__ __align__(16) uint8_t smem_w[];
-    __shared__ uint32_t s_x[2][64], s_cnt[2][4], s_t[64], s_map[64], s_w[4][32];
+    __shared__ uint32_t s_x[2][64], s_cnt[2][4], s_t[64], s_map[64], s_w[4][64];
     const uint32_t nseg = sb.ctl[1];
     if (blockIdx.x >= nseg) return;
     const TaskDesc d = sb.segs[blockIdx.x];
@@ -1085,13 +1109,13 @@ __global__ void __launch_bounds__(kWalkThreads, kMeta8 ? 4 : 12) k_seg_walk(SegB
     WalkWords nx = walk_load<kMeta8>(d.src, vec, k, top);
     __syncthreads();
     walk_put<kMeta8>(stage + (k & 1) * 4 * kWalkStride, nx, lut);
-    // 64 states spread evenly over the logarithm of the range, eight to a
-    // doubling, two neighbours a thread; the first tile leaves about 25 of them
-    const uint32_t q4 = lane & 3, up = lane >> 2;
-    uint32_t xs[2] = {(q4 == 0 ? 65536u : q4 == 1 ? 77936u : q4 == 2 ? 92682u : 110218u) << up,
-                      (q4 == 0 ? 71468u : q4 == 1 ? 84990u : q4 == 2 ? 101070u : 120194u) << up};
+    // 64 states spread evenly over the logarithm of the range, two neighbours
+    // a thread until at most 32 are left: one tile on text, two or three on
+    // nearly uniform symbols (dropping every second state after the first tile
+    // instead left 3 % of their segments without the true one)
+    uint32_t xs[2] = {walk_seed(2 * lane, 8), walk_seed(2 * lane + 1, 8)};
     uint32_t x = from_end ? 65536u : xs[0];
-    bool two = !from_end;
+    uint32_t two = from_end ? 0u : 6u;  // tiles of two states a thread at most
     if (from_end && 4 * rounds + warp < d.n) {  // the stream's incomplete last round
         const uint32_t i = 4 * rounds + warp;
         uint32_t ti = d.src[i];
@@ -1109,10 +1133,11 @@ __global__ void __launch_bounds__(kWalkThreads, kMeta8 ? 4 : 12) k_seg_walk(SegB
             const uint16_t* st = stage + (b * 4 + l) * kWalkStride;
             const uint32_t cnt = min(kWalkTile, top - r0);
             if (two) {
+                uint32_t x1[1];
                 if (first_form) walk_tile<true, 2>(xs, st, cnt, smem_w);
                 else walk_tile<false, 2>(xs, st, cnt, smem_w);
-                x = walk_halve(xs, s_w[warp]);
-                two = false;
+                two = walk_pack<2, 1>(xs, x1, s_w[warp]) <= 32 ? 0u : two - 1;
+                x = x1[0];
             } else {
                 uint32_t x1[1] = {x};
                 if (first_form) walk_tile<true, 1>(x1, st, cnt, smem_w);
@@ -1125,7 +1150,7 @@ __global__ void __launch_bounds__(kWalkThreads, kMeta8 ? 4 : 12) k_seg_walk(SegB
         bool lead = false;
         if (mode == 0) {
             const uint32_t c = walk_slots<32>(x, ns, lead, last);
-            if (lane == 0) s_cnt[b][warp] = c;
+            if (lane == 0) s_cnt[b][warp] = two ? 32u : c;  // (not fewer warps yet)
         } else if (active) {
             s_x[b][tid] = x;
             if (mode == 1) {
