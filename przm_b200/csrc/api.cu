@@ -82,6 +82,12 @@ struct DevBuf {
     template <class T> T* as() const { return reinterpret_cast<T*>(p); }
 };
 
+// A part of a device buffer.
+struct DevPart {
+    void* p = nullptr;
+    template <class T> T* as() const { return reinterpret_cast<T*>(p); }
+};
+
 struct HostBuf {
     void* p = nullptr;
     size_t cap = 0;
@@ -146,17 +152,25 @@ struct przmg_batch {
     std::vector<uint2> asm_items;  // every frame's part 0 first, then the literal parts
     std::vector<uint64_t> in_offs, out_offs, up_offs;
     uint64_t in_bytes = 0, desc_words = 0, stream_bytes = 0, ans_bytes = 0, out_bytes = 0;
-    DevBuf d_in, d_jobs, d_small, d_big, d_tiles, d_desc, d_slots, d_tile_lens, d_streams, d_job_lens, d_hist, d_tabs,
-        d_infos, d_ans, d_outs, d_plans, d_sizes, d_out, d_misc, d_lists;
+    DevBuf d_in, d_desc, d_slots, d_tile_lens, d_streams, d_hist, d_tabs, d_infos, d_ans, d_outs, d_plans, d_out, d_misc,
+        d_lists;
+    // the tables that describe the batch, laid out by batch_prepare in one
+    // buffer and uploaded from h_layout by one copy (nine copies of a few
+    // hundred bytes and a wait cost a one-input call 70 us); the frame sizes
+    // and stream lengths lie behind them and start as zeros
+    DevBuf d_layout;
+    HostBuf h_layout;
+    bool layout_in_flight = false;  // h_layout may still be read by a copy on the context's stream
+    DevPart d_jobs, d_small, d_big, d_tiles, d_job_lens, d_sizes, d_rtiles, d_up_offs, d_asm, d_asm_job, d_m12_seg0;
     // radix-strike tables (one per finder CTA) and the packed upload/download
     // staging belong to the batch, so batches on different streams never
     // share scratch
-    DevBuf d_rtiles, d_rx_toff, d_rx_list, d_rx_pred, d_stage_in, d_stage_out, d_stage_offs, d_up_offs;
+    DevBuf d_rx_toff, d_rx_list, d_rx_pred, d_stage_in, d_stage_out, d_stage_offs;
     DevBuf d_tile_sched;  // tokenizer tile weights [0, ntiles) and walk order [ntiles, 2 ntiles)
-    DevBuf d_asm;         // assembly work items (frame, part)
-    DevBuf d_asm_job;     // the same items grouped by input (plain per-input launches)
+    // d_asm: assembly work items (frame, part); d_asm_job: the same items
+    // grouped by input (plain per-input launches)
     DevBuf d_s3, d_s3f;   // P2 and up: per-input Section 3 regions and their S3Frame facts
-    DevBuf d_m12, d_m12_seg0;  // P2 and up: the Mode 12 chains' segments, each input's first
+    DevBuf d_m12;  // P2 and up: the Mode 12 chains' segments (d_m12_seg0: each input's first)
     uint64_t m12_segs_total = 0;
     std::vector<uint32_t> m12_seg0;
     DevBuf d_fib;         // P3: per-input fiber regions
@@ -199,13 +213,13 @@ struct przmg_batch {
         graph = nullptr;
     }
     void release() {
-        DevBuf* all[] = {&d_in, &d_jobs, &d_small, &d_big, &d_tiles, &d_desc, &d_slots, &d_tile_lens, &d_streams,
-                         &d_job_lens, &d_hist, &d_tabs, &d_infos, &d_ans, &d_outs, &d_plans, &d_sizes, &d_out, &d_misc,
-                         &d_lists, &d_rtiles, &d_rx_toff, &d_rx_list, &d_rx_pred, &d_stage_in,
-                         &d_stage_out, &d_stage_offs, &d_up_offs, &d_tile_sched, &d_asm, &d_asm_job,
-                         &d_fitems, &d_ftiles, &d_ftarget, &d_fctl, &d_s3, &d_s3f, &d_m12, &d_m12_seg0, &d_fib, &d_seg};
+        DevBuf* all[] = {&d_in, &d_layout, &d_desc, &d_slots, &d_tile_lens, &d_streams, &d_hist, &d_tabs, &d_infos,
+                         &d_ans, &d_outs, &d_plans, &d_out, &d_misc, &d_lists, &d_rx_toff, &d_rx_list, &d_rx_pred,
+                         &d_stage_in, &d_stage_out, &d_stage_offs, &d_tile_sched, &d_fitems, &d_ftiles, &d_ftarget,
+                         &d_fctl, &d_s3, &d_s3f, &d_m12, &d_fib, &d_seg};
         for (DevBuf* b : all) b->release();
         h_offs.release();
+        h_layout.release();
     }
     uint32_t* err_word() const { return d_misc.as<uint32_t>(); }
 };
@@ -416,13 +430,7 @@ static int32_t batch_prepare(przmg_batch* b, const uint64_t* sizes, uint32_t njo
     b->ans_bytes = ans + 64;
     b->out_bytes = out + 64;
     CK(b->d_in.ensure(b->in_bytes));
-    CK(b->d_jobs.ensure(sizeof(Job) * std::max<uint32_t>(njobs, 1)));
-    CK(b->d_small.ensure(sizeof(TileRef) * std::max<uint32_t>(b->nsmall, 1)));
-    CK(b->d_big.ensure(sizeof(uint32_t) * std::max<uint32_t>(b->nbig, 1)));
-    CK(b->d_tiles.ensure(sizeof(TokTile) * std::max<size_t>(b->tiles.size(), 1)));
     CK(b->d_tile_sched.ensure(2 * sizeof(uint32_t) * std::max<size_t>(b->tiles.size(), 1)));
-    CK(b->d_asm.ensure(sizeof(uint2) * std::max<size_t>(b->asm_items.size(), 1)));
-    CK(b->d_asm_job.ensure(sizeof(uint2) * std::max<size_t>(asm_job.size(), 1)));
     if (b->front) {
         CK(b->d_fitems.ensure(sizeof(FrontItem) * fitems.size()));
         CK(b->d_ftiles.ensure(sizeof(TokTile) * std::max<size_t>(ftiles.size(), 1)));
@@ -433,7 +441,6 @@ static int32_t batch_prepare(przmg_batch* b, const uint64_t* sizes, uint32_t njo
     CK(b->d_slots.ensure((size_t)b->ntiles * kSlotStride));
     CK(b->d_tile_lens.ensure((size_t)b->ntiles * S_COUNT * 4));
     CK(b->d_streams.ensure(b->stream_bytes));
-    CK(b->d_job_lens.ensure((size_t)njobs * S_COUNT * 4 + 16));
     CK(b->d_hist.ensure((size_t)njobs * 1024 * 4 + 16));
     CK(b->d_tabs.ensure((size_t)njobs * kModels * 256 * sizeof(EncSym) + 16));
     CK(b->d_infos.ensure((size_t)njobs * kModels * sizeof(TableInfo) + 16));
@@ -441,10 +448,7 @@ static int32_t batch_prepare(przmg_batch* b, const uint64_t* sizes, uint32_t njo
     CK(b->d_s3f.ensure(sizeof(S3Frame) * std::max<uint32_t>(njobs, 1)));
     CK(b->d_fib.ensure(fib + 64));
     b->m12_segs_total = m12s;
-    if (profile >= 2) {
-        CK(b->d_m12.ensure(m12_buf_bytes(m12s)));
-        CK(b->d_m12_seg0.ensure(4ull * std::max<uint32_t>(njobs, 1)));
-    }
+    if (profile >= 2) CK(b->d_m12.ensure(m12_buf_bytes(m12s)));
     if (profile >= 2 && !b->aux) {
         CK(cudaStreamCreateWithFlags(&b->aux, cudaStreamNonBlocking));
         CK(cudaEventCreateWithFlags(&b->ev_fork, cudaEventDisableTiming));
@@ -453,16 +457,13 @@ static int32_t batch_prepare(przmg_batch* b, const uint64_t* sizes, uint32_t njo
     CK(b->d_ans.ensure(b->ans_bytes));
     CK(b->d_outs.ensure((size_t)njobs * T_COUNT * sizeof(TaskOut) + 16));
     CK(b->d_plans.ensure((size_t)njobs * sizeof(Plan) + 16));
-    CK(b->d_sizes.ensure((size_t)njobs * 4 + 16));
     CK(b->d_out.ensure(b->out_bytes));
     CK(b->d_misc.ensure(64));
     b->seg_cap = seg_cap(segb);
     b->seg_cap_m8 = std::min(seg_cap(segb_m8), b->seg_cap);
     CK(b->d_lists.ensure((size_t)2 * (kModels * std::max<uint32_t>(njobs, 1) + b->seg_cap) * sizeof(TaskDesc) + 64));
     CK(b->d_seg.ensure(seg_bytes(b->seg_cap)));
-    CK(b->d_up_offs.ensure(8ull * std::max<uint32_t>(njobs, 1) + 64));
     if (b->nbig) {
-        CK(b->d_rtiles.ensure(sizeof(RxTile) * std::max<size_t>(b->rtiles.size(), 1)));
         CK(b->d_rx_toff.ensure((size_t)b->ntiles * kRxParts * 4 + 64));
         CK(b->d_rx_list.ensure(b->desc_words * 4));
         CK(b->d_rx_pred.ensure(b->desc_words * 4));
@@ -470,29 +471,49 @@ static int32_t batch_prepare(przmg_batch* b, const uint64_t* sizes, uint32_t njo
     b->up_offs.assign(njobs, 0);
     for (uint32_t i = 1; i < njobs; i++) b->up_offs[i] = b->up_offs[i - 1] + b->jobs[i - 1].n;
     cudaStream_t s = setup ? setup : b->ctx->stream;
-    if (njobs) CK(cudaMemcpyAsync(b->d_up_offs.p, b->up_offs.data(), 8ull * njobs, cudaMemcpyHostToDevice, s));
-    if (!b->rtiles.empty())
-        CK(cudaMemcpyAsync(b->d_rtiles.p, b->rtiles.data(), sizeof(RxTile) * b->rtiles.size(), cudaMemcpyHostToDevice, s));
-    CK(cudaMemcpyAsync(b->d_jobs.p, b->jobs.data(), sizeof(Job) * njobs, cudaMemcpyHostToDevice, s));
-    if (b->nsmall) CK(cudaMemcpyAsync(b->d_small.p, b->small.data(), sizeof(TileRef) * b->nsmall, cudaMemcpyHostToDevice, s));
-    if (b->nbig) CK(cudaMemcpyAsync(b->d_big.p, b->big.data(), sizeof(uint32_t) * b->nbig, cudaMemcpyHostToDevice, s));
-    if (!b->tiles.empty())
-        CK(cudaMemcpyAsync(b->d_tiles.p, b->tiles.data(), sizeof(TokTile) * b->tiles.size(), cudaMemcpyHostToDevice, s));
-    if (!b->asm_items.empty())
-        CK(cudaMemcpyAsync(b->d_asm.p, b->asm_items.data(), sizeof(uint2) * b->asm_items.size(), cudaMemcpyHostToDevice, s));
-    if (!asm_job.empty())
-        CK(cudaMemcpyAsync(b->d_asm_job.p, asm_job.data(), sizeof(uint2) * asm_job.size(), cudaMemcpyHostToDevice, s));
+    if (b->layout_in_flight) {
+        CK(cudaStreamSynchronize(b->ctx->stream));
+        b->layout_in_flight = false;
+    }
+    const struct { DevPart* part; const void* src; size_t bytes; } tables[] = {
+        {&b->d_jobs, b->jobs.data(), sizeof(Job) * njobs},
+        {&b->d_up_offs, b->up_offs.data(), 8ull * njobs},
+        {&b->d_rtiles, b->rtiles.data(), sizeof(RxTile) * b->rtiles.size()},
+        {&b->d_small, b->small.data(), sizeof(TileRef) * b->nsmall},
+        {&b->d_big, b->big.data(), sizeof(uint32_t) * b->nbig},
+        {&b->d_tiles, b->tiles.data(), sizeof(TokTile) * b->tiles.size()},
+        {&b->d_asm, b->asm_items.data(), sizeof(uint2) * b->asm_items.size()},
+        {&b->d_asm_job, asm_job.data(), sizeof(uint2) * asm_job.size()},
+        {&b->d_m12_seg0, b->m12_seg0.data(), 4ull * njobs},
+        {&b->d_sizes, nullptr, 4ull * njobs + 16},
+        {&b->d_job_lens, nullptr, 4ull * njobs * S_COUNT + 16},
+    };
+    size_t layout = 0;
+    for (const auto& t : tables) layout += align64(t.bytes + 16);
+    CK(b->d_layout.ensure(layout));
+    CK(b->h_layout.ensure(layout));
+    size_t at = 0;
+    for (const auto& t : tables) {
+        uint8_t* h = b->h_layout.as<uint8_t>() + at;
+        if (t.src && t.bytes) std::memcpy(h, t.src, t.bytes);
+        if (!t.src) std::memset(h, 0, t.bytes);
+        t.part->p = b->d_layout.as<uint8_t>() + at;
+        at += align64(t.bytes + 16);
+    }
+    CK(cudaMemcpyAsync(b->d_layout.p, b->h_layout.p, layout, cudaMemcpyHostToDevice, s));
     if (b->front) {
         CK(cudaMemcpyAsync(b->d_fitems.p, fitems.data(), sizeof(FrontItem) * fitems.size(), cudaMemcpyHostToDevice, s));
         if (!ftiles.empty())
             CK(cudaMemcpyAsync(b->d_ftiles.p, ftiles.data(), sizeof(TokTile) * ftiles.size(), cudaMemcpyHostToDevice, s));
         CK(cudaMemcpyAsync(b->d_ftarget.p, ftarget.data(), 4ull * njobs, cudaMemcpyHostToDevice, s));
     }
-    if (profile >= 2 && njobs)
-        CK(cudaMemcpyAsync(b->d_m12_seg0.p, b->m12_seg0.data(), 4ull * njobs, cudaMemcpyHostToDevice, s));
-    CK(cudaMemsetAsync(b->d_sizes.p, 0, (size_t)njobs * 4 + 16, s));
-    CK(cudaMemsetAsync(b->d_job_lens.p, 0, (size_t)njobs * S_COUNT * 4 + 16, s));
-    // the host-side vectors above must stay alive until the copies ran
+    // The context's one-input batch runs on the stream of this copy; others
+    // may be enqueued on any stream, and the front end's tables come from
+    // vectors that end here.
+    if (b == &b->ctx->single && s == b->ctx->stream && !b->front) {
+        b->layout_in_flight = true;
+        return PRZMG_OK;
+    }
     CK(cudaStreamSynchronize(s));
     return PRZMG_OK;
 }
@@ -788,6 +809,7 @@ static int32_t batch_check(przmg_batch* b) {
     uint32_t err = 0;
     CK(cudaMemcpyAsync(&err, b->err_word(), 4, cudaMemcpyDeviceToHost, b->ctx->stream));
     CK(cudaStreamSynchronize(b->ctx->stream));
+    b->layout_in_flight = false;
     if (err) return device_error(err);
     return PRZMG_OK;
 }
@@ -1540,6 +1562,7 @@ static int32_t batch_download_packed(przmg_batch* b, uint8_t* host, uint64_t cap
     uint32_t err = 0;
     CK(cudaMemcpyAsync(&err, b->err_word(), 4, cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));
+    if (s == b->ctx->stream) b->layout_in_flight = false;
     if (err) return device_error(err);
     std::vector<uint64_t> offs(b->njobs);
     uint64_t t = 0;

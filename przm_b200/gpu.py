@@ -9,6 +9,7 @@ from __future__ import annotations
 
 import ctypes as C
 import os
+import threading
 from dataclasses import dataclass
 
 import numpy as np
@@ -60,6 +61,27 @@ def _u8(data) -> np.ndarray:
 
 def _ptr(a: np.ndarray):
     return C.c_void_p(a.ctypes.data) if a.size else C.c_void_p(0)
+
+
+class _Scratch(threading.local):
+    """A thread's output buffer for one-input calls: fresh pages for every
+    call's worst-case size cost more than the call of a few MiB itself.  At
+    most 34 MB (the bound of a 16 MiB input) is kept."""
+
+    KEEP = 34 << 20
+
+    def __init__(self):
+        self.buf = np.empty(0, np.uint8)
+
+    def get(self, n: int) -> np.ndarray:
+        if n > self.KEEP:
+            return np.empty(n, np.uint8)
+        if len(self.buf) < n:
+            self.buf = np.empty(min(max(n, 2 * len(self.buf)), self.KEEP), np.uint8)
+        return self.buf[:n]
+
+
+_SCRATCH = _Scratch()
 
 
 # ---- types (gpu/types.go) ---------------------------------------------------
@@ -464,7 +486,7 @@ class GPUCompressor:
         with a coded Section 3) or PROFILE_ANS_SHEAF (and a coded Section 4)."""
         a = _u8(src)
         cap = FrameBound(len(a))
-        out = np.zeros(cap, np.uint8)
+        out = _SCRATCH.get(cap)
         n = C.c_uint64()
         p = _lib.Profile()
         fn = L().przmg_compress_d2d if profile == PROFILE_D2D else None
@@ -472,7 +494,7 @@ class GPUCompressor:
             _check(fn(self._h, _ptr(a), len(a), _ptr(out), cap, C.byref(n), C.byref(p)))
         else:
             _check(L().przmg_compress(self._h, _ptr(a), len(a), profile, _ptr(out), cap, C.byref(n), C.byref(p)))
-        return bytes(out[: n.value]), GPUProfile.of(p)
+        return out[: n.value].tobytes(), GPUProfile.of(p)
 
     def CompressBatch(self, inputs, profile: int = PROFILE_ANS, batched: bool = True):
         """Many inputs in one call; returns (frames, statuses, profile)."""
@@ -601,10 +623,10 @@ class GPUCompressor:
             u = int(f[5]) | int(f[6]) << 8 | int(f[7]) << 16
         else:
             u = 0
-        out = np.zeros(max(u, 1), np.uint8)
+        out = _SCRATCH.get(max(u, 1))
         n = C.c_uint64()
         _check(L().przmg_decompress(self._h, _ptr(f) if len(f) else None, len(f), _ptr(out), len(out), C.byref(n)))
-        return bytes(out[: n.value])
+        return out[: n.value].tobytes()
 
     def DecompressBatchDevice(self, dSrc: int, srcOffs, srcLens, dDst: int, dstOffs, dstCaps,
                               stream: int = 0) -> tuple[np.ndarray, np.ndarray]:
