@@ -181,6 +181,7 @@ struct przmg_batch {
     // the two branches)
     cudaStream_t aux = nullptr;
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
+    cudaEvent_t ev_fork8 = nullptr, ev_join8 = nullptr;  // and around the walk of split Meta8 tasks
     // per input i, where its items start in each work list ([i + 1] = end)
     std::vector<uint32_t> job_small0, job_rt0, job_big0, job_tile0, job_asm0;
     int launches_plain = 0;
@@ -202,8 +203,8 @@ struct przmg_batch {
     ~przmg_batch() {
         drop_graph();
         release();
-        if (ev_fork) cudaEventDestroy(ev_fork);
-        if (ev_join) cudaEventDestroy(ev_join);
+        for (cudaEvent_t e : {ev_fork, ev_join, ev_fork8, ev_join8})
+            if (e) cudaEventDestroy(e);
         if (aux) cudaStreamDestroy(aux);
     }
     void drop_graph() {
@@ -449,10 +450,10 @@ static int32_t batch_prepare(przmg_batch* b, const uint64_t* sizes, uint32_t njo
     CK(b->d_fib.ensure(fib + 64));
     b->m12_segs_total = m12s;
     if (profile >= 2) CK(b->d_m12.ensure(m12_buf_bytes(m12s)));
-    if (profile >= 2 && !b->aux) {
+    if ((profile >= 2 || segb_m8) && !b->aux) {
+        for (cudaEvent_t* e : {&b->ev_fork, &b->ev_join, &b->ev_fork8, &b->ev_join8})
+            if (!*e) CK(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
         CK(cudaStreamCreateWithFlags(&b->aux, cudaStreamNonBlocking));
-        CK(cudaEventCreateWithFlags(&b->ev_fork, cudaEventDisableTiming));
-        CK(cudaEventCreateWithFlags(&b->ev_join, cudaEventDisableTiming));
     }
     CK(b->d_ans.ensure(b->ans_bytes));
     CK(b->d_outs.ensure((size_t)njobs * T_COUNT * sizeof(TaskOut) + 16));
@@ -577,14 +578,24 @@ static Range job_range(const przmg_batch* b, uint32_t i) {
 
 // The rANS launches of a task list: the walk and the resolution of its
 // segments (none without segment scratch), the coding, the segments' sums.
-// nb_ad, nb_m8: blocks that hold every adaptive and every Meta8 task;
-// m8_segs: Meta8 tasks may be split.
+// nb_ad, nb_m8: blocks that hold every adaptive and every Meta8 task.  Where
+// Meta8 tasks may be split (aux given) their walk runs beside the adaptive
+// one's on a second stream, forked and joined by the two events: it has few
+// segments, but as long ones (256 uneven files: 0.89 ms after the other's 1.48).
 static cudaError_t launch_rans(const SegBufs& sb, const TaskDesc* lists, uint32_t list_cap, const uint32_t* counts,
                                uint32_t nb_ad, uint32_t nb_m8, const EncSym* tabs, const EncSym* meta8,
-                               const uint8_t* ctxlut, TaskOut* outs, cudaStream_t s, bool m8_segs = false) {
+                               const uint8_t* ctxlut, TaskOut* outs, cudaStream_t s, cudaStream_t aux = nullptr,
+                               cudaEvent_t fork = nullptr, cudaEvent_t join = nullptr) {
+    cudaError_t e = cudaSuccess;
     if (sb.cap) {
+        if (aux) {
+            if ((e = cudaEventRecord(fork, s)) != cudaSuccess) return e;
+            if ((e = cudaStreamWaitEvent(aux, fork, 0)) != cudaSuccess) return e;
+            k_seg_walk<true><<<sb.cap, kWalkThreads, kWalkSmemM8, aux>>>(sb, tabs, meta8, ctxlut);
+            if ((e = cudaEventRecord(join, aux)) != cudaSuccess) return e;
+        }
         k_seg_walk<false><<<sb.cap, kWalkThreads, kWalkSmemAd, s>>>(sb, tabs, meta8, ctxlut);
-        if (m8_segs) k_seg_walk<true><<<sb.cap, kWalkThreads, kWalkSmemM8, s>>>(sb, tabs, meta8, ctxlut);
+        if (aux && (e = cudaStreamWaitEvent(s, join, 0)) != cudaSuccess) return e;
         k_seg_resolve<<<sb.cap / 2, 128, 0, s>>>(sb, tabs, meta8, ctxlut);
     }
     k_rans<<<nb_ad + nb_m8, kRansWarps * 32, kRansSmem, s>>>(lists, list_cap, counts, nb_ad, tabs, meta8, ctxlut, outs, sb);
@@ -741,7 +752,8 @@ static int32_t launch_range(przmg_batch* b, cudaStream_t s, int stop_after, cons
             const uint32_t nb_ad = (nad + b->seg_cap + 8 * kRansWarps - 1) / (8 * kRansWarps);
             const uint32_t nb_m8 = (3 * R.nj + b->seg_cap_m8 + 8 * kRansWarps - 1) / (8 * kRansWarps);
             CK(launch_rans(sb, lists, list_cap, counts, nb_ad, nb_m8, b->d_tabs.as<EncSym>(), c->d_meta8.as<EncSym>(),
-                           c->d_ctxlut.as<uint8_t>(), b->d_outs.as<TaskOut>(), s, b->seg_cap_m8 != 0));
+                           c->d_ctxlut.as<uint8_t>(), b->d_outs.as<TaskOut>(), s, b->seg_cap_m8 ? b->aux : nullptr,
+                           b->ev_fork8, b->ev_join8));
             launches += 3 + (sb.cap ? 3 + (b->seg_cap_m8 != 0) : 0);
             if (b->profile >= 2) CK(cudaStreamWaitEvent(s, b->ev_join, 0));  // the Mode 12 chains
             CK(mark(7));

@@ -75,3 +75,19 @@ def test_frames_with_long_command_streams(comp, oracle, profile, want):
     # records: op, meta and var streams long enough to be split, as Meta8 and adaptive tasks
     a = W.gen("records", 21, 2_500_007)
     assert comp.Compress(a, profile)[0] == getattr(oracle, want)(a)
+
+
+@pytest.mark.parametrize("graph", [False, True])
+def test_meta8_walk_beside_the_adaptive_one(comp, oracle, graph):
+    # new bytes in the same buffers: a walk not waited for would leave the last call's states
+    b = gpu.DeviceBatch(comp, [2_500_007, 900_001], gpu.PROFILE_ANS)
+    try:
+        for seed in (21, 22, 23):
+            xs = [W.gen("records", seed, 2_500_007), W.gen("records", seed + 50, 900_001)]
+            for x, o in zip(xs, b.in_offs):
+                devmem.upload_to(b.d_in + int(o), x)
+            b.enqueue(graph=graph)
+            for x, o, n in zip(xs, b.out_offs, b.frame_sizes()):
+                assert devmem.download(b.d_out + int(o), int(n)) == oracle.compress_p1(x)
+    finally:
+        b.close()
