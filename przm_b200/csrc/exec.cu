@@ -19,7 +19,12 @@
 // k_dec_exec_serial.
 //
 // Measured on 128 mixed frames of 1 MiB: 26.0 ms with one warp walking each
-// frame, 1.8 ms so.
+// frame, 1.5 ms so.  A chunk's 16 000 cycles (of 34 000 with its copies, on the
+// frames of the shortest commands) went into chains of loads, four block sums
+// and the scan of the distances, 5 000 alone when its maps held four words
+// each; maps of four bytes, three sums of one barrier, and the next chunk's
+// first loads beside the copies: 1.83 -> 1.50 ms.  Registers for two blocks an
+// SM: 300 record frames of 150 kB 1.53 -> 1.40 ms (the call), 128 of 1 MiB alike.
 #include "common.cuh"
 
 namespace pz {
@@ -33,6 +38,10 @@ constexpr uint32_t kExCap = 1u << 26;           // sums of lengths saturate here
 // how the walk ends at a command
 enum ExecEvent : uint32_t { EV_BEFORE = 0, EV_AFTER = 1, EV_CORRUPT = 2, EV_UNSUPPORTED = 3, EV_SERIAL = 4, EV_NONE = 15 };
 
+struct ExecSums {  // of the warps, for a sum over the block
+    uint32_t a[kExThreads / 32], b[kExThreads / 32];
+};
+
 struct ExecShared {
     uint32_t start[kExThreads + 1];  // a command's first output byte
     uint32_t lend[kExThreads];       // the end of its literals
@@ -40,8 +49,11 @@ struct ExecShared {
     uint32_t dist[kExThreads];       // its match's distance; 0: a run of literal lsrc
     uint16_t vend[kExThreads], oend[kExThreads];  // ends of the chunk's varints in their windows
     __align__(16) uint16_t w[kExTile];            // a tile's bytes: 0x8000 | byte, or a place in the tile
-    uint32_t warp[32], warp2[32];
-    uint32_t rep[kExThreads / 32 + 1][4];
+    ExecSums sums[2];
+    uint32_t vars[kExThreads / 32];    // varints of a warp's commands
+    uint32_t rep[128 + kExThreads / 8];  // the repeat distances before the chunk; from 128 four of every warp
+    uint32_t rmap[kExThreads / 32];
+    uint8_t tok[kExThreads];           // the next bytes of the token stream
     uint32_t vwin[kExThreads], owin[kExThreads];  // the bytes of the chunk's varints
     uint16_t pos[kExThreads + 1];  // flat: where the chunk's commands start
     uint32_t npos;
@@ -51,8 +63,9 @@ struct ExecShared {
 };
 
 // Two sums at once over the block, each saturating at kExCap: the sums before
-// this thread in a and b, the totals in ta and tb.
-__device__ __forceinline__ void exec_scan2(uint32_t& a, uint32_t& b, uint32_t& ta, uint32_t& tb, ExecShared& S) {
+// this thread in a and b, the totals in ta and tb.  One barrier: another call
+// meanwhile takes another W.
+__device__ __forceinline__ void exec_scan2(uint32_t& a, uint32_t& b, uint32_t& ta, uint32_t& tb, ExecSums& W) {
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     uint32_t x = min(a, kExCap), y = min(b, kExCap);
 #pragma unroll
@@ -64,46 +77,49 @@ __device__ __forceinline__ void exec_scan2(uint32_t& a, uint32_t& b, uint32_t& t
         }
     }
     if (lane == 31) {
-        S.warp[warp] = x;
-        S.warp2[warp] = y;
+        W.a[warp] = x;
+        W.b[warp] = y;
     }
     const uint32_t ex = __shfl_up_sync(0xFFFFFFFFu, x, 1), ey = __shfl_up_sync(0xFFFFFFFFu, y, 1);
     __syncthreads();
-    uint32_t bx = 0, by = 0;
+    a = lane ? ex : 0u;
+    b = lane ? ey : 0u;
     ta = tb = 0;
 #pragma unroll
-    for (uint32_t w = 0; w < kExThreads / 32; w++) {
-        if (w == warp) {
-            bx = ta;
-            by = tb;
+    for (uint32_t w = 0; w < kExThreads / 32; w++) {  // (16 sums of at most kExCap: no carry)
+        const uint32_t p = W.a[w], q = W.b[w];
+        if (w < warp) {
+            a += p;
+            b += q;
         }
-        ta = min(ta + S.warp[w], kExCap);
-        tb = min(tb + S.warp2[w], kExCap);
+        ta += p;
+        tb += q;
     }
-    a = min(bx + (lane ? ex : 0u), kExCap);
-    b = min(by + (lane ? ey : 0u), kExCap);
-    __syncthreads();
+    a = min(a, kExCap);
+    b = min(b, kExCap);
+    ta = min(ta, kExCap);
+    tb = min(tb, kExCap);
 }
 
-// A map of the four repeat distances: entry i a distance, or kRepFrom | j, the
-// j-th before.
-constexpr uint32_t kRepFrom = 0x80000000u;
-struct RepMap {
-    uint32_t e[4];
-};
-__device__ __forceinline__ uint32_t rep_of(const RepMap& a, uint32_t v) {
-    const uint32_t j = v & 3u;
-    const uint32_t s = j == 0 ? a.e[0] : j == 1 ? a.e[1] : j == 2 ? a.e[2] : a.e[3];
-    return (v & kRepFrom) ? s : v;
+// A map of the four repeat distances, a byte each: 0x80 | where a new distance
+// stands, or j, the j-th before.  A command moves one to the front or pushes a
+// new one; two maps are composed by a byte permute.
+constexpr uint32_t kRepSame = 0x03020100u;
+__device__ __forceinline__ uint32_t rep_then(uint32_t a, uint32_t b) {  // a, then b
+    const uint32_t m = ((b >> 7) & 0x01010101u) * 0xFFu;
+    uint32_t s = (b & ~m) | (0x07060504u & m);  // new distances are taken from b, the others from a
+    s |= s >> 4;
+    return __byte_perm(a, b, __byte_perm(s, 0u, 0x4420));
 }
-__device__ __forceinline__ RepMap rep_then(const RepMap& a, const RepMap& b) {  // a, then b
-    RepMap r;
+// The maps of this lane and all lanes before it, one after another.
+__device__ __forceinline__ uint32_t rep_scan(uint32_t x) {
+    const uint32_t lane = threadIdx.x & 31;
 #pragma unroll
-    for (int i = 0; i < 4; i++) r.e[i] = rep_of(a, b.e[i]);
-    return r;
-}
-__device__ __forceinline__ RepMap rep_identity() {
-    return RepMap{{kRepFrom | 0u, kRepFrom | 1u, kRepFrom | 2u, kRepFrom | 3u}};
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t a = __shfl_up_sync(0xFFFFFFFFu, x, o);
+        if (lane >= (uint32_t)o) x = rep_then(a, x);
+    }
+    return x;
 }
 
 // Varint of len (1-4) bytes at p.
@@ -115,17 +131,20 @@ __device__ __forceinline__ uint32_t exec_varint(const uint8_t* p, uint32_t len) 
     return r;
 }
 
-// Bytes [at + 4 tid, ...+ 4) of s[0, n), 0x80 past its end, into win: which of
-// them end a varint.
-__device__ __forceinline__ uint32_t exec_window(const uint8_t* s, uint32_t at, uint32_t n, uint32_t* win) {
+// Bytes [at + 4 tid, ...+ 4) of s[0, n), 0x80 past its end, and which of such
+// bytes end a varint.
+__device__ __forceinline__ uint32_t exec_word(const uint8_t* s, uint32_t at, uint32_t n) {
     const uint32_t p = at + 4 * threadIdx.x;
-    uint32_t w = 0x80808080u, m = 0;
+    uint32_t w = 0x80808080u;
     if (p + 4 <= n) {
         w = (uint32_t)s[p] | ((uint32_t)s[p + 1] << 8) | ((uint32_t)s[p + 2] << 16) | ((uint32_t)s[p + 3] << 24);
     } else {
         for (uint32_t i = 0; p + i < n; i++) w ^= (0x80u ^ s[p + i]) << (8 * i);
     }
-    win[threadIdx.x] = w;
+    return w;
+}
+__device__ __forceinline__ uint32_t exec_ends(uint32_t w) {
+    uint32_t m = 0;
 #pragma unroll
     for (uint32_t i = 0; i < 4; i++) m |= ((w >> (8 * i + 7)) & 1u) << i;
     return m ^ 15u;
@@ -297,7 +316,7 @@ __device__ void exec_copy(ExecShared& S, uint8_t* dst, const uint8_t* __restrict
     }
 }
 
-__global__ void __launch_bounds__(kExThreads) k_dec_exec(const uint8_t* __restrict__ src, const DecJob* __restrict__ jobs,
+__global__ void __launch_bounds__(kExThreads, 2) k_dec_exec(const uint8_t* __restrict__ src, const DecJob* __restrict__ jobs,
                                                          DecInfo* __restrict__ infos, uint8_t* __restrict__ out) {
     __shared__ ExecShared S;
     const uint32_t f = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -320,9 +339,21 @@ __global__ void __launch_bounds__(kExThreads) k_dec_exec(const uint8_t* __restri
     const bool split = I.cmd_mode == 1;
     const uint32_t jlim = split ? I.cmd_orig : cl;
     uint32_t cp = 0, mp = 0, vp = 0, j = 0, lp = 0, dp = 0, op0 = 0;
-    RepMap reps;
-    if ((I.flags & 0x01) && I.stride > 1) reps = RepMap{{1, I.stride, 2 * I.stride, 3 * I.stride}};
-    else reps = RepMap{{1, 4, 8, 16}};
+    if (tid < 4) {
+        const bool st = (I.flags & 0x01) && I.stride > 1;
+        S.rep[tid] = st ? (tid ? tid * I.stride : 1u) : (tid ? 2u << tid : 1u);
+    }
+    // the chunk's first bytes of each stream, loaded while the one before is copied
+    uint32_t pre_op = 0, pre_tok = 0, pre_var = 0, pre_off = 0;
+    auto fetch = [&]() {
+        if (split) {
+            pre_op = cp + tid < cl ? cs[cp + tid] : 0u;
+            pre_tok = mp + tid < ml ? ms[mp + tid] : 0u;
+            pre_var = exec_word(vs, vp, vl);
+        }
+        pre_off = exec_word(offs, op0, ol);
+    };
+    fetch();
     for (;;) {
         // the chunk's commands: the next 512 opcodes, or in a flat stream the
         // commands that one thread finds in its next bytes
@@ -361,7 +392,7 @@ __global__ void __launch_bounds__(kExThreads) k_dec_exec(const uint8_t* __restri
         uint32_t ev = EV_NONE, op = 0, m = 0, isvar = 0, isexp = 0, kind = 0, k = 0, llit = 0, lmatch = 0;
         bool bad = false;
         if (tid < n) {
-            op = cs[at];
+            op = split ? pre_op : cs[at];
             if (op < 0x80u) {
                 llit = (op >> 4) & 7u; lmatch = ((op >> 2) & 3u) + bmin; k = op & 3u; kind = 1;
             } else if (op < 0xC0u) {
@@ -378,22 +409,29 @@ __global__ void __launch_bounds__(kExThreads) k_dec_exec(const uint8_t* __restri
             }
         }
         // operands: tokens, then the varints that the opcodes and tokens ask for
-        uint32_t tot;
-        const uint32_t s1 = block_exclusive_scan<kExThreads>(m | (isexp << 16), S.warp, tot);
-        const uint32_t mi = s1 & 0xFFFFu, ei = s1 >> 16, nexp = tot >> 16;
+        const uint32_t vm = split ? exec_ends(pre_var) : 0u, em = exec_ends(pre_off);
+        S.vwin[tid] = pre_var;
+        S.owin[tid] = pre_off;
+        S.tok[tid] = (uint8_t)pre_tok;
+        uint32_t s1 = m | (isexp << 12), s2 = __popc(vm) | (__popc(em) << 12), t1, t2;
+        exec_scan2(s1, s2, t1, t2, S.sums[0]);  // (fields of at most 512 and 2048, all below kExCap)
+        const uint32_t mi = s1 & 0xFFFu, ei = s1 >> 12, nexp = t1 >> 12, nv = t2 & 0xFFFu, ne = t2 >> 12;
         const uint32_t mt = split ? mp + mi : at + 1;
         if (m) {
             uint32_t tok = 0;
-            if (mt < (split ? ml : cl)) tok = (split ? ms : cs)[mt];
+            if (mt < (split ? ml : cl)) tok = split ? S.tok[mi] : cs[mt];
             else bad = true;
             llit = tok >> 4; lmatch = (tok & 15u) + bmin; isvar = (tok & 15u) == 15u && !bad;
         }
-        const uint32_t em = exec_window(offs, op0, ol, S.owin), vm = split ? exec_window(vs, vp, vl, S.vwin) : 0u;
-        const uint32_t s2 = block_exclusive_scan<kExThreads>(__popc(vm) | (__popc(em) << 16), S.warp, tot);
-        const uint32_t nv = tot & 0xFFFFu, ne = tot >> 16;
-        exec_put_ends(S.vend, vm, s2 & 0xFFFFu);
-        exec_put_ends(S.oend, em, s2 >> 16);
-        const uint32_t vi = block_exclusive_scan<kExThreads>(isvar, S.warp, tot);  // (its barriers publish the ends)
+        exec_put_ends(S.vend, vm, s2 & 0xFFFu);
+        exec_put_ends(S.oend, em, s2 >> 12);
+        const uint32_t vb = __ballot_sync(0xFFFFFFFFu, isvar);
+        if (lane == 0) S.vars[warp] = __popc(vb);
+        __syncthreads();  // the ends too
+        uint32_t vi = __popc(vb & ((1u << lane) - 1u));
+#pragma unroll
+        for (uint32_t w = 0; w < kExThreads / 32; w++)
+            if (w < warp) vi += S.vars[w];
         uint32_t vlen = 0, vbefore = 0, vval = 0;
         if (split) {
             if (vi) vbefore = S.vend[vi - 1];
@@ -429,56 +467,28 @@ __global__ void __launch_bounds__(kExThreads) k_dec_exec(const uint8_t* __restri
         // literals and output before the command
         uint32_t li = llit + (kind == 4), oi = llit + (kind ? lmatch : 0u), tl, to;
         if (tid >= n) li = oi = 0;
-        exec_scan2(li, oi, tl, to, S);
+        exec_scan2(li, oi, tl, to, S.sums[1]);
         li += lp;
         oi += dp;
         // the repeat distances before it
-        RepMap own = rep_identity();
-        if (kind == 1) {
-            own.e[0] = kRepFrom | k;
-            if (k >= 1) own.e[1] = kRepFrom | 0u;
-            if (k >= 2) own.e[2] = kRepFrom | 1u;
-            if (k >= 3) own.e[3] = kRepFrom | 2u;
-        } else if (kind == 3) {
-            own = RepMap{{d, kRepFrom | 0u, kRepFrom | 1u, kRepFrom | 2u}};
+        uint32_t own = kRepSame;
+        if (kind == 1) own = k == 0 ? kRepSame : k == 1 ? 0x03020001u : k == 2 ? 0x03010002u : 0x02010003u;
+        else if (kind == 3) own = 0x02010080u | lane;
+        const uint32_t inc = rep_scan(own), up = __shfl_up_sync(0xFFFFFFFFu, inc, 1), last = __shfl_sync(0xFFFFFFFFu, inc, 31);
+        const uint32_t mine = ((lane ? up : kRepSame) >> (8 * k)) & 0xFFu;  // (kind 1: its distance)
+        const uint32_t dn = __shfl_sync(0xFFFFFFFFu, d, mine & 31u);
+        const uint32_t dw = __shfl_sync(0xFFFFFFFFu, d, (last >> (8 * (lane & 3u))) & 31u);
+        if (lane < 4) S.rep[128 + 4 * warp + lane] = dw;  // the warp's new distances
+        if (lane == 0) {
+            const uint32_t nw = ((last >> 7) & 0x01010101u) * 0xFFu;
+            S.rmap[warp] = (last & ~nw) | (((0x80u | warp << 2) * 0x01010101u | kRepSame) & nw);
         }
-        RepMap inc = own;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            RepMap a;
-#pragma unroll
-            for (int i = 0; i < 4; i++) a.e[i] = __shfl_up_sync(0xFFFFFFFFu, inc.e[i], o);
-            if (lane >= (uint32_t)o) inc = rep_then(a, inc);
-        }
-        if (lane == 31) {
-#pragma unroll
-            for (int i = 0; i < 4; i++) S.rep[warp][i] = inc.e[i];
-        }
-        RepMap before;
-#pragma unroll
-        for (int i = 0; i < 4; i++) before.e[i] = __shfl_up_sync(0xFFFFFFFFu, inc.e[i], 1);
-        if (lane == 0) before = rep_identity();
         if (tid == 0) S.event = 0xFFFFFFFFu;
         __syncthreads();
-        if (warp == 0) {  // the maps of the warps before each, from the distances before the chunk
-            constexpr uint32_t kW = kExThreads / 32;
-            RepMap a;
-            for (int i = 0; i < 4; i++) a.e[i] = lane == 0 || lane > kW ? reps.e[i] : S.rep[lane - 1][i];
-#pragma unroll
-            for (int o = 1; o <= (int)kW; o <<= 1) {
-                RepMap b;
-                for (int i = 0; i < 4; i++) b.e[i] = __shfl_up_sync(0xFFFFFFFFu, a.e[i], o);
-                if (lane >= (uint32_t)o) a = rep_then(b, a);
-            }
-            __syncwarp();
-            if (lane <= kW)
-                for (int i = 0; i < 4; i++) S.rep[lane][i] = a.e[i];
-        }
-        __syncthreads();
-        const RepMap base = RepMap{{S.rep[warp][0], S.rep[warp][1], S.rep[warp][2], S.rep[warp][3]}};
-        const RepMap all = RepMap{{S.rep[kExThreads / 32][0], S.rep[kExThreads / 32][1], S.rep[kExThreads / 32][2],
-                                   S.rep[kExThreads / 32][3]}};
-        if (kind == 1) d = rep_of(base, rep_of(before, kRepFrom | k));
+        const uint32_t warps = rep_scan(lane < kExThreads / 32 ? S.rmap[lane] : kRepSame);
+        const uint32_t all = __shfl_sync(0xFFFFFFFFu, warps, 31), pre = __shfl_sync(0xFFFFFFFFu, warps, warp ? warp - 1 : 0);
+        if (kind == 1) d = mine & 0x80u ? dn : S.rep[((warp ? pre : kRepSame) >> (8 * mine)) & 0xFFu];
+        const uint32_t rep = tid < 4 ? S.rep[(all >> (8 * tid)) & 0xFFu] : 0u;  // after the chunk
         // how the walk fares at this command
         if (tid > n) {
             ev = EV_NONE;
@@ -510,6 +520,7 @@ __global__ void __launch_bounds__(kExThreads) k_dec_exec(const uint8_t* __restri
             return;
         }
         const uint32_t E = type == EV_AFTER ? e + 1 : e;
+        if (tid < 4) S.rep[tid] = rep;
         if (tid < E) {
             S.start[tid] = oi;
             S.lend[tid] = kind == 4 ? oi : oi + llit;
@@ -528,8 +539,18 @@ __global__ void __launch_bounds__(kExThreads) k_dec_exec(const uint8_t* __restri
             S.start[E] = S.st[5];
         }
         __syncthreads();
-        const uint32_t end = S.st[5];
-        exec_copy(S, dst, lit, dp, end, E);
+        const uint32_t from = dp, end = S.st[5];
+        if (type == EV_NONE) {
+            mp = S.st[1];
+            vp = S.st[2];
+            j = S.st[3];
+            lp = S.st[4];
+            dp = end;
+            cp = split ? S.st[0] : cp + S.pos[n];
+            op0 += nexp ? S.oend[nexp - 1] : 0u;
+            fetch();
+        }
+        exec_copy(S, dst, lit, from, end, E);
         if (type != EV_NONE) {
             if (tid == 0) {
                 uint32_t err = end == u ? D_OK : D_CORRUPT;
@@ -553,14 +574,6 @@ __global__ void __launch_bounds__(kExThreads) k_dec_exec(const uint8_t* __restri
             }
             return;
         }
-        mp = S.st[1];
-        vp = S.st[2];
-        j = S.st[3];
-        lp = S.st[4];
-        dp = end;
-        cp = split ? S.st[0] : cp + S.pos[n];
-        op0 += nexp ? S.oend[nexp - 1] : 0u;
-        reps = all;
         __syncthreads();  // the next chunk rewrites the shared state
     }
 }
