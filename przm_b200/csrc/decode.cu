@@ -12,11 +12,10 @@
 //                  chain on lane 0, one symbol at a time (each symbol's
 //                  context is the symbol before it);
 //   k_dec_lists    the adaptive V-ANS bodies, longest first;
-//   k_dec_adaptive eight bodies per warp: a group of four lanes per body,
-//                  lane l holding interleaved state l; the four states share
-//                  one stream pointer, so each round of four symbols waits
-//                  for the one before it (matrix -> frequencies -> model,
-//                  built by the warp).
+//   k_dec_adaptive one body per warp, eight lanes for each of its four
+//                  interleaved states; they share one stream pointer, so each
+//                  round of four symbols waits for the one before it (matrix
+//                  -> frequencies -> model, built by the warp).
 //   k_dec_prefix   one block per frame with a distance-prefix Section 3:
 //                  extra-bit offsets and varint lengths by block scans, the
 //                  distances rebuilt and written as LEB128 varints.
@@ -567,11 +566,13 @@ __global__ void __launch_bounds__(1024) k_dec_lists(const DecTask* __restrict__ 
 
 // One adaptive body per warp (entry blockIdx.x of the list, longest first: the
 // long bodies then start on different SMs; taken by task slot, those of 128
-// frames shared 37 SMs), for batches whose bodies all fit on the SMs at once;
-// k_dec_adaptive takes eight bodies per warp when there are many.  The body's four states
-// are held by eight lanes each (a branch around 28 idle lanes would cost each
-// vote a convergence check), which run up to 64 rounds of four symbols at a
-// time; then the lanes turn the rounds' slots into symbols, write them, and
+// frames shared 37 SMs).  Eleven such warps fit an SM, whose issue slots they
+// then fill; eight bodies per warp, four lanes each, took longer at every
+// number of frames (the call, mixed data: 640 frames of 4-128 KiB 7.2 ms
+// against 2.1, 3000 of 30-200 kB 14.5 against 5.3, 10000 of 1-4 KiB 1.71
+// against 1.57).  The body's four states are held by eight lanes each (a
+// branch around 28 idle lanes would cost each vote a convergence check), which
+// run up to 64 rounds of four symbols at a time; then the lanes turn the rounds' slots into symbols, write them, and
 // put the next stream bytes into the ring (their loads in flight since the
 // rounds before).  A state needs 0, 1 or 2 bytes (x < 2^16, x < 2^8 after the
 // step, the reference's loop), in the order of the states.  Two ballots of
@@ -581,8 +582,8 @@ __global__ void __launch_bounds__(1024) k_dec_lists(const DecTask* __restrict__ 
 // cycles by the instructions' latencies (table load 25, step 12, compare and
 // vote 17, byte selection 28, address 8), 100 in a one-warp loop, against 177
 // there with the stream read from global memory, a symbol stored each round
-// and population counts (27.4 ms for 128 mixed frames of 1 MiB).  Tried in
-// that loop: thresholds for the votes beside the table entry (8 bytes an
+// and population counts (128 mixed frames of 1 MiB: 27.4 ms so, 13.6 now).
+// Tried in that loop: thresholds for the votes beside the table entry (8 bytes an
 // entry) 124, all offsets of a state tried on eight lanes and the right one
 // shuffled in 178, the four states in one thread 215.
 constexpr uint32_t kDecRing = 2048, kDecRounds = 64;
@@ -621,7 +622,7 @@ __device__ __forceinline__ uint32_t dec1_rounds(Dec1Shared& S, uint32_t& x, uint
     return q;
 }
 
-__global__ void __launch_bounds__(32) k_dec_adaptive1(const DecTask* __restrict__ tasks, const uint32_t* __restrict__ list,
+__global__ void __launch_bounds__(32) k_dec_adaptive(const DecTask* __restrict__ tasks, const uint32_t* __restrict__ list,
                                                       DecInfo* __restrict__ infos) {
     __shared__ __align__(16) Dec1Shared S;
     if (blockIdx.x >= list[0]) return;
@@ -729,161 +730,6 @@ __global__ void __launch_bounds__(32) k_dec_adaptive1(const DecTask* __restrict_
         dst[i] = (uint8_t)dec_sym(e);
         uint32_t xn = dec_next(x0, e);
         ok = bw.renorm(xn);
-    }
-    if (!ok) dec_fail(infos, t.frame, D_CORRUPT);
-}
-
-// Adaptive bodies, eight per warp: lane group g (lanes 4g .. 4g + 3) of
-// block b decodes task list[8 b + g], lane 4g + l holding state l.  The warp
-// builds the eight models one after another (per model the symbol of every
-// slot and (f - 1) << 20 | cumulative frequency per symbol, 5 KiB), then all
-// groups run their rounds together, so one warp instruction advances eight
-// chains; the list is sorted by length (k_dec_lists), so a warp's chains
-// end close together.
-constexpr uint32_t kDecGroups = 8;
-// Batches of up to this many frames decode their adaptive bodies one per
-// warp (k_dec_adaptive1): at 13 such warps per SM their bodies all run at
-// once.  Measured on 1 MiB frames: 128 frames 29.4 ms one per warp against
-// 67 ms eight per warp; 2560 frames 89 ms (whole decode) eight per warp
-// against 97 ms.
-constexpr uint32_t kDecOneWarpFrames = 512;
-constexpr uint32_t kDecModel = 4096 + 256 * 4;
-constexpr uint32_t kDecAdaptiveSmem = kDecGroups * kDecModel + 256 * 2 + kDecGroups * 4;
-
-// The decoded state after symbol slot x & 4095 with model word g = (f - 1)
-// << 20 | cumulative frequency: f (x >> 12) + (x & 4095) - cum (the rANS
-// decode step, przm_dec.c:187-199).
-__device__ __forceinline__ uint32_t dec_step(uint32_t x, uint32_t g) {
-    return ((g >> 20) + 1) * (x >> 12) + (x & 4095u) - (g & 0xFFFFFu);
-}
-
-__global__ void __launch_bounds__(32) k_dec_adaptive(const DecTask* __restrict__ tasks, const uint32_t* __restrict__ list,
-                                                     DecInfo* __restrict__ infos) {
-    extern __shared__ __align__(16) uint8_t smem_d[];
-    uint16_t* freq = reinterpret_cast<uint16_t*>(smem_d + kDecGroups * kDecModel);
-    uint32_t* gp = reinterpret_cast<uint32_t*>(smem_d + kDecGroups * kDecModel + 512);
-    const uint32_t lane = threadIdx.x, g = lane >> 2, l = lane & 3;
-    const uint32_t base = blockIdx.x * kDecGroups, cnt = list[0];
-    if (base >= cnt) return;
-    // the models, one after another by the whole warp; gp[k]: group k's
-    // stream offset after its matrix (0: no task, or a corrupt matrix)
-    for (uint32_t k = 0; k < kDecGroups; k++) {
-        uint32_t p = 0;
-        if (base + k < cnt) {
-            const DecTask t = tasks[list[4 + base + k]];
-            const uint8_t* s = reinterpret_cast<const uint8_t*>(t.src);
-            for (uint32_t i = lane; i < 256; i += 32) freq[i] = 0;
-            __syncwarp();
-            if (lane == 0) p = dec_matrix(s, t.slen, freq);
-            p = __shfl_sync(0xFFFFFFFFu, p, 0);
-            if (p == 0 || p + 16 > t.slen) {
-                if (lane == 0) dec_fail(infos, t.frame, D_CORRUPT);
-                p = 0;
-            } else {
-                // lane l takes symbols 8l .. 8l + 7 (the frequencies sum to
-                // 4096, so every slot is written)
-                uint8_t* sym = smem_d + k * kDecModel;
-                uint32_t* fct = reinterpret_cast<uint32_t*>(sym + 4096);
-                uint32_t f8[8], loc = 0;
-#pragma unroll
-                for (int q = 0; q < 8; q++) { f8[q] = freq[lane * 8 + q]; loc += f8[q]; }
-                uint32_t x = loc;
-#pragma unroll
-                for (int o = 1; o < 32; o <<= 1) {
-                    const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, x, o);
-                    if (lane >= (uint32_t)o) x += y;
-                }
-                uint32_t c = x - loc;
-                for (int q = 0; q < 8; q++) {
-                    fct[lane * 8 + q] = f8[q] ? ((f8[q] - 1) << 20) | c : 0u;
-                    for (uint32_t j = 0; j < f8[q]; j++) sym[c + j] = (uint8_t)(lane * 8 + q);
-                    c += f8[q];
-                }
-            }
-        }
-        if (lane == 0) gp[k] = p;
-        __syncwarp();
-    }
-    // this lane's group and state
-    const bool has = base + g < cnt;
-    DecTask t = {};
-    if (has) t = tasks[list[4 + base + g]];
-    uint32_t p = gp[g];
-    const bool valid = has && p != 0;
-    const uint8_t* s = reinterpret_cast<const uint8_t*>(t.src);
-    uint8_t* dst = reinterpret_cast<uint8_t*>(t.dst);
-    const uint32_t n = t.n, slen = t.slen;
-    const uint8_t* sym = smem_d + g * kDecModel;
-    const uint32_t* fct = reinterpret_cast<const uint32_t*>(sym + 4096);
-    uint32_t x = valid ? drd32(s + p + 4 * l) : 0u;
-    p += 16;
-    const uint32_t gm = 0xFu << (4 * g), lt = (1u << lane) - 1u;
-    // every lane takes part in each warp vote below, whether its group has a
-    // task or not (a lane that skipped one would leave the others waiting)
-    const uint32_t vb = __ballot_sync(0xFFFFFFFFu, valid && x >= 65536u);
-    const bool fast = valid && (vb & gm) == gm;
-    uint32_t i = 0;
-    const uintptr_t sa = reinterpret_cast<uintptr_t>(s);
-    // Rounds of four symbols per group.  The round's eight stream bytes come
-    // from three aligned words (below p + 12; the loop keeps p + 16 <= the
-    // stream's length).  A state needs 0, 1 or 2 bytes (x < 2^16, x < 2^8
-    // after the step); two ballots of those tests, each group reading its
-    // own four bits, give every lane its offset o (the bytes of the group's
-    // lanes before it) and the pointer's advance.  One byte permute puts
-    // bytes o, o + 1 in the low half of y, a second shifts them into x.
-    for (;;) {
-        const bool act = fast && i + 4 <= n && p + 16 <= slen;
-        if (!__any_sync(0xFFFFFFFFu, act)) break;
-        uint32_t lo = 0, hi = 0, sv = 0;
-        if (act) {
-            const uint32_t* w = reinterpret_cast<const uint32_t*>((sa + p) & ~uintptr_t(3));
-            const uint32_t sh = 8u * (uint32_t)((sa + p) & 3u);
-            const uint32_t w0 = w[0], w1 = w[1], w2 = w[2];
-            lo = __funnelshift_r(w0, w1, sh);
-            hi = __funnelshift_r(w1, w2, sh);
-            sv = sym[x & 4095];
-            x = dec_step(x, fct[sv]);
-        }
-        const bool r1 = act && x < 65536u, r2 = act && x < 256u;
-        const uint32_t b1 = __ballot_sync(0xFFFFFFFFu, r1) & gm, b2 = __ballot_sync(0xFFFFFFFFu, r2) & gm;
-        if (act) {
-            const uint32_t o = __popc(b1 & lt) + __popc(b2 & lt);
-            const uint32_t y = __byte_perm(lo, hi, 17u * o + 16u);
-            x = __byte_perm(x, y, r2 ? 0x1045u : (r1 ? 0x2104u : 0x3210u));
-            p += __popc(b1) + __popc(b2);
-            dst[i + l] = (uint8_t)sv;
-            i += 4;
-        }
-    }
-    uint32_t x0 = __shfl_sync(0xFFFFFFFFu, x, 4 * g), x1 = __shfl_sync(0xFFFFFFFFu, x, 4 * g + 1),
-             x2 = __shfl_sync(0xFFFFFFFFu, x, 4 * g + 2), x3 = __shfl_sync(0xFFFFFFFFu, x, 4 * g + 3);
-    if (l != 0 || !valid) return;
-    // the rest (the stream's last 16 bytes, or initial states below 2^16)
-    // byte by byte, on the group's first lane
-    bool ok = true;
-    ByteWin bw;
-    bw.init(s, slen, p);
-    bw.prefetch();
-    for (; i + 4 <= n && ok; i += 4) {  // vans_run_4x_loop, przm_dec.c:201-255
-        bw.step();
-        const uint32_t s0 = sym[x0 & 4095], s1 = sym[x1 & 4095], s2 = sym[x2 & 4095], s3 = sym[x3 & 4095];
-        x0 = dec_step(x0, fct[s0]);
-        x1 = dec_step(x1, fct[s1]);
-        x2 = dec_step(x2, fct[s2]);
-        x3 = dec_step(x3, fct[s3]);
-        ok = bw.renorm(x0) && bw.renorm(x1) && bw.renorm(x2) && bw.renorm(x3);
-        dst[i] = (uint8_t)s0;
-        dst[i + 1] = (uint8_t)s1;
-        dst[i + 2] = (uint8_t)s2;
-        dst[i + 3] = (uint8_t)s3;
-    }
-    uint32_t xs[4] = {x0, x1, x2, x3};
-    for (; i < n && ok; i++) {
-        bw.step();
-        const uint32_t v = sym[xs[i & 3] & 4095];
-        dst[i] = (uint8_t)v;
-        xs[i & 3] = dec_step(xs[i & 3], fct[v]);
-        ok = bw.renorm(xs[i & 3]);
     }
     if (!ok) dec_fail(infos, t.frame, D_CORRUPT);
 }
