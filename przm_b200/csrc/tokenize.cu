@@ -109,7 +109,7 @@ __device__ uint32_t warp_match_end(const uint8_t* src, uint32_t a, uint32_t b, u
 // decisions at a time then become records, lane by lane; which repeat slot a
 // distance is in is a scan of the lists of the three latest distinct
 // distances.  Measured on 12 KB of records (one tile): 300 us with the
-// search.  Every decision
+// search, 142 us so.  Every decision
 // becomes a record in shared memory (16 bytes, the fourth word unused):
 //   r0 = q - tile start | literals before q << 16
 //   r1 = match or run length | kind << 16 | repeat slot << 18
@@ -812,8 +812,8 @@ __global__ void __launch_bounds__(1024) k_tile_order(const uint32_t* __restrict_
 // streams (przm_tokenizer.cuh:474-609) and counts the byte histograms of the
 // literal stream and of the three command substreams, privatised per warp in
 // shared memory.  One block per frame, or several with a run of its tiles
-// each where the frames alone leave SMs idle (one frame of 4 MiB took 0.30 ms
-// with one block); their counts then meet in the frame's histogram by atomics.
+// each where the frames alone leave SMs idle (one frame of 4 MiB: 0.30 ms with
+// one block, 0.035 so); their counts then meet in the frame's histogram by atomics.
 // ---------------------------------------------------------------------------
 constexpr uint32_t kGatherThreads = 512;
 
