@@ -855,6 +855,7 @@ static int32_t ctx_setup(Ctx* c) {
     CK(cudaFuncSetAttribute(k_rans, cudaFuncAttributeMaxDynamicSharedMemorySize, kRansSmem));
     CK(cudaFuncSetAttribute(k_front, cudaFuncAttributeMaxDynamicSharedMemorySize, kFrontSmem));
     CK(cudaFuncSetAttribute(k_dec_sheaf, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(ShShared)));
+    CK(cudaFuncSetAttribute(k_dec_exec<1024>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(ExecShared<1024>)));
     CK(cudaDeviceGetAttribute(&c->clock_khz, cudaDevAttrClockRate, c->device));
     CK(c->d_meta8.ensure(8 * 256 * sizeof(EncSym)));
     CK(c->d_ctxlut.ensure(256));

@@ -3,12 +3,12 @@
 //
 // The reference walks the commands one after another; only two things in that
 // walk are serial: the repeat distances and the bytes a match copies from
-// output written just before.  Here 512 commands are taken at a time, a
+// output written just before.  Here 512 or 1024 commands are taken at a time, a
 // thread each.  Where a command's operand bytes, literals and output start are
 // sums over the commands before it; the repeat distances before it are a scan
 // of maps on four distances (each command moves one to the front or pushes a
 // new one); the first command that ends the walk or fails decides, as in the
-// walk.  The output is then made 4096 bytes at a time: every byte finds its
+// walk.  The output is then made eight bytes a thread at a time: every byte finds its
 // command, literals and matches from before the tile load their byte, and the
 // others point at a byte of the tile and follow the pointers, which jump
 // twice as far each time.
@@ -19,45 +19,48 @@
 // k_dec_exec_serial.
 //
 // Measured on 128 mixed frames of 1 MiB: 26.0 ms with one warp walking each
-// frame, 1.5 ms so.  A chunk's 16 000 cycles (of 34 000 with its copies, on the
+// frame, 1.25 ms so.  A chunk's 16 000 cycles (of 34 000 with its copies, on the
 // frames of the shortest commands) went into chains of loads, four block sums
 // and the scan of the distances, 5 000 alone when its maps held four words
 // each; maps of four bytes, three sums of one barrier, and the next chunk's
 // first loads beside the copies: 1.83 -> 1.50 ms.  Registers for two blocks an
 // SM: 300 record frames of 150 kB 1.53 -> 1.40 ms (the call), 128 of 1 MiB alike.
+// 1024 threads where the frames leave SMs to one each: 1.52 -> 1.25 ms.
 #include "common.cuh"
 
 namespace pz {
 
-constexpr uint32_t kExThreads = 512;
-constexpr uint32_t kExTile = 4096, kExPer = kExTile / kExThreads;
-constexpr uint32_t kExWindow = 4 * kExThreads;  // bytes that hold a chunk's varints, at most four each
-constexpr uint32_t kExFlat = 6 * kExThreads;    // a flat command's bytes: opcode, token, varint
-constexpr uint32_t kExCap = 1u << 26;           // sums of lengths saturate here, above every frame's size
+// NT threads: NT commands a chunk, 8 NT bytes a tile, 4 NT bytes that hold a
+// chunk's varints (at most four each), 6 NT that hold flat commands (opcode,
+// token, varint).
+constexpr uint32_t kExPer = 8;
+constexpr uint32_t kExCap = 1u << 26;  // sums of lengths saturate here, above every frame's size
 
 // how the walk ends at a command
 enum ExecEvent : uint32_t { EV_BEFORE = 0, EV_AFTER = 1, EV_CORRUPT = 2, EV_UNSUPPORTED = 3, EV_SERIAL = 4, EV_NONE = 15 };
 
+template <uint32_t NT>
 struct ExecSums {  // of the warps, for a sum over the block
-    uint32_t a[kExThreads / 32], b[kExThreads / 32];
+    uint32_t a[NT / 32], b[NT / 32];
 };
 
+template <uint32_t NT>
 struct ExecShared {
-    uint32_t start[kExThreads + 1];  // a command's first output byte
-    uint32_t lend[kExThreads];       // the end of its literals
-    uint32_t lsrc[kExThreads];       // where they start in the literal stream
-    uint32_t dist[kExThreads];       // its match's distance; 0: a run of literal lsrc
-    uint16_t vend[kExThreads], oend[kExThreads];  // ends of the chunk's varints in their windows
-    __align__(16) uint16_t w[kExTile];            // a tile's bytes: 0x8000 | byte, or a place in the tile
-    ExecSums sums[2];
-    uint32_t vars[kExThreads / 32];    // varints of a warp's commands
-    uint32_t rep[128 + kExThreads / 8];  // the repeat distances before the chunk; from 128 four of every warp
-    uint32_t rmap[kExThreads / 32];
-    uint8_t tok[kExThreads];           // the next bytes of the token stream
-    uint32_t vwin[kExThreads], owin[kExThreads];  // the bytes of the chunk's varints
-    uint16_t pos[kExThreads + 1];  // flat: where the chunk's commands start
+    uint32_t start[NT + 1];  // a command's first output byte
+    uint32_t lend[NT];       // the end of its literals
+    uint32_t lsrc[NT];       // where they start in the literal stream
+    uint32_t dist[NT];       // its match's distance; 0: a run of literal lsrc
+    uint16_t vend[NT], oend[NT];  // ends of the chunk's varints in their windows
+    __align__(16) uint16_t w[kExPer * NT];  // a tile's bytes: 0x8000 | byte, or a place in the tile
+    ExecSums<NT> sums[2];
+    uint32_t vars[NT / 32];    // varints of a warp's commands
+    uint32_t rep[128 + NT / 8];  // the repeat distances before the chunk; from 128 four of every warp
+    uint32_t rmap[NT / 32];
+    uint8_t tok[NT];           // the next bytes of the token stream
+    uint32_t vwin[NT], owin[NT];  // the bytes of the chunk's varints
+    uint16_t pos[NT + 1];  // flat: where the chunk's commands start
     uint32_t npos;
-    __align__(16) uint8_t flat[kExFlat + 16];
+    __align__(16) uint8_t flat[6 * NT + 16];
     uint32_t event;
     uint32_t st[12];  // the reader's state after the chunk, or at the end of the walk
 };
@@ -65,7 +68,8 @@ struct ExecShared {
 // Two sums at once over the block, each saturating at kExCap: the sums before
 // this thread in a and b, the totals in ta and tb.  One barrier: another call
 // meanwhile takes another W.
-__device__ __forceinline__ void exec_scan2(uint32_t& a, uint32_t& b, uint32_t& ta, uint32_t& tb, ExecSums& W) {
+template <uint32_t NT>
+__device__ __forceinline__ void exec_scan2(uint32_t& a, uint32_t& b, uint32_t& ta, uint32_t& tb, ExecSums<NT>& W) {
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     uint32_t x = min(a, kExCap), y = min(b, kExCap);
 #pragma unroll
@@ -86,7 +90,7 @@ __device__ __forceinline__ void exec_scan2(uint32_t& a, uint32_t& b, uint32_t& t
     b = lane ? ey : 0u;
     ta = tb = 0;
 #pragma unroll
-    for (uint32_t w = 0; w < kExThreads / 32; w++) {  // (16 sums of at most kExCap: no carry)
+    for (uint32_t w = 0; w < NT / 32; w++) {  // (at most 32 sums of at most kExCap: no carry)
         const uint32_t p = W.a[w], q = W.b[w];
         if (w < warp) {
             a += p;
@@ -149,11 +153,12 @@ __device__ __forceinline__ uint32_t exec_ends(uint32_t w) {
     for (uint32_t i = 0; i < 4; i++) m |= ((w >> (8 * i + 7)) & 1u) << i;
     return m ^ 15u;
 }
+template <uint32_t NT>
 __device__ __forceinline__ void exec_put_ends(uint16_t* ends, uint32_t m, uint32_t k) {
 #pragma unroll
     for (uint32_t i = 0; i < 4; i++)
         if ((m >> i) & 1u) {
-            if (k < kExThreads) ends[k] = (uint16_t)(4 * threadIdx.x + i + 1);
+            if (k < NT) ends[k] = (uint16_t)(4 * threadIdx.x + i + 1);
             k++;
         }
 }
@@ -169,15 +174,16 @@ __device__ __forceinline__ void exec_put_ends(uint16_t* ends, uint32_t m, uint32
 // next command at nearly every byte), 1.83 ms so.
 constexpr uint32_t kExPieces = 4;
 constexpr uint32_t kExBias = kExPer;  // a place in the tile is kept as its index + 8, so that none is below 0
-__device__ void exec_copy(ExecShared& S, uint8_t* dst, const uint8_t* __restrict__ lit, uint32_t dp, uint32_t end,
+template <uint32_t NT>
+__device__ void exec_copy(ExecShared<NT>& S, uint8_t* dst, const uint8_t* __restrict__ lit, uint32_t dp, uint32_t end,
                           uint32_t E) {
     static_assert(kExPer == 8, "two words of bytes, four of places");
     const uint32_t tid = threadIdx.x;
     volatile const uint16_t* w = S.w;
     // tiles begin on 8-byte boundaries of the address
     for (int32_t tb = (int32_t)dp - (int32_t)((reinterpret_cast<uintptr_t>(dst) + dp) & 7u); tb < (int32_t)end;
-         tb += kExTile) {
-        const int32_t lo = max(tb, (int32_t)dp), hi = min(tb + (int32_t)kExTile, (int32_t)end);
+         tb += kExPer * NT) {
+        const int32_t lo = max(tb, (int32_t)dp), hi = min(tb + (int32_t)(kExPer * NT), (int32_t)end);
         const int32_t p0 = tb + (int32_t)(kExPer * tid);
         const int32_t pa = max(p0, lo), pz = min(p0 + (int32_t)kExPer, hi);  // own bytes
         uint32_t x[2] = {0, 0};              // their values
@@ -316,9 +322,11 @@ __device__ void exec_copy(ExecShared& S, uint8_t* dst, const uint8_t* __restrict
     }
 }
 
-__global__ void __launch_bounds__(kExThreads, 2) k_dec_exec(const uint8_t* __restrict__ src, const DecJob* __restrict__ jobs,
+template <uint32_t NT>
+__global__ void __launch_bounds__(NT, 1024 / NT) k_dec_exec(const uint8_t* __restrict__ src, const DecJob* __restrict__ jobs,
                                                          DecInfo* __restrict__ infos, uint8_t* __restrict__ out) {
-    __shared__ ExecShared S;
+    extern __shared__ __align__(16) uint8_t smem_x[];
+    ExecShared<NT>& S = *reinterpret_cast<ExecShared<NT>*>(smem_x);
     const uint32_t f = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const DecInfo I = infos[f];
     if (I.err || I.u_size == 0) return;
@@ -327,7 +335,7 @@ __global__ void __launch_bounds__(kExThreads, 2) k_dec_exec(const uint8_t* __res
     const uint32_t u = I.u_size;
     if (I.stored) {
         const uint8_t* s = src + jb.src_off + 8;
-        for (uint32_t i = tid; i < u; i += kExThreads) dst[i] = s[i];
+        for (uint32_t i = tid; i < u; i += NT) dst[i] = s[i];
         return;
     }
     const uint8_t* cs = reinterpret_cast<const uint8_t*>(I.cmd);
@@ -357,14 +365,14 @@ __global__ void __launch_bounds__(kExThreads, 2) k_dec_exec(const uint8_t* __res
     for (;;) {
         // the chunk's commands: the next 512 opcodes, or in a flat stream the
         // commands that one thread finds in its next bytes
-        uint32_t n = min(kExThreads, cl - cp), at = cp + tid;
+        uint32_t n = min(NT, cl - cp), at = cp + tid;
         if (!split) {
-            for (uint32_t i = tid; i < kExFlat && cp + i < cl; i += kExThreads) S.flat[i] = cs[cp + i];
+            for (uint32_t i = tid; i < 6 * NT && cp + i < cl; i += NT) S.flat[i] = cs[cp + i];
             __syncthreads();
             if (tid == 0) {
-                const uint32_t have = min(kExFlat, cl - cp);
+                const uint32_t have = min(6 * NT, cl - cp);
                 uint32_t p = 0, k = 0;
-                while (k < kExThreads && p < have) {
+                while (k < NT && p < have) {
                     const uint32_t op = S.flat[p];
                     S.pos[k++] = (uint16_t)p;
                     p++;
@@ -413,9 +421,9 @@ __global__ void __launch_bounds__(kExThreads, 2) k_dec_exec(const uint8_t* __res
         S.vwin[tid] = pre_var;
         S.owin[tid] = pre_off;
         S.tok[tid] = (uint8_t)pre_tok;
-        uint32_t s1 = m | (isexp << 12), s2 = __popc(vm) | (__popc(em) << 12), t1, t2;
-        exec_scan2(s1, s2, t1, t2, S.sums[0]);  // (fields of at most 512 and 2048, all below kExCap)
-        const uint32_t mi = s1 & 0xFFFu, ei = s1 >> 12, nexp = t1 >> 12, nv = t2 & 0xFFFu, ne = t2 >> 12;
+        uint32_t s1 = m | (isexp << 13), s2 = __popc(vm) | (__popc(em) << 13), t1, t2;
+        exec_scan2(s1, s2, t1, t2, S.sums[0]);  // (fields of at most NT and 4 NT, all below kExCap)
+        const uint32_t mi = s1 & 0x1FFFu, ei = s1 >> 13, nexp = t1 >> 13, nv = t2 & 0x1FFFu, ne = t2 >> 13;
         const uint32_t mt = split ? mp + mi : at + 1;
         if (m) {
             uint32_t tok = 0;
@@ -423,14 +431,14 @@ __global__ void __launch_bounds__(kExThreads, 2) k_dec_exec(const uint8_t* __res
             else bad = true;
             llit = tok >> 4; lmatch = (tok & 15u) + bmin; isvar = (tok & 15u) == 15u && !bad;
         }
-        exec_put_ends(S.vend, vm, s2 & 0xFFFu);
-        exec_put_ends(S.oend, em, s2 >> 12);
+        exec_put_ends<NT>(S.vend, vm, s2 & 0x1FFFu);
+        exec_put_ends<NT>(S.oend, em, s2 >> 13);
         const uint32_t vb = __ballot_sync(0xFFFFFFFFu, isvar);
         if (lane == 0) S.vars[warp] = __popc(vb);
         __syncthreads();  // the ends too
         uint32_t vi = __popc(vb & ((1u << lane) - 1u));
 #pragma unroll
-        for (uint32_t w = 0; w < kExThreads / 32; w++)
+        for (uint32_t w = 0; w < NT / 32; w++)
             if (w < warp) vi += S.vars[w];
         uint32_t vlen = 0, vbefore = 0, vval = 0;
         if (split) {
@@ -485,7 +493,7 @@ __global__ void __launch_bounds__(kExThreads, 2) k_dec_exec(const uint8_t* __res
         }
         if (tid == 0) S.event = 0xFFFFFFFFu;
         __syncthreads();
-        const uint32_t warps = rep_scan(lane < kExThreads / 32 ? S.rmap[lane] : kRepSame);
+        const uint32_t warps = rep_scan(lane < NT / 32 ? S.rmap[lane] : kRepSame);
         const uint32_t all = __shfl_sync(0xFFFFFFFFu, warps, 31), pre = __shfl_sync(0xFFFFFFFFu, warps, warp ? warp - 1 : 0);
         if (kind == 1) d = mine & 0x80u ? dn : S.rep[((warp ? pre : kRepSame) >> (8 * mine)) & 0xFFu];
         const uint32_t rep = tid < 4 ? S.rep[(all >> (8 * tid)) & 0xFFu] : 0u;  // after the chunk

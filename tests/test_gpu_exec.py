@@ -79,3 +79,19 @@ def test_plain_distance_opcodes_and_what_is_around_them(comp):
     for o, w in zip(outs, want):
         assert o == w
     assert st[4] not in (0, st[5]) and st[5] != 0 and st[6:] == [st[5]] * 5
+
+
+@pytest.mark.parametrize("copies", [1, 12])
+def test_edges_of_both_block_sizes(comp, copies):
+    # 14 frames take 1024 threads each, 168 frames 512
+    lits = bytes(range(8))
+    counts = (510, 511, 512, 1022, 1023, 1024)  # commands after the first
+    frames = [flat_frame(b"\xfa" + b"\x00" * k, b"", lits, 8 + 4 * k) for k in counts]
+    want = [lits + bytes([7]) * (4 * k) for k in counts]
+    xs = [x for n in (8191, 8192, 8193, 16_385) for x in (period(5, n), W.gen("records", n, n))]
+    frames += [comp.Compress(x, gpu.PROFILE_ANS)[0] for x in xs]
+    want += [x.tobytes() for x in xs]
+    st, outs = decode(comp, frames * copies, [len(w) for w in want] * copies, 1)
+    assert st == [0] * len(outs)
+    bad = [i for i, (w, o) in enumerate(zip(want * copies, outs)) if w != o]
+    assert not bad, bad
