@@ -22,7 +22,7 @@
 //   k_dec_sheaf    two warps per sheaf frame: the literals re-interleaved
 //                  from their four fibers by the class of the bytes before
 //                  each (the order of the fibers is serial by the format).
-//   k_dec_exec     (exec.cu) one block per frame: 512 commands at a time,
+//   k_dec_exec     (exec.cu) one block per frame: 512 or 1024 commands at a time,
 //                  the output made in tiles;
 //   k_dec_exec_serial  one warp per frame that uses opcodes of the
 //                  reference's CPU compressor: the command walk, every lane
