@@ -16,7 +16,8 @@
 // Takes the opcodes of the tokenizer: fused repeat (< 0x80), fused explicit
 // (0x80-0xBF), long repeat (0xC0-0xC3), literal runs (0xF0, 0xF3-0xFA), byte
 // runs (0xF1).  A frame that reaches another known opcode is left to
-// k_dec_exec_serial.
+// k_dec_exec_warp, and so are short frames (exec_short_cap) and, in calls of
+// many frames, those of flat command streams.
 //
 // Measured on 128 mixed frames of 1 MiB: 26.0 ms with one warp walking each
 // frame, 1.25 ms so.  A chunk's 16 000 cycles (of 34 000 with its copies, on the
@@ -322,9 +323,23 @@ __device__ void exec_copy(ExecShared<NT>& S, uint8_t* dst, const uint8_t* __rest
     }
 }
 
+// A call of nf frames whose capacities are at most this is walked by a warp per
+// frame alone.  A chunk takes a block 8 to 12 us however few its commands; the
+// walk takes 20 to 50 us per 1000 bytes, but 28 frames an SM at once instead of
+// one or two.  Measured (walk, chunks; us): one frame of 500 bytes 10, 15 and
+// of 1000 bytes 29, 21; 600 of 1000 bytes 26-34, 37-45 and of 2000 54-84, 61-83;
+// 3000 of 2000 bytes 72-107, 190-309; 12000 of 200 bytes 10, 300.
+inline uint32_t exec_short_cap(uint32_t nf, uint32_t sms) { return nf <= 2 * sms ? 768u : nf <= 8 * sms ? 1536u : 2304u; }
+
+// flat_to_warps (calls of more than 8 frames an SM): frames of flat streams of
+// short commands are left to k_dec_exec_warp, because one thread finds a
+// chunk's commands here, and two blocks an SM hide less of that than 28 walks
+// (3000 frames of 4000 bytes: 142-254 us walked, 414-604 so; 600 frames: alike
+// or slower).
 template <uint32_t NT>
 __global__ void __launch_bounds__(NT, 1024 / NT) k_dec_exec(const uint8_t* __restrict__ src, const DecJob* __restrict__ jobs,
-                                                         DecInfo* __restrict__ infos, uint8_t* __restrict__ out) {
+                                                         DecInfo* __restrict__ infos, uint8_t* __restrict__ out,
+                                                         bool flat_to_warps) {
     extern __shared__ __align__(16) uint8_t smem_x[];
     ExecShared<NT>& S = *reinterpret_cast<ExecShared<NT>*>(smem_x);
     const uint32_t f = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -345,6 +360,10 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_dec_exec(const uint8_t* __res
     const uint8_t* offs = reinterpret_cast<const uint8_t*>(I.off);
     const uint32_t cl = I.cmd_len, ml = I.meta_len, vl = I.var_len, ll = I.lit_len, ol = I.off_len, bmin = I.bmin;
     const bool split = I.cmd_mode == 1;
+    if (flat_to_warps && !split && u / 64 <= cl) {
+        if (tid == 0) infos[f].serial = 1;
+        return;
+    }
     const uint32_t jlim = split ? I.cmd_orig : cl;
     uint32_t cp = 0, mp = 0, vp = 0, j = 0, lp = 0, dp = 0, op0 = 0;
     if (tid < 4) {

@@ -1,0 +1,95 @@
+"""Short frames are decoded by a warp each: the same bytes and statuses as by
+the command blocks (which a longer frame in the call brings on), at the sizes
+and frame counts where one goes over to the other, and no slower than the
+other stages of the call."""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+from przm_b200 import devmem, gpu
+from przm_b200 import workloads as W
+
+from .gpu_profile import kernels, total
+from .test_gpu_exec import flat_frame
+
+pytestmark = pytest.mark.gpu
+
+
+def layout(frames, caps):
+    so = np.concatenate([[0], np.cumsum([len(f) for f in frames])]).astype(np.uint64)
+    do = np.concatenate([[0], np.cumsum([(c + 15) // 16 * 16 for c in caps])]).astype(np.uint64)
+    d_src = devmem.upload(np.frombuffer(b"".join(frames) + bytes(64), np.uint8))
+    return d_src, devmem.alloc(int(do[-1]) + 64), so, do
+
+
+def decode(comp, frames, caps):
+    d_src, d_dst, so, do = layout(frames, caps)
+    st, ln = comp.DecompressBatchDevice(d_src.ptr, so[:-1], [len(f) for f in frames], d_dst.ptr, do[:-1], caps)
+    host = devmem.download(d_dst.ptr, int(do[-1]))
+    return [int(x) for x in st], [host[int(a):int(a) + int(n)] for a, n in zip(do, ln)]
+
+
+def frames_up_to(comp, cap, profile):
+    xs = [W.gen(k, 3 * n + profile, n) for k in ("records", "markov", "table", "uniform") for n in (1, 7, 100, cap // 2, cap - 1, cap)]
+    xs += [np.zeros(cap, np.uint8), np.resize(np.arange(5, dtype=np.uint8), cap)]
+    return [comp.Compress(x, profile)[0] for x in xs], [len(x) for x in xs], [x.tobytes() for x in xs]
+
+
+@pytest.mark.parametrize("profile", [0, 1, 2, 3])
+@pytest.mark.parametrize("count,cap", [(1, 768), (148, 768), (149, 768), (296, 769), (297, 1536), (1184, 1537), (1185, 2304), (1300, 2305)])
+def test_same_bytes_at_the_borders(comp, profile, count, cap):
+    fr, caps, want = frames_up_to(comp, cap, profile)
+    pick = [i % len(fr) for i in range(count - 1)] + [len(fr) - 3]  # (the last: `cap` bytes)
+    st, outs = decode(comp, [fr[i] for i in pick], [caps[i] for i in pick])
+    assert st == [0] * count
+    bad = [i for i, o in zip(pick, outs) if o != want[i]]
+    assert not bad, bad
+
+
+def test_damaged_short_frames_as_in_a_call_with_a_long_one(comp):
+    rng = np.random.default_rng(5)
+    base = [comp.Compress(W.gen(k, 9, 700), p)[0] for k in ("records", "markov") for p in (0, 1, 2)]
+    lits = bytes(range(8))
+    frames = [flat_frame(b"\xfa" + t, o, lits, n) for t, o, n in (
+        (b"\xc7\x0c", b"", 24), (b"\xe0\x01", b"", 24), (b"\xf2", b"", 24), (b"\x8f", b"\x08", 40), (b"\x84", b"\x09", 16), (b"", b"", 9))]
+    for fr in base:
+        for _ in range(20):
+            b = bytearray(fr)
+            b[int(rng.integers(8, len(b)))] ^= 1 << int(rng.integers(0, 8))
+            frames.append(bytes(b))
+    caps = [700] * len(frames)
+    short = decode(comp, frames, caps)
+    big = comp.Compress(W.gen("records", 2, 20_000), 1)[0]
+    st, outs = decode(comp, frames + [big], caps + [20_000])
+    assert st[-1] == 0
+    assert short[0] == st[:-1]
+    assert [o for s, o in zip(*short) if s == 0] == [o for s, o in zip(st[:-1], outs) if s == 0]
+
+
+def test_flat_frames_of_a_call_of_many(comp):
+    # more than 8 frames an SM, one of them long: flat streams of short commands are walked, the others are not
+    xs = [W.gen(("records", "uniform", "table")[i % 3], i, 300 + 37 * (i % 90)) for i in range(1200)] + [W.gen("records", 1, 40_000)]
+    frames = [comp.Compress(x, i % 2)[0] for i, x in enumerate(xs)]
+    st, outs = decode(comp, frames, [len(x) for x in xs])
+    assert st == [0] * len(xs)
+    assert [o == x.tobytes() for o, x in zip(outs, xs)] == [True] * len(xs)
+
+
+def test_launches_of_a_short_frame(comp):
+    fr = np.frombuffer(comp.Compress(W.gen("records", 1, 100), 1)[0], np.uint8)
+    ks = [n for n, _ in kernels(lambda: comp.Decompress(fr))]
+    assert len(ks) == 6, ks  # parse, static models, adaptive bodies, prefix, sheaf, commands
+
+
+@pytest.mark.parametrize("profile", [0, 1])
+def test_many_short_frames_cost_less_than_empty_slots(comp, profile):
+    # k_dec_static only finds that these frames' 160 000 slots have no static body: 112 us
+    n, count = 200, 20_000
+    xs = [W.gen("records", i, n) for i in range(40)]
+    fr = [comp.Compress(x, profile)[0] for x in xs]
+    frames = [fr[i % 40] for i in range(count)]
+    d_src, d_dst, so, do = layout(frames, [n] * count)
+    ln = [len(f) for f in frames]
+    ks = kernels(lambda: comp.DecompressBatchDevice(d_src.ptr, so[:-1], ln, d_dst.ptr, do[:-1], [n] * count))
+    assert total(ks, "k_dec_exec", "k_dec_adaptive") < total(ks, "k_dec_static"), ks
