@@ -93,3 +93,18 @@ def test_many_short_frames_cost_less_than_empty_slots(comp, profile):
     ln = [len(f) for f in frames]
     ks = kernels(lambda: comp.DecompressBatchDevice(d_src.ptr, so[:-1], ln, d_dst.ptr, do[:-1], [n] * count))
     assert total(ks, "k_dec_exec", "k_dec_adaptive") < total(ks, "k_dec_static"), ks
+
+
+@pytest.mark.parametrize("profile", [0, 1])
+def test_frames_of_byte_runs_are_walked(comp, profile):
+    # k_dec_static only finds that the 20 000 slots have no static body: 16 us
+    xs = [np.full(60_000 + i % 7, i % 3, np.uint8) for i in range(2500)]
+    frames = [comp.Compress(x, profile)[0] for x in xs[:21]]
+    frames = [frames[i % 21] for i in range(len(xs))]
+    caps = [len(x) for x in xs]
+    st, outs = decode(comp, frames[:60], caps[:60])
+    assert st == [0] * 60 and outs == [x.tobytes() for x in xs[:60]]
+    d_src, d_dst, so, do = layout(frames, caps)
+    ln = [len(f) for f in frames]
+    ks = kernels(lambda: comp.DecompressBatchDevice(d_src.ptr, so[:-1], ln, d_dst.ptr, do[:-1], caps))
+    assert total(ks, "k_dec_exec<") < 2 * total(ks, "k_dec_static"), ks
