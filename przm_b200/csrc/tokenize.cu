@@ -126,6 +126,7 @@ constexpr uint32_t kTokWin = 1024;   // descriptor window entries
 constexpr uint32_t kTokRec = 256;    // records buffered before emission
 constexpr uint32_t kTokWarps = 4;    // warps (tiles) per block
 constexpr uint32_t kLongLit = 128;   // literal runs copied 16 bytes per lane
+constexpr uint32_t kWarpLit = 2048;  // ... by the whole warp, four loads of each lane in flight
 
 struct TokSmem {
     uint32_t desc[kTokWin];
@@ -247,10 +248,11 @@ __device__ void warp_copy_hist(uint8_t* __restrict__ d, const uint8_t* s, uint32
     }
 }
 
-// Copies n bytes s -> d with eight lanes (t: 0..7), as warp_copy_hist.
-__device__ __forceinline__ void copy_run8(uint8_t* __restrict__ d, const uint8_t* __restrict__ s, uint32_t n, uint32_t t) {
+// Copies n bytes s -> d with T lanes (t: 0 .. T - 1), as warp_copy_hist.
+__device__ __forceinline__ void copy_run(uint8_t* __restrict__ d, const uint8_t* __restrict__ s, uint32_t n, uint32_t t,
+                                         uint32_t T) {
     const uint32_t head = min(n, (uint32_t)((16 - (reinterpret_cast<uintptr_t>(d) & 15)) & 15));
-    for (uint32_t i = t; i < head; i += 8) d[i] = s[i];
+    for (uint32_t i = t; i < head; i += T) d[i] = s[i];
     d += head;
     s += head;
     n -= head;
@@ -259,15 +261,15 @@ __device__ __forceinline__ void copy_run8(uint8_t* __restrict__ d, const uint8_t
     const uint32_t* sw = reinterpret_cast<const uint32_t*>(reinterpret_cast<uintptr_t>(s) & ~uintptr_t(3));
     uint4* d4 = reinterpret_cast<uint4*>(d);
     uint32_t v = t;
-    for (; v + 24 < nv; v += 32) {
+    for (; v + 3 * T < nv; v += 4 * T) {
         uint4 o[4];
 #pragma unroll
-        for (int u = 0; u < 4; u++) o[u] = ld16_shifted<false>(sw, v + 8 * u, sh);
+        for (int u = 0; u < 4; u++) o[u] = ld16_shifted<false>(sw, v + T * u, sh);
 #pragma unroll
-        for (int u = 0; u < 4; u++) d4[v + 8 * u] = o[u];
+        for (int u = 0; u < 4; u++) d4[v + T * u] = o[u];
     }
-    for (; v < nv; v += 8) d4[v] = ld16_shifted<false>(sw, v, sh);
-    for (uint32_t i = 16 * nv + t; i < n; i += 8) d[i] = s[i];
+    for (; v < nv; v += T) d4[v] = ld16_shifted<false>(sw, v, sh);
+    for (uint32_t i = 16 * nv + t; i < n; i += T) d[i] = s[i];
 }
 
 // Writes records [0, nrec) of the warp's buffer.
@@ -358,8 +360,11 @@ __device__ void tok_emit(const uint4* rec, uint32_t nrec, const uint8_t* tile_sr
         // literal runs of these records: runs of kLongLit bytes or more with
         // 16-byte copies, four at a time by eight lanes each (one at a time by
         // the warp, each waits for its loads: 23 000 cycles for 32 runs of 200
-        // bytes), the shorter ones all lanes over their concatenated bytes,
-        // four bytes per lane in flight
+        // bytes), but one at a time those of kWarpLit, where the warp's loads
+        // in flight are one run's (a run of 32 KiB by eight lanes alone made
+        // the kernel 66 us for 148 inputs of 64 KiB without a match, 45 so);
+        // the shorter ones all lanes over their concatenated bytes, four bytes
+        // per lane in flight
         {
             const uint32_t cl = c[S_LIT];
             const bool lng = cl >= kLongLit;
@@ -394,16 +399,22 @@ __device__ void tok_emit(const uint4* rec, uint32_t nrec, const uint8_t* tile_sr
                 for (int u = 0; u < 4; u++)
                     if (b0 + 32 * u + lane < ts) dl[di[u]] = vb[u];
             }
-            uint32_t lm = __ballot_sync(0xFFFFFFFFu, lng);
+            uint32_t lm = __ballot_sync(0xFFFFFFFFu, lng), wm = __ballot_sync(0xFFFFFFFFu, cl >= kWarpLit);
             while (lm) {
-                // lanes 8 g .. 8 g + 7 take the g-th run left
-                uint32_t m = lm;
-                for (uint32_t g = 0; g < (lane >> 3); g++) m &= m - 1;
+                // lanes 8 g .. 8 g + 7 take the g-th run left, or all the first of kWarpLit or the last
+                const uint32_t T = wm || !(lm & (lm - 1)) ? 32u : 8u;
+                uint32_t m = wm ? wm : lm;
+                for (uint32_t g = 0; g < lane / T; g++) m &= m - 1;
                 const uint32_t j = m ? __ffs(m) - 1 : 0;
                 const uint32_t run = __shfl_sync(0xFFFFFFFFu, cl, j), at = __shfl_sync(0xFFFFFFFFu, dx, j),
                                src_at = __shfl_sync(0xFFFFFFFFu, from, j);
-                if (m) copy_run8(dl + at, tile_src + src_at, run, lane & 7);
-                for (uint32_t g = 0; g < 4; g++) lm &= lm - 1;
+                if (m) copy_run(dl + at, tile_src + src_at, run, lane & (T - 1), T);
+                if (wm) {
+                    lm &= ~(wm & (0u - wm));
+                    wm &= wm - 1;
+                } else {
+                    for (uint32_t g = 0; g < 4; g++) lm &= lm - 1;
+                }
             }
         }
 #pragma unroll
