@@ -530,6 +530,11 @@ __device__ void tokenize_tile(const uint8_t* __restrict__ in, const Job* __restr
             const uint32_t nz = spread8_4(cap0 >> s8) | (spread8_4(cap1 >> s8) << 1) | (spread8_4(cap2 >> s8) << 2) |
                                 (spread8_4(cap3 >> s8) << 3);
             wsum = __ballot_sync(0xFFFFFFFFu, nz != 0);
+            if (wsum == 0) {  // (148 inputs of 64 KiB without a match: 87 us with the rest of this, 45 so)
+                sm.nz[lane] = 0;
+                __syncwarp();
+                return;
+            }
             uint32_t eq = 0;
             if (radix) {
                 // candidate base + r starts at byte 8 (base + r); uint4 u = 32 i + t
@@ -556,8 +561,9 @@ __device__ void tokenize_tile(const uint8_t* __restrict__ in, const Job* __restr
             } else {
                 // positions base + 32 lane .. + 31 (32-aligned, inputs are 16-aligned
                 // and padded by 64 bytes past n): the runs of twelve equal bytes,
-                // nine neighbours whose four bytes are equal
-                if (base + 32 * lane < e_hi) {
+                // nine neighbours whose four bytes are equal; looked at in words
+                // with a descriptor, and in those after them
+                if (base + 32 * lane < e_hi && (((wsum | (wsum << 1)) >> lane) & 1u)) {
                     const uint4* s4 = reinterpret_cast<const uint4*>(src + base + 32 * lane);
                     const uint4 a = __ldg(s4), b = __ldg(s4 + 1), c = __ldg(s4 + 2);
                     const uint32_t w[12] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w, c.x, c.y, c.z, c.w};
