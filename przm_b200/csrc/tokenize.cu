@@ -846,6 +846,10 @@ __device__ void gather_item(const Job* __restrict__ jobs, uint32_t j, const uint
     {
         const Job job = jobs[j];
         uint8_t* sreg = streams + job.str_off;
+        // the part's tiles (64-bit divisions, once per stream, took a third of
+        // a short input: 20 000 of 200 bytes 619 us with them, 483 without)
+        const uint32_t t0 = parts == 1 ? 0u : job.ntiles * part / parts;
+        const uint32_t t1 = parts == 1 ? job.ntiles : job.ntiles * (part + 1) / parts;
         __syncthreads();
         for (uint32_t i = tid; i < 4 * 4 * 256; i += nthr) (&s_hist[0][0][0])[i] = 0;
         for (int s = 0; s < S_COUNT; s++) {
@@ -878,8 +882,7 @@ __device__ void gather_item(const Job* __restrict__ jobs, uint32_t j, const uint
             uint8_t* dst = sreg + stream_base(job, s);
             const int hs = s == S_LIT ? 0 : (s == S_OP ? 1 : (s == S_META ? 2 : (s == S_VAR ? 3 : -1)));
             // one warp per tile
-            const uint32_t t1 = (uint32_t)((uint64_t)job.ntiles * (part + 1) / parts);
-            for (uint32_t t = (uint32_t)((uint64_t)job.ntiles * part / parts) + warp; t < t1; t += nthr / 32) {
+            for (uint32_t t = t0 + warp; t < t1; t += nthr / 32) {
                 const uint32_t o = s_off[t], l = s_off[t + 1] - o;
                 const uint8_t* sp = slots + (uint64_t)(job.tile0 + t) * kSlotStride + slot_base(s);
                 warp_copy_hist<kC>(dst + o, sp, l, hs >= 0 ? s_hist[hs][warp & 3] : nullptr, lane);
