@@ -200,6 +200,41 @@ struct GoSort {
 // Normalisers (one warp per histogram).  All lanes return the same table.
 // ---------------------------------------------------------------------------
 
+// +1 to the frequencies of the `diff` symbols of the largest counts (lowest
+// symbol first among equal ones), of a histogram whose counts lie in at most
+// four groups of 32 symbols (bits of `groups`): the others are left out on both
+// sides of the comparisons.  Measured with all eight: 2000 streams of 300 bytes
+// of text 40 us in k_stream_norm, one 17.3; 15 and 11 so, and alphabets in more
+// groups as before where this is a function of its own, 4 us longer with it
+// inline.  (The comparison
+// in bitwise form: with short-circuits it was branches, five times as long.)
+__device__ __noinline__ void warp_raise_largest4(const uint32_t* __restrict__ cnt, uint16_t* __restrict__ freq,
+                                                    uint32_t groups, uint32_t diff, uint32_t lane) {
+    uint32_t c[4], id[4], rank[4], m = groups;
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        id[k] = lane + 32 * (m ? __ffs(m) - 1 : 0);
+        c[k] = m ? cnt[id[k]] : 0u;
+        rank[k] = 0;
+        m &= m - 1;
+    }
+    for (m = groups; m; m &= m - 1) {
+        const uint32_t t0 = 32 * (__ffs(m) - 1);
+#pragma unroll 2
+        for (uint32_t t = t0; t < t0 + 32; t += 4) {
+            const uint32_t ct[4] = {cnt[t], cnt[t + 1], cnt[t + 2], cnt[t + 3]};
+#pragma unroll
+            for (uint32_t u = 0; u < 4; u++)
+#pragma unroll
+                for (int k = 0; k < 4; k++)
+                    rank[k] += (uint32_t)(ct[u] > c[k]) | ((uint32_t)(ct[u] == c[k]) & (uint32_t)(t + u < id[k]));
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < 4; k++)
+        if (c[k] && rank[k] < diff) freq[id[k]] = (uint16_t)(freq[id[k]] + 1);
+}
+
 // literals.NormalizeFrequencies + adjustFrequencySum
 // (core/literals/literals.go:78-140): f = 1 + c*(4096-unique)/total, then the
 // shortfall goes +1 each to the symbols with the largest counts (lowest
@@ -226,20 +261,28 @@ __device__ void warp_normalize_frequencies(const uint32_t* __restrict__ cnt /* s
     const int diff = 4096 - (int)(sum & 0xFFFF);
     if (diff > 0) {
         // rank among active symbols by (count desc, symbol asc), a lane's
-        // eight symbols against four counts at a time
-        uint32_t c[8], rank[8];
+        // eight symbols against four counts at a time; a lane's four where
+        // that holds every active one
+        uint32_t groups = 0;  // bit k: a count among symbols 32 k .. 32 k + 31
 #pragma unroll
-        for (uint32_t k = 0; k < 8; k++) { c[k] = cnt[lane + 32 * k]; rank[k] = 0; }
-        for (uint32_t t = 0; t < 256; t += 4) {
-            const uint32_t ct[4] = {cnt[t], cnt[t + 1], cnt[t + 2], cnt[t + 3]};
+        for (uint32_t k = 0; k < 8; k++) groups |= __any_sync(0xFFFFFFFFu, cnt[lane + 32 * k] != 0) ? 1u << k : 0u;
+        if (__popc(groups) <= 4) {
+            warp_raise_largest4(cnt, freq, groups, (uint32_t)diff, lane);
+        } else {
+            uint32_t c[8], rank[8];
 #pragma unroll
-            for (uint32_t u = 0; u < 4; u++)
+            for (uint32_t k = 0; k < 8; k++) { c[k] = cnt[lane + 32 * k]; rank[k] = 0; }
+            for (uint32_t t = 0; t < 256; t += 4) {
+                const uint32_t ct[4] = {cnt[t], cnt[t + 1], cnt[t + 2], cnt[t + 3]};
 #pragma unroll
-                for (uint32_t k = 0; k < 8; k++) rank[k] += ct[u] > c[k] || (ct[u] == c[k] && t + u < lane + 32 * k) ? 1 : 0;
+                for (uint32_t u = 0; u < 4; u++)
+#pragma unroll
+                    for (uint32_t k = 0; k < 8; k++) rank[k] += ct[u] > c[k] || (ct[u] == c[k] && t + u < lane + 32 * k) ? 1 : 0;
+            }
+#pragma unroll
+            for (uint32_t k = 0; k < 8; k++)
+                if (c[k] && rank[k] < (uint32_t)diff) freq[lane + 32 * k] = (uint16_t)(freq[lane + 32 * k] + 1);
         }
-#pragma unroll
-        for (uint32_t k = 0; k < 8; k++)
-            if (c[k] && rank[k] < (uint32_t)diff) freq[lane + 32 * k] = (uint16_t)(freq[lane + 32 * k] + 1);
     } else if (diff < 0 && lane == 0) {
         for (int it = 0; it < -diff; it++)
             for (int s = 255; s >= 0; s--)
