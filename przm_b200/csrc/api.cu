@@ -726,7 +726,7 @@ static int32_t launch_range(przmg_batch* b, cudaStream_t s, int stop_after, cons
                                    b->d_m12_seg0.as<uint32_t>(), R.j0};
                 CK(launch_m12(mf, R.nj, most, m12_bufs(b->d_m12.p, b->m12_segs_total), c->d_dist12.as<EncSym>(), b->aux));
                 CK(cudaEventRecord(b->ev_join, b->aux));
-                launches += m12_segs(most) > 1 ? 4 : 2;
+                launches += m12_segs(most) > 1 ? 4 : 1;
             }
             if (b->profile >= 3) {  // Section 4: the literals' four foliations
                 k_frame_fibers<<<dim3(R.nj, 4), kFibThreads, 0, s>>>(b->d_jobs.as<Job>(), R.j0, b->d_job_lens.as<uint32_t>(),

@@ -149,6 +149,7 @@ __global__ void __launch_bounds__(kS3Threads) k_s3_frame(const Job* __restrict__
 constexpr uint32_t kM12Seg = 2048, kM12Warm = 1024;
 constexpr uint32_t kM12Split = 6144;  // codes up to which one warp codes the chain as fast as segments are found
 static_assert(4 * kStitchRounds % kM12Seg == 0, "stitch passes start at segment ends");
+static_assert(kM12Split <= 4 * kStitchRounds, "a chain of one segment is one stitch pass");
 
 struct M12Task {
     const uint8_t* codes;
@@ -323,19 +324,23 @@ __global__ void __launch_bounds__(32) k_m12_code(Tasks tasks, M12Bufs mb, const 
         at -= 32;
         __syncwarp();
     }
-    if (lane == 0) {
+    if (segs == 1) {  // the totals, which k_m12_sum has of chains in segments (one stitch pass at most)
+        if (lane < 4) io.cum[0] = lane == 0 ? bytes : 0u;
+        if (lane == 0) tasks.put(blockIdx.y, bytes, x);
+    } else if (lane == 0) {
         mb.bytes[t.seg0 + c] = bytes;
         mb.last[t.seg0 + c] = x;
     }
 }
 
 // Warp b of the grid: the totals of task b (bytes, last state) through
-// tasks.put, and the running counts of its record layout, all on lane 0.
+// tasks.put, and the running counts of its record layout, all on lane 0.  Of
+// tasks in segments: a launch of its own took 67 us for 20 000 short ones.
 template <class Tasks>
 __global__ void __launch_bounds__(32) k_m12_sum(Tasks tasks, M12Bufs mb) {
     const M12Task t = tasks.get(blockIdx.x);
     const uint32_t segs = m12_segs(t.n), lane = threadIdx.x;
-    if (segs == 0) return;
+    if (segs < 2) return;
     constexpr uint32_t kPass = 4 * kStitchRounds / kM12Seg;  // segments of a stitch pass
     uint32_t above = 0;
     for (int32_t c0 = (int32_t)segs - 1; c0 >= 0; c0 -= 32) {
@@ -400,7 +405,7 @@ static cudaError_t launch_m12(const Tasks& tasks, uint32_t n, uint32_t max_codes
             k_m12_resolve<<<m, 32, 0, s>>>(part, mb, tab12);
         }
         k_m12_code<<<dim3(segs ? segs : 1, m), 32, 0, s>>>(part, mb, tab12);
-        k_m12_sum<<<m, 32, 0, s>>>(part, mb);
+        if (segs > 1) k_m12_sum<<<m, 32, 0, s>>>(part, mb);
     }
     return cudaGetLastError();
 }
