@@ -181,7 +181,10 @@ struct przmg_batch {
     // the two branches)
     cudaStream_t aux = nullptr;
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
-    cudaEvent_t ev_fork8 = nullptr, ev_join8 = nullptr;  // and around the walk of split Meta8 tasks
+    // the walk of split Meta8 tasks, on aux where there are no Mode 12 chains:
+    // the rANS launch waits for the walk, but not for the chains
+    cudaStream_t aux8 = nullptr;
+    cudaEvent_t ev_fork8 = nullptr, ev_join8 = nullptr;
     // per input i, where its items start in each work list ([i + 1] = end)
     std::vector<uint32_t> job_small0, job_rt0, job_big0, job_tile0, job_asm0;
     int launches_plain = 0;
@@ -205,7 +208,8 @@ struct przmg_batch {
         release();
         for (cudaEvent_t e : {ev_fork, ev_join, ev_fork8, ev_join8})
             if (e) cudaEventDestroy(e);
-        if (aux) cudaStreamDestroy(aux);
+        for (cudaStream_t a : {aux, aux8})
+            if (a) cudaStreamDestroy(a);
     }
     void drop_graph() {
         if (exec) cudaGraphExecDestroy(exec);
@@ -455,6 +459,7 @@ static int32_t batch_prepare(przmg_batch* b, const uint64_t* sizes, uint32_t njo
             if (!*e) CK(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
         CK(cudaStreamCreateWithFlags(&b->aux, cudaStreamNonBlocking));
     }
+    if (profile >= 2 && segb_m8 && !b->aux8) CK(cudaStreamCreateWithFlags(&b->aux8, cudaStreamNonBlocking));
     CK(b->d_ans.ensure(b->ans_bytes));
     CK(b->d_outs.ensure((size_t)njobs * T_COUNT * sizeof(TaskOut) + 16));
     CK(b->d_plans.ensure((size_t)njobs * sizeof(Plan) + 16));
@@ -752,8 +757,8 @@ static int32_t launch_range(przmg_batch* b, cudaStream_t s, int stop_after, cons
             const uint32_t nb_ad = (nad + b->seg_cap + 8 * kRansWarps - 1) / (8 * kRansWarps);
             const uint32_t nb_m8 = (3 * R.nj + b->seg_cap_m8 + 8 * kRansWarps - 1) / (8 * kRansWarps);
             CK(launch_rans(sb, lists, list_cap, counts, nb_ad, nb_m8, b->d_tabs.as<EncSym>(), c->d_meta8.as<EncSym>(),
-                           c->d_ctxlut.as<uint8_t>(), b->d_outs.as<TaskOut>(), s, b->seg_cap_m8 ? b->aux : nullptr,
-                           b->ev_fork8, b->ev_join8));
+                           c->d_ctxlut.as<uint8_t>(), b->d_outs.as<TaskOut>(), s,
+                           !b->seg_cap_m8 ? nullptr : b->profile >= 2 ? b->aux8 : b->aux, b->ev_fork8, b->ev_join8));
             launches += 3 + (sb.cap ? 3 + (b->seg_cap_m8 != 0) : 0);
             if (b->profile >= 2) CK(cudaStreamWaitEvent(s, b->ev_join, 0));  // the Mode 12 chains
             CK(mark(7));
