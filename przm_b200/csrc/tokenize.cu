@@ -110,7 +110,8 @@ __device__ uint32_t warp_match_end(const uint8_t* src, uint32_t a, uint32_t b, u
 // distance is in is a scan of the lists of the three latest distinct
 // distances.  Measured on 12 KB of records (one tile): 300 us with the
 // search, 142 us so.  Every decision
-// becomes a record in shared memory (16 bytes, the fourth word unused):
+// becomes a record in shared memory (three words: with a fourth
+// the front end's blocks, eight of these each, fit an SM twice, not three times):
 //   r0 = q - tile start | literals before q << 16
 //   r1 = match or run length | kind << 16 | repeat slot << 18
 //   r2 = offset
@@ -128,11 +129,11 @@ constexpr uint32_t kTokWarps = 4;    // warps (tiles) per block
 constexpr uint32_t kLongLit = 128;   // literal runs copied 16 bytes per lane
 constexpr uint32_t kWarpLit = 2048;  // ... by the whole warp, four loads of each lane in flight
 
-struct TokSmem {
+struct __align__(16) TokSmem {  // (desc is written 16 bytes at a time)
     uint32_t desc[kTokWin];
     uint32_t nz[kTokWin / 32];  // non-zero descriptors of the window, word per 32 entries
     uint32_t eq[kTokWin / 32];  // ... where a run of equal bytes may be a run-length token
-    uint4 rec[kTokRec];         // records (x, y, z; w unused): one 16-byte store each
+    uint32_t rec[3 * kTokRec];  // records
     uint16_t next[kTokWin];     // where the walk goes from an entry: the entry after it, or flags
 };
 // flags of a successor: the entry only passes the walk on to the one after it
@@ -272,13 +273,19 @@ __device__ __forceinline__ void copy_run(uint8_t* __restrict__ d, const uint8_t*
     for (uint32_t i = 16 * nv + t; i < n; i += T) d[i] = s[i];
 }
 
+__device__ __forceinline__ void tok_put(uint32_t* rec, uint32_t i, uint32_t r0, uint32_t r1, uint32_t r2) {
+    rec[3 * i] = r0;
+    rec[3 * i + 1] = r1;
+    rec[3 * i + 2] = r2;
+}
+
 // Writes records [0, nrec) of the warp's buffer.
-__device__ void tok_emit(const uint4* rec, uint32_t nrec, const uint8_t* tile_src, TokTileOut& o, uint32_t lane) {
+__device__ void tok_emit(const uint32_t* rec, uint32_t nrec, const uint8_t* tile_src, TokTileOut& o, uint32_t lane) {
     for (uint32_t g = 0; g < nrec; g += 32) {
         const uint32_t i = g + lane;
         const bool v = i < nrec;
         uint32_t r0 = 0, r1 = 0, r2 = 0;
-        if (v) { const uint4 x = rec[i]; r0 = x.x; r1 = x.y; r2 = x.z; }
+        if (v) { r0 = rec[3 * i]; r1 = rec[3 * i + 1]; r2 = rec[3 * i + 2]; }
         const uint32_t q = r0 & 0xFFFFu, lit = r0 >> 16, len = r1 & 0xFFFFu, kind = (r1 >> 16) & 3u, k = r1 >> 18;
         // literal-op count, op byte and the rest, per record kind
         uint32_t flush = 0, litLen = 0, base = 0;
@@ -474,10 +481,9 @@ __device__ void tokenize_tile(const uint8_t* __restrict__ in, const Job* __restr
             if (lane == 0) before = reps;
             if (v) {
                 const int k = d == before.r0 ? 0 : d == before.r1 ? 1 : d == before.r2 ? 2 : -1;
-                sm.rec[nrec + lane] =
-                    my_run ? make_uint4((q - start) | ((q - from) << 16), len | (2u << 16), 0u, 0u)
-                           : make_uint4((q - start) | ((q - from) << 16),
-                                        len | ((k >= 0 ? 1u : 0u) << 16) | ((uint32_t)(k >= 0 ? k : 0) << 18), d, 0u);
+                tok_put(sm.rec, nrec + lane, (q - start) | ((q - from) << 16),
+                        my_run ? len | (2u << 16) : len | ((k >= 0 ? 1u : 0u) << 16) | ((uint32_t)(k >= 0 ? k : 0) << 18),
+                        my_run ? 0u : d);
             }
             reps.r0 = __shfl_sync(0xFFFFFFFFu, inc.r0, 31);
             reps.r1 = __shfl_sync(0xFFFFFFFFu, inc.r1, 31);
@@ -718,7 +724,7 @@ __device__ void tokenize_tile(const uint8_t* __restrict__ in, const Job* __restr
         }
         if (cnt) flush();
         if (o.ok && litStart < end) {  // trailing literals (:440-464)
-            if (lane == 0) sm.rec[nrec] = make_uint4((end - start) | ((end - litStart) << 16), 3u << 16, 0u, 0u);
+            if (lane == 0) tok_put(sm.rec, nrec, (end - start) | ((end - litStart) << 16), 3u << 16, 0u);
             nrec++;
         }
         __syncwarp();
