@@ -764,7 +764,8 @@ static int32_t launch_range(przmg_batch* b, cudaStream_t s, int stop_after, cons
             uint32_t* counts = reinterpret_cast<uint32_t*>(lists + 2 * list_cap);
             k_task_list<<<1, 1024, 0, s>>>(b->d_jobs.as<Job>(), R.j0, R.nj, b->d_job_lens.as<uint32_t>(),
                                            b->d_s3f.as<S3Frame>(), b->d_streams.as<uint8_t>(), b->d_s3.as<uint8_t>(),
-                                           b->d_fib.as<uint8_t>(), b->d_ans.as<uint8_t>(), lists, list_cap, counts, sb);
+                                           b->d_fib.as<uint8_t>(), b->d_ans.as<uint8_t>(), b->d_infos.as<TableInfo>(), lists,
+                                           list_cap, counts, sb);
             CK(cudaGetLastError());
             const uint32_t nad = (b->profile >= 3 ? kModels : b->profile >= 2 ? 5 : 4) * R.nj;  // adaptive tasks at most
             const uint32_t nb_ad = (nad + b->seg_cap + 8 * kRansWarps - 1) / (8 * kRansWarps);

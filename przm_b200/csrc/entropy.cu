@@ -1,6 +1,7 @@
 // entropy.cu -- frequency normalisation, 4-lane interleaved rANS (V-ANS and
 // Meta8) and stitching of the lane outputs into the reference byte order.
 #include "common.cuh"
+#include "split.h"
 #include "meta8_tables.h"
 
 namespace pz {
@@ -353,17 +354,24 @@ __device__ void warp_build_table(const uint16_t* __restrict__ freq /* smem */, E
     const uint32_t present = __ballot_sync(0xFFFFFFFFu, cols != 0);
     if (cols && (lane & 1) == 0) len += 2;
     uint32_t at = len, total = act;
+    float bits = 0;  // of a symbol, by the model
+#pragma unroll
+    for (int k = 0; k < 8; k++)
+        if (f[k]) bits += (float)f[k] * (12.0f - __log2f((float)f[k]));
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
         const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, at, o), z = __shfl_up_sync(0xFFFFFFFFu, total, o);
+        const float w = __shfl_up_sync(0xFFFFFFFFu, bits, o);
         if (lane >= (uint32_t)o) {
             at += y;
             total += z;
+            bits += w;
         }
     }
     if (lane == 31) {
         info->active = total;
         info->mat_len = 2 + at;
+        info->apart = seg_apart(fmaxf(bits, 0.0f) / 4096.0f, total);
     }
     uint8_t* out = info->mat + 2 + at - len;
     if (lane < 2) {  // the row mask: the even bits of the ballot
@@ -718,15 +726,12 @@ constexpr uint32_t kNoSeg = 0xFFFFFFFFu;
 //                  the next segment's true first state (equal states, equal
 //                  symbols: the walk is the chain).  A state that is not
 //                  among them (0.2 % of the segments of text, 1.4 % of those
-//                  of uniform bytes) walks on until it is;
+//                  of uniform bytes; most where symbols have a hundredth of a
+//                  bit, see seg_apart) walks on until it is;
 //   k_rans         codes every segment from its true first state;
 //   k_seg_sums     adds the byte counts of the segments above.
 // The bytes are those of one chain from end to end.
 constexpr uint32_t kWalkers = 32;
-constexpr uint32_t kWarm = 4096;     // rounds walked above a segment
-constexpr uint32_t kSegMin = 2048;   // shortest segment, in rounds
-constexpr int kSegSizes = 24;        // lengths: 2048, 3072, 4096, 6144, 8192, ...
-__host__ __device__ constexpr uint32_t seg_len(int i) { return ((i & 1) ? 3 * kSegMin / 2 : kSegMin) << (i >> 1); }
 constexpr uint32_t kMarks = 8;       // 0: the segment's first round; m: 256 << m rounds in; the last: its end
 constexpr uint32_t kSegMax = 1776;   // segments of one call at most: 12 blocks of the walk per SM
 
@@ -743,7 +748,7 @@ struct SegBufs {
     uint32_t* bytes;   // [cap][4] bytes emitted
     uint32_t* marks;   // [cap][kMarks][4][kWalkers]
     uint32_t cap;
-    uint32_t weight;   // of the GPU's time against the call's latency (see cut_cost)
+    uint32_t weight;   // of the GPU's time against the call's latency (cut_cost, split.h)
 };
 __host__ __device__ constexpr uint64_t seg_bytes(uint32_t cap) {
     return 256 + (uint64_t)cap * (sizeof(TaskDesc) + sizeof(SplitTask) / 2 + 16 + 16 + kMarks * 4 * kWalkers * 4) + 64;
@@ -766,50 +771,26 @@ __host__ __device__ inline SegBufs seg_bufs(void* base, uint32_t cap, uint32_t w
     b.weight = weight;
     return b;
 }
-// Segments of a task of n symbols at segment length len: [0, len), [len, 2
-// len), ..., the last up to the stream's end.  1: not split, because it has
-// no more rounds than the call's cut or is hardly longer than a segment.
-__host__ __device__ inline uint32_t seg_count(uint32_t n, uint32_t len, uint32_t cut) {
-    const uint32_t rounds = (n + 3) >> 2;
-    return rounds <= cut || rounds < len + len / 2 ? 1u : (rounds + len - 1) / len;
-}
-// The cut of a call: tasks of more rounds are split.  The longest task left
-// whole takes 26 ns a round; walking the split ones takes the whole GPU 0.05
-// ns a round (SegBufs::weight times: 1 where the call waits for its result,
-// 3 where other batches in flight would use the GPU meanwhile: with ten in
-// flight 256 frames of 1 MiB take 3.1 ms a step whole and 4.2 ms split, with
-// three in flight 64 frames 3.3 and 1.7); and 0.2 ms pass before a segment
-// can be coded.  In units of 0.05 ns.  Below kCutMin rounds the walk and the
-// coding of the shortest segments (kWarm + kSegMin and kSegMin rounds) take
-// as long as the chain itself.
-constexpr uint32_t kCutMin = 2 * (kWarm + kSegMin);
-__host__ __device__ constexpr uint32_t seg_cut(int i) { return ((i & 1) ? 3 * kCutMin / 2 : kCutMin) << (i >> 1); }
-__host__ __device__ inline uint64_t cut_cost(uint64_t longest_whole, uint64_t split_rounds, uint32_t weight) {
-    return 520 * longest_whole + (split_rounds ? weight * split_rounds + 4200000 : 0);
-}
-// Most segments a task of up to n symbols, or several of n in all, can have.
-__host__ __device__ inline uint64_t seg_bound(uint64_t n) {
-    return (n >> 2) + 1 <= kCutMin ? 0 : (n >> 2) / kSegMin + 1;
-}
 inline uint32_t seg_cap(uint64_t bound) { return (uint32_t)(bound < kSegMax ? (bound + 1) & ~1ull : kSegMax); }
 
 // Task list: every active entry of [0, total) (get(e, d) fills the task and
 // says whether it is active), split by model kind and ordered longest-first
 // (by the bit length of the symbol count) so that the 8 tasks sharing a warp
-// have similar lengths and the long chains start first.  The segment length
-// is the shortest with which the tasks above the cut together have at most
-// sb.cap segments.  One block.
+// have similar lengths and the long chains start first.  Which are split is
+// best_cut's (split.h), by their rounds and models; the segment length is the
+// shortest with which the tasks above the cut together have at most sb.cap
+// segments.  One block.
 template <class Get>
-__device__ void build_task_list(uint32_t total, Get get, TaskDesc* __restrict__ lists, uint32_t list_cap,
-                                uint32_t* __restrict__ counts, const SegBufs& sb) {
+__device__ void build_task_list(uint32_t total, Get get, const TableInfo* __restrict__ infos, TaskDesc* __restrict__ lists,
+                                uint32_t list_cap, uint32_t* __restrict__ counts, const SegBufs& sb) {
     __shared__ uint32_t s_cnt[2][33];
     __shared__ uint32_t s_pos[2][33];
-    __shared__ uint32_t s_segs[kSegSizes];
+    __shared__ uint32_t s_segs[kSegSizes], s_apart[kSegSizes];
     __shared__ unsigned long long s_rounds[kSegSizes];
     __shared__ uint32_t s_len, s_nseg, s_nsplit, s_longest, s_cut;
     const uint32_t tid = threadIdx.x;
     if (tid < 66) (&s_cnt[0][0])[tid] = 0;
-    if (tid < kSegSizes) { s_segs[tid] = 0; s_rounds[tid] = 0; }
+    if (tid < kSegSizes) { s_segs[tid] = s_apart[tid] = 0; s_rounds[tid] = 0; }
     if (tid == 0) s_len = s_nseg = s_nsplit = s_longest = 0;
     __syncthreads();
     if (sb.cap) {
@@ -817,23 +798,16 @@ __device__ void build_task_list(uint32_t total, Get get, TaskDesc* __restrict__ 
             TaskDesc d;
             if (!get(e, d)) continue;
             const uint32_t rounds = (d.n + 3) >> 2;
-            int i = -1;  // the highest cut below it
-            while (i + 1 < kSegSizes && rounds > seg_cut(i + 1)) i++;
-            if (i >= 0) atomicAdd(&s_rounds[i], (unsigned long long)rounds);
+            const int i = seg_cut_below(rounds);
+            if (i >= 0) {
+                const uint32_t apart = d.m8 ? 0u : infos[d.tab].apart;  // (Meta8 symbols have three bits at least)
+                atomicAdd(&s_rounds[i], (unsigned long long)seg_walk_rounds(rounds, apart));
+                atomicMax(&s_apart[i], seg_apart_rounds(rounds, apart));
+            }
             atomicMax(&s_longest, rounds);
         }
         __syncthreads();
-        if (tid == 0) {
-            uint64_t best = cut_cost(s_longest, 0, sb.weight), above = 0;
-            s_cut = 0xFFFFFFFFu;
-            for (int i = kSegSizes - 1; i >= 0; i--) {
-                above += s_rounds[i];
-                if (above && cut_cost(seg_cut(i), above, sb.weight) < best) {
-                    best = cut_cost(seg_cut(i), above, sb.weight);
-                    s_cut = seg_cut(i);
-                }
-            }
-        }
+        if (tid == 0) s_cut = best_cut(s_rounds, s_apart, s_longest, sb.weight);
         __syncthreads();
         for (uint32_t e = tid; e < total && s_cut != 0xFFFFFFFFu; e += blockDim.x) {
             TaskDesc d;
@@ -909,8 +883,9 @@ __global__ void __launch_bounds__(1024) k_task_list(const Job* __restrict__ jobs
                                                     const uint32_t* __restrict__ job_lens,
                                                     const S3Frame* __restrict__ s3f, const uint8_t* __restrict__ streams,
                                                     const uint8_t* __restrict__ s3base, const uint8_t* __restrict__ fibbase,
-                                                    uint8_t* __restrict__ ans, TaskDesc* __restrict__ lists,
-                                                    uint32_t list_cap, uint32_t* __restrict__ counts, SegBufs sb) {
+                                                    uint8_t* __restrict__ ans, const TableInfo* __restrict__ infos,
+                                                    TaskDesc* __restrict__ lists, uint32_t list_cap,
+                                                    uint32_t* __restrict__ counts, SegBufs sb) {
     auto get = [&](uint32_t e, TaskDesc& d) {
         const uint32_t j = j0 + e / T_COUNT;
         const int t = (int)(e % T_COUNT);
@@ -929,7 +904,7 @@ __global__ void __launch_bounds__(1024) k_task_list(const Job* __restrict__ jobs
         d.m8 = task_is_m8(t) ? 1u : 0u;
         return true;
     };
-    build_task_list(njobs * T_COUNT, get, lists, list_cap, counts, sb);
+    build_task_list(njobs * T_COUNT, get, infos, lists, list_cap, counts, sb);
 }
 
 // A symbol's entry as the walk takes it: {m, t1, c, (4096 - f) << 5 | s} of

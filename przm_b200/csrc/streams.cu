@@ -104,10 +104,10 @@ __global__ void k_stream_norm(const STask* __restrict__ tasks, uint32_t ntasks, 
 // The streams with symbols as the rANS kernel's task list (lists[list_cap],
 // counts[0]; no Meta8 tasks).
 __global__ void __launch_bounds__(1024) k_stream_list(const STask* __restrict__ tasks, uint32_t ntasks,
-                                                      TaskDesc* __restrict__ lists, uint32_t list_cap,
+                                                      const TableInfo* __restrict__ infos, TaskDesc* __restrict__ lists, uint32_t list_cap,
                                                       uint32_t* __restrict__ counts, SegBufs sb) {
     auto get = [&](uint32_t e, TaskDesc& d) { return stream_desc(tasks[e], e, d); };
-    build_task_list(ntasks, get, lists, list_cap, counts, sb);
+    build_task_list(ntasks, get, infos, lists, list_cap, counts, sb);
 }
 
 constexpr int kStitchThreads = 256;

@@ -1,0 +1,127 @@
+"""Which rANS tasks are coded as segments: the rule by rounds, and its estimate
+of the rounds that stay apart against walkers restated here.  (CPU)"""
+from __future__ import annotations
+
+import ctypes as C
+import os
+import subprocess
+
+import numpy as np
+import pytest
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "przm_b200", "csrc")
+SHIM = """
+#include "split.h"
+extern "C" uint32_t apart(float bits, uint32_t symbols) { return pz::seg_apart(bits, symbols); }
+extern "C" uint32_t cut(const uint32_t* rounds, const uint32_t* apart, uint32_t n, uint32_t weight) {
+    unsigned long long walk[pz::kSegSizes] = {};
+    uint32_t most[pz::kSegSizes] = {}, longest = 0;
+    for (uint32_t k = 0; k < n; k++) {
+        const int i = pz::seg_cut_below(rounds[k]);
+        longest = rounds[k] > longest ? rounds[k] : longest;
+        if (i < 0) continue;
+        walk[i] += pz::seg_walk_rounds(rounds[k], apart[k]);
+        const uint32_t a = pz::seg_apart_rounds(rounds[k], apart[k]);
+        most[i] = a > most[i] ? a : most[i];
+    }
+    return pz::best_cut(walk, most, longest, weight);
+}
+"""
+WHOLE = 0xFFFFFFFF
+M = 1 << 18  # rounds of a stream of 1 MiB
+
+
+@pytest.fixture(scope="module")
+def rule(tmp_path_factory):
+    d = tmp_path_factory.mktemp("split")
+    (d / "shim.cpp").write_text(SHIM)
+    so = d / "shim.so"
+    subprocess.run(["g++", "-std=c++17", "-O1", "-shared", "-fPIC", "-I", CSRC, "-o", so, d / "shim.cpp"], check=True)
+    lib = C.CDLL(str(so))
+    lib.apart.argtypes = [C.c_float, C.c_uint32]
+    lib.apart.restype = lib.cut.restype = C.c_uint32
+    return lib
+
+
+def apart(rule, weights) -> int:
+    f = np.array([w for w in weights if w], float)
+    assert f.sum() == 4096
+    return rule.apart(float((f * (12 - np.log2(f))).sum() / 4096), len(f))
+
+
+def cut(rule, tasks, weight=1) -> int:
+    r = np.array([t[0] for t in tasks], np.uint32)
+    a = np.array([t[1] for t in tasks], np.uint32)
+    p = lambda x: x.ctypes.data_as(C.POINTER(C.c_uint32))
+    return rule.cut(p(r), p(a), len(r), weight)
+
+
+def one(p: float, others: int = 1) -> list[int]:
+    """Weights of a symbol of probability p and of others of equal ones."""
+    rest = max(others, round(4096 * (1 - p)))
+    w = [rest // others + (i < rest % others) for i in range(others)]
+    return [4096 - sum(w)] + w
+
+
+def test_models_of_a_bit_and_more_are_not_held_back(rule):
+    for w in ([16] * 256, [1024] * 4, one(0.8, 15), one(0.7), [4096]):
+        assert apart(rule, w) == 0
+
+
+@pytest.mark.parametrize("tasks,weight,split", [
+    # the figures beside the rule: text as before the models counted
+    ([(M, 0)] * 64, 1, True), ([(M, 0)] * 64, 3, True), ([(M, 0)] * 256, 1, True), ([(M, 0)] * 256, 3, False),
+    ([(4 * M, 0)], 1, True), ([(12_288, 0)], 1, False), ([(15_000, 0)], 1, False), ([(24_000, 0)], 1, True),
+    # 64 streams of 1 MiB, by the probability of their first symbol: whole from where segments take longer
+    ([(M, 0.95)] * 64, 1, True), ([(M, 0.99)] * 64, 1, True), ([(M, 0.995)] * 64, 1, False), ([(M, 0.999)] * 64, 1, False),
+    ([(M, 0.9999)] * 64, 1, False), ([(M, 0.99)] * 64, 3, False),
+    # one stream of 4 MiB
+    ([(4 * M, 0.99)], 1, True), ([(4 * M, 0.999)], 1, True), ([(4 * M, 0.9999)], 1, False),
+    # one long stream of text among short ones that stay apart: it alone is split
+    ([(4 * M, 0)] + [(20_000, 0.999)] * 200, 1, True),
+])
+def test_what_is_split(rule, tasks, weight, split):
+    t = [(r, apart(rule, one(p)) if p else 0) for r, p in tasks]
+    c = cut(rule, t, weight)
+    assert (c != WHOLE) == split
+    if split and len(set(t)) > 1:
+        assert 20_000 <= c < 4 * M
+
+
+def step(x, f, c):
+    """The encoder's step, on arrays of states."""
+    x = np.where(x >= f << 20, x >> 16, np.where(x >= f << 12, x >> 8, x))
+    return (x // f << 12) + x % f + c
+
+
+def share_apart(weights: list[int], seed: int, streams: int = 160) -> float:
+    """The share of segments of 2048 rounds whose true first state no walker has."""
+    w = np.array(weights, np.int64)
+    cum = np.concatenate([[0], np.cumsum(w)[:-1]])
+    rng = np.random.default_rng(seed)
+    k = np.arange(64)
+    x = np.concatenate([np.full((streams, 1), 65536, np.int64),
+                        np.tile((np.exp2(k % 8 / 8) * 65536).astype(np.int64) << (k // 8), (streams, 1))], 1)
+    for i in range(6000 + 4096):
+        s = rng.choice(len(w), streams, p=w / 4096)
+        f, c = w[s][:, None], cum[s][:, None]
+        if i < 6000:  # the true state alone
+            x[:, :1] = step(x[:, :1], f, c)
+            continue
+        x = step(x, f, c)
+        if (i - 6000) % 512 == 511 and (i - 6000) // 512 == 5:  # 32 of what is left, in ring order
+            for row in x:
+                r = row[1:]
+                d = r[r != np.roll(r, 1)] if (r != np.roll(r, 1)).any() else r[:1]
+                pick = d[np.minimum(np.arange(32), len(d) - 1)] if len(d) <= 32 else d[np.arange(32) * len(d) // 32]
+                row[1:] = np.concatenate([pick, pick])
+    return float((x[:, 1:] != x[:, :1]).all(1).mean())
+
+
+@pytest.mark.parametrize("weights", [one(0.999), one(0.99), one(0.98), one(0.95), one(0.9), one(0.99, 15), one(0.8, 15), [16] * 256],
+                         ids=["999", "99", "98", "95", "90", "99 of 16", "80 of 16", "uniform"])
+def test_the_estimate_against_the_walk(rule, weights):
+    # it stands for the slowest of many lanes: not below the mean share by more
+    # than 160 segments tell (three standard deviations, 0.12), and above by 0.2 at most
+    share, told = share_apart(weights, 3), apart(rule, weights) / 256
+    assert share - 0.12 <= told <= share + 0.2, (share, told)
