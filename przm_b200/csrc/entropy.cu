@@ -18,7 +18,10 @@ __host__ __device__ inline EncSym make_encsym(uint32_t f, uint32_t c) {
     if (f == 0) { e.m = 0; e.t1 = 0xFFFFFFFFu; e.t2 = 0xFFFFFFFFu; e.w = 0; return e; }
     uint32_t s = 0;
     while ((2u << s) <= f) s++;  // floor(log2 f)
-    if (f == 1) { e.m = 1u << 31; s = 31; }
+    // (a caller's table may hold any weight: above 4096 the fields of w run over,
+    // the shift to 32 and more, and the quotient is 0)
+    if (f > 4096) e.m = 0;
+    else if (f == 1) { e.m = 1u << 31; s = 31; }
     else if ((f & (f - 1)) == 0) { e.m = 1u << (32 - s); s = 0; }
     else e.m = (uint32_t)(((1ull << (32 + s)) + f - 1) / f);
     e.t1 = 4096u * f;
