@@ -465,8 +465,8 @@ static int32_t batch_prepare(przmg_batch* b, const uint64_t* sizes, uint32_t njo
     CK(b->d_plans.ensure((size_t)njobs * sizeof(Plan) + 16));
     CK(b->d_out.ensure(b->out_bytes));
     CK(b->d_misc.ensure(64));
-    b->seg_cap = seg_cap(segb);
-    b->seg_cap_m8 = std::min(seg_cap(segb_m8), b->seg_cap);
+    b->seg_cap = seg_cap(segb, (uint32_t)b->ctx->sms);
+    b->seg_cap_m8 = std::min(seg_cap(segb_m8, (uint32_t)b->ctx->sms), b->seg_cap);
     CK(b->d_lists.ensure((size_t)2 * (kModels * std::max<uint32_t>(njobs, 1) + b->seg_cap) * sizeof(TaskDesc) + 64));
     CK(b->d_seg.ensure(seg_bytes(b->seg_cap)));
     if (b->nbig) {
@@ -759,7 +759,7 @@ static int32_t launch_range(przmg_batch* b, cudaStream_t s, int stop_after, cons
             CK(cudaGetLastError());
             CK(mark(6));
             const uint32_t list_cap = kModels * b->njobs + b->seg_cap;
-            const SegBufs sb = seg_bufs(b->d_seg.p, b->seg_cap, b == &c->single ? 1u : 3u);
+            const SegBufs sb = seg_bufs(b->d_seg.p, b->seg_cap, (uint32_t)c->sms, b == &c->single ? 1u : 3u);
             TaskDesc* lists = b->d_lists.as<TaskDesc>();
             uint32_t* counts = reinterpret_cast<uint32_t*>(lists + 2 * list_cap);
             k_task_list<<<1, 1024, 0, s>>>(b->d_jobs.as<Job>(), R.j0, R.nj, b->d_job_lens.as<uint32_t>(),

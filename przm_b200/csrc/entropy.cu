@@ -736,7 +736,7 @@ constexpr uint32_t kNoSeg = 0xFFFFFFFFu;
 // The bytes are those of one chain from end to end.
 constexpr uint32_t kWalkers = 32;
 constexpr uint32_t kMarks = 8;       // 0: the segment's first round; m: 256 << m rounds in; the last: its end
-constexpr uint32_t kSegMax = 1776;   // segments of one call at most: 12 blocks of the walk per SM
+constexpr uint32_t kSegMax = 1776;   // segments of one call at most, and 12 per SM: as many blocks of the walk
 
 struct SplitTask {
     TaskDesc d;
@@ -752,11 +752,12 @@ struct SegBufs {
     uint32_t* marks;   // [cap][kMarks][4][kWalkers]
     uint32_t cap;
     uint32_t weight;   // of the GPU's time against the call's latency (cut_cost, split.h)
+    uint32_t sms;      // of the device
 };
 __host__ __device__ constexpr uint64_t seg_bytes(uint32_t cap) {
     return 256 + (uint64_t)cap * (sizeof(TaskDesc) + sizeof(SplitTask) / 2 + 16 + 16 + kMarks * 4 * kWalkers * 4) + 64;
 }
-__host__ __device__ inline SegBufs seg_bufs(void* base, uint32_t cap, uint32_t weight = 1) {
+__host__ __device__ inline SegBufs seg_bufs(void* base, uint32_t cap, uint32_t sms, uint32_t weight = 1) {
     SegBufs b;
     uint8_t* p = static_cast<uint8_t*>(base);
     b.ctl = reinterpret_cast<uint32_t*>(p);
@@ -772,9 +773,13 @@ __host__ __device__ inline SegBufs seg_bufs(void* base, uint32_t cap, uint32_t w
     b.marks = reinterpret_cast<uint32_t*>(p);
     b.cap = cap;
     b.weight = weight;
+    b.sms = sms;
     return b;
 }
-inline uint32_t seg_cap(uint64_t bound) { return (uint32_t)(bound < kSegMax ? (bound + 1) & ~1ull : kSegMax); }
+inline uint32_t seg_cap(uint64_t bound, uint32_t sms) {
+    const uint32_t most = 12 * sms < kSegMax ? 12 * sms : kSegMax;
+    return (uint32_t)(bound < most ? (bound + 1) & ~1ull : most);
+}
 
 // Task list: every active entry of [0, total) (get(e, d) fills the task and
 // says whether it is active), split by model kind and ordered longest-first
@@ -1114,7 +1119,7 @@ __global__ void __launch_bounds__(kWalkThreads, kMeta8 ? 4 : 12) k_seg_walk(SegB
     uint16_t* stage = reinterpret_cast<uint16_t*>(smem_w + kTab * 16 + (kMeta8 ? 256 : 0));
     const EncSym* gt = kMeta8 ? meta8 : tabs + (uint64_t)d.tab * 256;
     // the form with the short chain once at most two of its warps share a scheduler
-    auto latency = [&](uint32_t mode) { return nseg * (4u >> mode) <= 2u * 4 * 148; };
+    auto latency = [&](uint32_t mode) { return nseg * (4u >> mode) <= 2u * 4 * sb.sms; };
     uint32_t mode = 0;  // mode 0, 1, 2: 32, 16, 8 states of a lane
     bool first_form = !latency(mode);
     for (uint32_t i = tid; i < kTab; i += kWalkThreads) {
