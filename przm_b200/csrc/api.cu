@@ -155,11 +155,13 @@ struct przmg_batch {
     DevBuf d_in, d_desc, d_slots, d_tile_lens, d_streams, d_hist, d_tabs, d_infos, d_ans, d_outs, d_plans, d_out, d_misc,
         d_lists;
     // the tables that describe the batch, laid out by batch_prepare in one
-    // buffer and uploaded from h_layout by one copy (nine copies of a few
-    // hundred bytes and a wait cost a one-input call 70 us); the frame sizes
-    // and stream lengths lie behind them and start as zeros
+    // buffer and uploaded by one copy (nine copies of a few hundred bytes and a
+    // wait cost a one-input call 70 us), from h_layout where a batch is laid out
+    // again and again; the frame sizes and stream lengths lie behind them and
+    // start as zeros
     DevBuf d_layout;
     HostBuf h_layout;
+    bool laid_out = false;
     bool layout_in_flight = false;  // h_layout may still be read by a copy on the context's stream
     DevPart d_jobs, d_small, d_big, d_tiles, d_job_lens, d_sizes, d_rtiles, d_up_offs, d_asm, d_asm_job, d_m12_seg0;
     // radix-strike tables (one per finder CTA) and the packed upload/download
@@ -497,16 +499,28 @@ static int32_t batch_prepare(przmg_batch* b, const uint64_t* sizes, uint32_t njo
     size_t layout = 0;
     for (const auto& t : tables) layout += align64(t.bytes + 16);
     CK(b->d_layout.ensure(layout));
-    CK(b->h_layout.ensure(layout));
+    // pinned memory of its own would cost a batch that is laid out once far more
+    // than the copy (creating one of a 1000-byte input 1.5 to 3.5 ms with it,
+    // 0.05 ms without; 64 of 1 MiB 5.7 and 3.3 ms)
+    std::vector<uint8_t> once;
+    uint8_t* host = nullptr;
+    if (b == &b->ctx->single || b->laid_out) {
+        CK(b->h_layout.ensure(layout));
+        host = b->h_layout.as<uint8_t>();
+    } else {
+        once.resize(layout);
+        host = once.data();
+    }
+    b->laid_out = true;
     size_t at = 0;
     for (const auto& t : tables) {
-        uint8_t* h = b->h_layout.as<uint8_t>() + at;
+        uint8_t* h = host + at;
         if (t.src && t.bytes) std::memcpy(h, t.src, t.bytes);
         if (!t.src) std::memset(h, 0, t.bytes);
         t.part->p = b->d_layout.as<uint8_t>() + at;
         at += align64(t.bytes + 16);
     }
-    CK(cudaMemcpyAsync(b->d_layout.p, b->h_layout.p, layout, cudaMemcpyHostToDevice, s));
+    CK(cudaMemcpyAsync(b->d_layout.p, host, layout, cudaMemcpyHostToDevice, s));
     if (b->front) {
         CK(cudaMemcpyAsync(b->d_fitems.p, fitems.data(), sizeof(FrontItem) * fitems.size(), cudaMemcpyHostToDevice, s));
         if (!ftiles.empty())
