@@ -82,6 +82,16 @@ def test_launches_of_a_short_frame(comp):
     assert len(ks) == 6, ks  # parse, static models, adaptive bodies, prefix, sheaf, commands
 
 
+@pytest.mark.parametrize("count,listed", [(19, False), (512, False), (513, True)])
+def test_short_bodies_need_no_list(comp, count, listed):
+    x = W.gen("markov", 1, 700)
+    fr = comp.Compress(x, 1)[0]
+    ks = [n for n, _ in kernels(lambda: decode(comp, [fr] * count, [700] * count))]
+    assert ("k_dec_lists" in ks) == listed, ks
+    st, outs = decode(comp, [fr] * count, [700] * count)
+    assert st == [0] * count and outs == [x.tobytes()] * count
+
+
 @pytest.mark.parametrize("profile", [0, 1])
 def test_many_short_frames_cost_less_than_empty_slots(comp, profile):
     # k_dec_static only finds that these frames' 160 000 slots have no static body: 112 us
