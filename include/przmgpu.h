@@ -458,7 +458,9 @@ int32_t przmg_decompress(przmg_ctx* ctx, const uint8_t* src, uint64_t src_len, u
 /* count device-resident frames (d_src + src_offs[i], src_lens[i] bytes) into
  * d_dst + dst_offs[i] (dst_caps[i] bytes): status[i] (PRZMG_OK or the frame's
  * error) and out_lens[i] per frame; waits for the work (enqueued on
- * `stream`, 0 = the context's).  The return value is the call's own status. */
+ * `stream`, 0 = the context's).  The return value is the call's own status.
+ * A frame and an output are read in whole aligned units of up to 16 bytes, so
+ * bytes beside them in those units are read (not used, and not written). */
 int32_t przmg_decompress_batch_device(przmg_ctx* ctx, uint64_t d_src, const uint64_t* src_offs,
                                       const uint32_t* src_lens, uint64_t count, uint64_t d_dst,
                                       const uint64_t* dst_offs, const uint32_t* dst_caps, int32_t* status,

@@ -35,7 +35,9 @@
 // normalisation flag, delta-masked matches, the nibble-plane literal form,
 // the dictionary-word opcodes) come back as PRZMG_ERR_UNSUPPORTED; they
 // decode on the host.  Every read of a frame is bounds-checked against its
-// length, every write against the capacities the host gave.
+// length, every write against the capacities the host gave; some loads take the
+// whole aligned unit of 4 or 16 bytes around the bytes they want, so they also
+// read what lies beside a frame or an output in its last unit.
 #include "common.cuh"
 
 namespace pz {

@@ -208,12 +208,12 @@ struct GoSort {
 // symbol first among equal ones), of a histogram whose counts lie in at most
 // four groups of 32 symbols (bits of `groups`): the others are left out on both
 // sides of the comparisons.  Measured with all eight: 2000 streams of 300 bytes
-// of text 40 us in k_stream_norm, one 17.3; 15 and 11 so, and alphabets in more
-// groups as before where this is a function of its own, 4 us longer with it
-// inline.  (The comparison
-// in bitwise form: with short-circuits it was branches, five times as long.)
+// of text 40 us in k_stream_norm, one 17.3; 15 and 11 so.  A function of its
+// own, because inline it made alphabets in more groups 4 us longer; the
+// comparison in bitwise form, because with short-circuits it was branches, five
+// times as long.
 __device__ __noinline__ void warp_raise_largest4(const uint32_t* __restrict__ cnt, uint16_t* __restrict__ freq,
-                                                    uint32_t groups, uint32_t diff, uint32_t lane) {
+                                                 uint32_t groups, uint32_t diff, uint32_t lane) {
     uint32_t c[4], id[4], rank[4], m = groups;
 #pragma unroll
     for (int k = 0; k < 4; k++) {
@@ -440,8 +440,7 @@ __global__ void __launch_bounds__(32 * kModels) k_normalize(const Job* __restric
 // lanes' bytes into one stream in processing order and reverses it; here each
 // lane writes its own bytes in order together with 2-bit counts per round,
 // and the stitch below interleaves them into exactly that reversed stream.
-// The division is a multiply-high by a per-symbol reciprocal (exact for
-// x < 2^24, see EncSym).
+// The division is a multiply-high by a per-symbol reciprocal (see EncSym).
 // ---------------------------------------------------------------------------
 struct LaneIO {
     uint8_t* bytes;     // lane byte stream

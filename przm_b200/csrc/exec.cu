@@ -388,7 +388,7 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_dec_exec(const uint8_t* __res
     };
     fetch();
     for (;;) {
-        // the chunk's commands: the next 512 opcodes, or in a flat stream the
+        // the chunk's commands: the next NT opcodes, or in a flat stream the
         // commands that one thread finds in its next bytes
         uint32_t n = min(NT, cl - cp), at = cp + tid;
         if (!split) {
