@@ -50,14 +50,16 @@ PZ_HD inline uint32_t seg_apart(float bits, uint32_t symbols) {
 // use the GPU meanwhile: with ten in flight 256 frames of 1 MiB take 3.1 ms a
 // step whole and 4.2 ms split, with three in flight 64 frames 3.3 and 1.7); the
 // rounds that stay apart are walked again one after another, 24 ns each, task
-// by task side by side, 27 with what a segment's coding takes meanwhile; and 0.2
-// ms pass before a segment can be coded.  In units of 0.05 ns.  Below kCutMin
+// by task side by side, 27 with what a segment's coding takes meanwhile, less
+// what the lowest cut counts as left whole where they are longer; and 0.2 ms
+// pass before a segment can be coded.  In units of 0.05 ns.  Below kCutMin
 // rounds the walk and the coding of the shortest segments (kWarm + kSegMin and
 // kSegMin rounds) take as long as the chain itself.  Measured on 64 streams of
 // 1 MiB (all kernels, whole and split, ms): 5.8 bits a symbol 8.0 and 2.7, 0.081
 // bits 7.3 and 6.7, 0.046 bits 7.0 and 8.3, 0.012 bits 7.3 and 9.0; one stream
-// of 4 MiB at 0.012 bits 26.4 and 21.9, at 0.0016 bits 26.4 and 26.7.  One of
-// 256 KiB at 0.012 bits is left whole at 1.7 where segments take 1.5.
+// of 4 MiB at 0.012 bits 26.4 and 21.9, at 0.0016 bits 26.4 and 26.7; 256 of
+// 256 KiB at 0.081 bits (the call) 1.9 and 4.3, 200 of 1 MiB 7.2 and 11.1; one of
+// 256 KiB at 0.046 bits 1.7 and 1.4, at 0.012 bits 1.7 and 1.5 (left whole).
 constexpr uint32_t kCutMin = 2 * (kWarm + kSegMin);
 PZ_HD constexpr uint32_t seg_cut(int i) { return ((i & 1) ? 3 * kCutMin / 2 : kCutMin) << (i >> 1); }
 PZ_HD inline int seg_cut_below(uint32_t rounds) {  // the highest cut below it, -1: none
@@ -66,7 +68,9 @@ PZ_HD inline int seg_cut_below(uint32_t rounds) {  // the highest cut below it, 
     return i;
 }
 PZ_HD inline uint64_t cut_cost(uint64_t longest_whole, uint64_t walk_rounds, uint64_t apart_rounds, uint32_t weight) {
-    return 520 * longest_whole + (walk_rounds ? weight * walk_rounds + 540 * apart_rounds + 4200000 : 0);
+    const uint64_t apart = 540 * apart_rounds, counted = 520 * kCutMin;
+    return 520 * longest_whole +
+           (walk_rounds ? weight * walk_rounds + (apart > counted ? apart - counted : 0) + 4200000 : 0);
 }
 // A task's rounds as its walk costs them, and those that stay apart.
 PZ_HD inline uint64_t seg_walk_rounds(uint32_t rounds, uint32_t apart) { return rounds + (uint64_t)rounds * apart * 3 / 512; }

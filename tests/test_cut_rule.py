@@ -77,6 +77,8 @@ def test_models_of_a_bit_and_more_are_not_held_back(rule):
     ([(M, 0.9999)] * 64, 1, False), ([(M, 0.99)] * 64, 3, False),
     # one stream of 4 MiB
     ([(4 * M, 0.99)], 1, True), ([(4 * M, 0.999)], 1, True), ([(4 * M, 0.9999)], 1, False),
+    # one stream of 256 KiB
+    ([(M // 4, 0.99)], 1, True), ([(M // 4, 0.995)], 1, True), ([(M // 4, 0.9999)], 1, False),
     # one long stream of text among short ones that stay apart: it alone is split
     ([(4 * M, 0)] + [(20_000, 0.999)] * 200, 1, True),
 ])
