@@ -259,7 +259,7 @@ struct TableInfo {            // adaptive model of one (job, stream)
     uint32_t mat_len;
     uint32_t active;
     uint8_t mat[600];         // serialized 16x16 joint-nibble matrix (<= 2 + 32 + 512)
-    uint32_t apart;           // share of a long chain that segments leave to be walked on, in 1/256 (seg_apart)
+    uint32_t apart;           // how the walkers of its segments fall together (seg_apart)
 };
 
 // ---- device helpers --------------------------------------------------------

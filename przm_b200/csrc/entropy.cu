@@ -357,24 +357,27 @@ __device__ void warp_build_table(const uint16_t* __restrict__ freq /* smem */, E
     const uint32_t present = __ballot_sync(0xFFFFFFFFu, cols != 0);
     if (cols && (lane & 1) == 0) len += 2;
     uint32_t at = len, total = act;
-    float bits = 0;  // of a symbol, by the model
+    uint32_t most = 0, off = 0;  // what seg_apart asks of the model
 #pragma unroll
     for (int k = 0; k < 8; k++)
-        if (f[k]) bits += (float)f[k] * (12.0f - __log2f((float)f[k]));
+        if (f[k]) {
+            most = max(most, f[k]);
+            off += seg_off_power(f[k]);
+        }
+    most = __reduce_max_sync(0xFFFFFFFFu, most);
+    off = __reduce_add_sync(0xFFFFFFFFu, off);
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
         const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, at, o), z = __shfl_up_sync(0xFFFFFFFFu, total, o);
-        const float w = __shfl_up_sync(0xFFFFFFFFu, bits, o);
         if (lane >= (uint32_t)o) {
             at += y;
             total += z;
-            bits += w;
         }
     }
     if (lane == 31) {
         info->active = total;
         info->mat_len = 2 + at;
-        info->apart = seg_apart(fmaxf(bits, 0.0f) / 4096.0f, total);
+        info->apart = seg_apart(most, total, off / 4096);
     }
     uint8_t* out = info->mat + 2 + at - len;
     if (lane < 2) {  // the row mask: the even bits of the ballot
@@ -728,8 +731,8 @@ constexpr uint32_t kNoSeg = 0xFFFFFFFFu;
 //                  the next segment's true first state (equal states, equal
 //                  symbols: the walk is the chain).  A state that is not
 //                  among them (0.2 % of the segments of text, 1.4 % of those
-//                  of uniform bytes; most where symbols have a hundredth of a
-//                  bit, see seg_apart) walks on until it is;
+//                  of uniform bytes; most where one symbol has 99 % and more,
+//                  see seg_apart) walks on until it is;
 //   k_rans         codes every segment from its true first state;
 //   k_seg_sums     adds the byte counts of the segments above.
 // The bytes are those of one chain from end to end.
@@ -807,7 +810,7 @@ __device__ void build_task_list(uint32_t total, Get get, const TableInfo* __rest
             const uint32_t rounds = (d.n + 3) >> 2;
             const int i = seg_cut_below(rounds);
             if (i >= 0) {
-                const uint32_t apart = d.m8 ? 0u : infos[d.tab].apart;  // (Meta8 symbols have three bits at least)
+                const uint32_t apart = d.m8 ? 0u : infos[d.tab].apart;  // (Meta8 models have no symbol so frequent)
                 atomicAdd(&s_rounds[i], (unsigned long long)seg_walk_rounds(rounds, apart));
                 atomicMax(&s_apart[i], seg_apart_rounds(rounds, apart));
             }

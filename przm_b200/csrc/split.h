@@ -19,6 +19,8 @@ constexpr uint32_t kSegMin = 2048;   // shortest segment, in rounds
 constexpr int kSegSizes = 24;        // lengths: 2048, 3072, 4096, 6144, 8192, ...
 PZ_HD constexpr uint32_t seg_len(int i) { return ((i & 1) ? 3 * kSegMin / 2 : kSegMin) << (i >> 1); }
 
+constexpr uint32_t kOffPowers = 918;  // 0.014, see seg_apart
+
 // Segments of a task of n symbols at segment length len: [0, len), [len, 2
 // len), ..., the last up to the stream's end.  1: not split, because it has
 // no more rounds than the call's cut or is hardly longer than a segment.
@@ -27,39 +29,63 @@ PZ_HD inline uint32_t seg_count(uint32_t n, uint32_t len, uint32_t cut) {
     return rounds <= cut || rounds < len + len / 2 ? 1u : (rounds + len - 1) / len;
 }
 
-// Share of a long chain's rounds, in 1/256, that lie in segments whose first
-// state no walker has, so that they are walked one after another
-// (k_seg_resolve).  States fall together where bytes are shifted out, so it
-// depends on the model's bits a symbol.  Measured on the slowest of 256 lanes of
-// 1 MiB streams, by that kernel's time over 24 ns a round of the chain: 0.96 at
-// 0.012 bits, 0.83 at 0.046, 0.64 at 0.081, 0.51 at 0.14, 0.33 at 0.29, 0.20 at
-// 0.37, 0.07 at 0.52, 0.02 and less from 0.6 on (one symbol of 90 to 99.9 %, the
-// others equal or geometric); the line through these.  Not told by the bits:
-// few symbols of equal frequencies that are powers of two, whose states keep
-// their distances (two symbols 0.81, four 0.45, sixteen 0.25).  A single symbol
-// leaves a state as it is, so the walkers have it.
-PZ_HD inline uint32_t seg_apart(float bits, uint32_t symbols) {
-    const float share = 1.05f - 1.4f * sqrtf(bits);
-    return symbols < 2 || !(share > 0.0f) ? 0u : share < 1.0f ? (uint32_t)(256.0f * share) : 256u;
+// How a model's walkers fall together, in 1/256: low half, the share of a long
+// chain's rounds that lie in segments whose first state no walker has, so that
+// they are walked one after another (k_seg_resolve); high half, what the walk
+// itself takes more because its walkers stay many.
+//   By the rate of all symbols but the most frequent: states fall together where
+//   symbols shift them out or set them anew.  Restated on the CPU (256 segments,
+//   one other symbol, three, 15 or six geometric ones, which do not matter): 0.91
+//   at 0.001, 0.55 at 0.01, 0.4 at 0.02, 0.3 at 0.03, 0.17 at 0.05, 0.06 at 0.07,
+//   none at 0.1; of the slowest of 256 lanes a little more; the line through these.
+//   By how far frequencies are from powers of two (the mean of |log2 f| less the
+//   nearest whole number; 1.0 stands for 65536): steps by nearly such
+//   frequencies keep the states' distances.  0.2 to 0.45 below 0.002, 0.2 at 0.005,
+//   0.1 at 0.009 and none from 0.014 on, of the slowest lane 0.4 to 0.7 (coin
+//   tosses, four or 16 equally likely symbols; of 32 and more the counts of 4 MiB
+//   and less are farther off).  Exact powers lose no first state, but hardly a
+//   walker falls onto another.
+// A single symbol leaves a state as it is, so the walkers have it.
+PZ_HD inline uint32_t seg_apart(uint32_t most, uint32_t symbols, uint32_t off_powers) {
+    if (symbols < 2) return 0;
+    const float root = sqrtf((float)(4096 - (int)most > 0 ? 4096 - most : 0) / 4096.0f);
+    float share = fmaxf(1.02f - 3.8f * root, 0.0f), slow = fminf(fmaxf(1.2f - 2.0f * root, 0.0f), 0.8f);
+    if (off_powers < kOffPowers) {
+        const float kept = 0.67f - 0.67f / kOffPowers * (float)off_powers;
+        slow = fmaxf(slow, fminf(4.0f * kept, 0.8f));
+        if (off_powers) share = fmaxf(share, kept);
+    }
+    return (uint32_t)(256.0f * share) | (uint32_t)(256.0f * slow) << 16;
+}
+// A symbol's part of off_powers, times its frequency; the sum's 4096th is it.
+PZ_HD inline uint32_t seg_off_power(uint32_t f) {
+    if ((f & (f - 1)) == 0) return 0;
+    const float l = log2f((float)f);
+    return (uint32_t)(65536.0f * fabsf(l - rintf(l)) * (float)f);
 }
 
 // The cut of a call: tasks of more rounds are split.  The longest task left
 // whole takes 26 ns a round; walking the split ones takes the whole GPU 0.05
-// ns a round, up to 2.5 times that where all walkers stay apart (weight times:
+// ns a round, up to 1.8 times that where walkers stay many (weight times:
 // 1 where the call waits for its result, 3 where other batches in flight would
 // use the GPU meanwhile: with ten in flight 256 frames of 1 MiB take 3.1 ms a
-// step whole and 4.2 ms split, with three in flight 64 frames 3.3 and 1.7); the
-// rounds that stay apart are walked again one after another, 24 ns each, task
-// by task side by side, 27 with what a segment's coding takes meanwhile, less
-// what the lowest cut counts as left whole where they are longer; and 0.2 ms
-// pass before a segment can be coded.  In units of 0.05 ns.  Below kCutMin
+// step whole and 4.2 ms split, with three in flight 64 frames 3.3 and 1.7), and
+// coding them 0.008; the rounds that stay apart are walked again one after another,
+// 27 ns each, task by task side by side, 0.2 ms more where there are many; and 0.2
+// ms pass before a segment can be coded.  The lowest cut counts as a chain of
+// kCutMin rounds left whole also where nothing is, so that much of the rounds
+// that stay apart is counted already.  In units of 0.05 ns.  Below kCutMin
 // rounds the walk and the coding of the shortest segments (kWarm + kSegMin and
-// kSegMin rounds) take as long as the chain itself.  Measured on 64 streams of
-// 1 MiB (all kernels, whole and split, ms): 5.8 bits a symbol 8.0 and 2.7, 0.081
-// bits 7.3 and 6.7, 0.046 bits 7.0 and 8.3, 0.012 bits 7.3 and 9.0; one stream
-// of 4 MiB at 0.012 bits 26.4 and 21.9, at 0.0016 bits 26.4 and 26.7; 256 of
-// 256 KiB at 0.081 bits (the call) 1.9 and 4.3, 200 of 1 MiB 7.2 and 11.1; one of
-// 256 KiB at 0.046 bits 1.7 and 1.4, at 0.012 bits 1.7 and 1.5 (left whole).
+// kSegMin rounds) take as long as the chain itself.  Measured (the call, whole
+// and split, ms; * what the rule takes):
+//                      256 x 256 KiB  96 x 128 KiB  64 x 1 MiB   256 x 1 MiB
+//   Zipf               2.01  1.72*    1.03  0.75*   7.66  1.64*  7.62   4.52*
+//   one symbol 90 %    1.93* 2.81     0.99  1.11*   7.07  3.05*  7.37   6.40*
+//   95 %               1.93* 3.44     0.98* 1.37    7.05  3.97*  7.35*  9.08
+//   97 %               1.92* 3.84     0.98* 1.40    7.04  5.11*  7.33* 11.55
+//   two, 50 % each     1.91* 4.34     0.97* 1.54    7.04  6.62*  7.29* 11.39
+//   16 equally likely  1.95* 2.97     1.00  1.11*   7.14  4.16*  7.47*  8.07
+PZ_HD inline uint64_t min64(uint64_t a, uint64_t b) { return a < b ? a : b; }
 constexpr uint32_t kCutMin = 2 * (kWarm + kSegMin);
 PZ_HD constexpr uint32_t seg_cut(int i) { return ((i & 1) ? 3 * kCutMin / 2 : kCutMin) << (i >> 1); }
 PZ_HD inline int seg_cut_below(uint32_t rounds) {  // the highest cut below it, -1: none
@@ -68,13 +94,13 @@ PZ_HD inline int seg_cut_below(uint32_t rounds) {  // the highest cut below it, 
     return i;
 }
 PZ_HD inline uint64_t cut_cost(uint64_t longest_whole, uint64_t walk_rounds, uint64_t apart_rounds, uint32_t weight) {
-    const uint64_t apart = 540 * apart_rounds, counted = 520 * kCutMin;
-    return 520 * longest_whole +
-           (walk_rounds ? weight * walk_rounds + (apart > counted ? apart - counted : 0) + 4200000 : 0);
+    if (!walk_rounds) return 520 * longest_whole;
+    const uint64_t apart = 540 * apart_rounds + min64(6 * walk_rounds / 5, 4000000), counted = 520 * kCutMin;
+    return 520 * longest_whole + weight * walk_rounds + walk_rounds / 6 + (apart > counted ? apart - counted : 0) + 4200000;
 }
 // A task's rounds as its walk costs them, and those that stay apart.
-PZ_HD inline uint64_t seg_walk_rounds(uint32_t rounds, uint32_t apart) { return rounds + (uint64_t)rounds * apart * 3 / 512; }
-PZ_HD inline uint32_t seg_apart_rounds(uint32_t rounds, uint32_t apart) { return (uint32_t)((uint64_t)rounds * apart / 256); }
+PZ_HD inline uint64_t seg_walk_rounds(uint32_t rounds, uint32_t apart) { return rounds + (uint64_t)rounds * (apart >> 16) / 256; }
+PZ_HD inline uint32_t seg_apart_rounds(uint32_t rounds, uint32_t apart) { return (uint32_t)((uint64_t)rounds * (apart & 0xFFFFu) / 256); }
 // walk[i]: the sum of seg_walk_rounds of the tasks whose highest cut below is
 // i; apart[i]: the most seg_apart_rounds of one; longest: the most rounds of
 // one task.  0xFFFFFFFF: nothing is split.
