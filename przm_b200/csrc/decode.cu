@@ -734,30 +734,37 @@ __device__ __forceinline__ void dec_adaptive_body(Dec1Shared& S, const DecTask& 
     if (!ok) dec_fail(infos, t.frame, D_CORRUPT);
 }
 
-// The bodies of the task slots (list null: block b has slot b, for calls that
-// need no order) or of the list.  kLoop:
-// calls with more slots than blocks fit the SMs at once; a block that is done
-// takes the list's next body.  A block a slot would mostly be blocks without a
-// body: 20 000 frames of 200 bytes, which have none, took 84 us so, 3.5 with
-// the blocks that fit.
+// The bodies, a block each: of the task slots (kSlots, calls that need no
+// order), or of the list (kListed).  kResident: calls with more slots than
+// blocks fit the SMs at once; a block that is done takes the list's next body.
+// A block a slot would mostly be blocks without a body: 20 000 frames of 200
+// bytes, which have none, took 84 us so, 3.5 with the blocks that fit.  One
+// kernel for each, and the slot's kind and length read for the test alone:
+// with the ways in joined, or the test on t, the rounds came out 2.2 % longer
+// (one frame of 300 001 bytes 4027 us, 3941 so).
+enum { kSlots, kListed, kResident };
 constexpr uint32_t kDecResident = 11;  // blocks an SM, by their shared memory
-template <bool kLoop>
-__global__ void __launch_bounds__(32) k_dec_adaptive(const DecTask* __restrict__ tasks, uint32_t* list,
+template <int kWay>
+__global__ void __launch_bounds__(32) k_dec_adaptive(const DecTask* __restrict__ tasks, uint32_t* __restrict__ list,
                                                       DecInfo* __restrict__ infos) {
     __shared__ __align__(16) Dec1Shared S;
-    if (!list) {
+    if (kWay == kSlots) {
+        if (__ldcg(&tasks[blockIdx.x].kind) != DT_ADAPTIVE || __ldcg(&tasks[blockIdx.x].n) == 0) return;
         const DecTask t = tasks[blockIdx.x];
-        if (t.kind == DT_ADAPTIVE && t.n) dec_adaptive_body(S, t, infos);
-        return;
-    }
-    const uint32_t count = list[0];
-    for (uint32_t b = blockIdx.x; b < count;) {
-        const DecTask t = tasks[list[4 + b]];
         dec_adaptive_body(S, t, infos);
-        if (!kLoop) return;
-        __syncwarp();
-        if (threadIdx.x == 0) b = gridDim.x + atomicAdd(&list[1], 1u);
-        b = __shfl_sync(0xFFFFFFFFu, b, 0);
+    } else if (kWay == kListed) {
+        if (blockIdx.x >= list[0]) return;
+        const DecTask t = tasks[list[4 + blockIdx.x]];
+        dec_adaptive_body(S, t, infos);
+    } else {
+        const uint32_t count = list[0];
+        for (uint32_t b = blockIdx.x; b < count;) {
+            const DecTask t = tasks[list[4 + b]];
+            dec_adaptive_body(S, t, infos);
+            __syncwarp();
+            if (threadIdx.x == 0) b = gridDim.x + atomicAdd(&list[1], 1u);
+            b = __shfl_sync(0xFFFFFFFFu, b, 0);
+        }
     }
 }
 

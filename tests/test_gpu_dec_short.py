@@ -118,3 +118,16 @@ def test_frames_of_byte_runs_are_walked(comp, profile):
     ln = [len(f) for f in frames]
     ks = kernels(lambda: comp.DecompressBatchDevice(d_src.ptr, so[:-1], ln, d_dst.ptr, do[:-1], caps))
     assert total(ks, "k_dec_exec<") < 2 * total(ks, "k_dec_static"), ks
+
+
+@pytest.mark.parametrize("count,way", [(1, 0), (18, 0), (19, 1), (407, 1), (408, 2), (900, 2)])
+def test_ways_to_the_adaptive_bodies(comp, count, way):
+    # a block per slot up to one an SM, then in the list's order, then blocks that stay (148 SMs, eight slots a frame)
+    xs = [W.gen("markov", i, 5000 + 13 * i) for i in range(20)]
+    fr = [comp.Compress(x, 1)[0] for x in xs]
+    pick = [i % 20 for i in range(count)]
+    frames, caps = [fr[i] for i in pick], [len(xs[i]) for i in pick]
+    st, outs = decode(comp, frames, caps)
+    assert st == [0] * count and [o == xs[i].tobytes() for o, i in zip(outs, pick)] == [True] * count
+    ks = [n for n, _ in kernels(lambda: decode(comp, frames, caps))]
+    assert f"k_dec_adaptive<{way}>" in ks, ks
