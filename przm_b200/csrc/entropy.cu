@@ -796,11 +796,11 @@ __device__ void build_task_list(uint32_t total, Get get, const TableInfo* __rest
     __shared__ uint32_t s_cnt[2][33];
     __shared__ uint32_t s_pos[2][33];
     __shared__ uint32_t s_segs[kSegSizes], s_apart[kSegSizes];
-    __shared__ unsigned long long s_rounds[kSegSizes];
+    __shared__ unsigned long long s_walk[kSegSizes];
     __shared__ uint32_t s_len, s_nseg, s_nsplit, s_longest, s_cut;
     const uint32_t tid = threadIdx.x;
     if (tid < 66) (&s_cnt[0][0])[tid] = 0;
-    if (tid < kSegSizes) { s_segs[tid] = s_apart[tid] = 0; s_rounds[tid] = 0; }
+    if (tid < kSegSizes) { s_segs[tid] = s_apart[tid] = 0; s_walk[tid] = 0; }
     if (tid == 0) s_len = s_nseg = s_nsplit = s_longest = 0;
     __syncthreads();
     if (sb.cap) {
@@ -811,13 +811,13 @@ __device__ void build_task_list(uint32_t total, Get get, const TableInfo* __rest
             const int i = seg_cut_below(rounds);
             if (i >= 0) {
                 const uint32_t apart = d.m8 ? 0u : infos[d.tab].apart;  // (Meta8 models have no symbol so frequent)
-                atomicAdd(&s_rounds[i], (unsigned long long)seg_walk_rounds(rounds, apart));
+                atomicAdd(&s_walk[i], (unsigned long long)seg_walk_cost(rounds, apart, sb.weight));
                 atomicMax(&s_apart[i], seg_apart_rounds(rounds, apart));
             }
             atomicMax(&s_longest, rounds);
         }
         __syncthreads();
-        if (tid == 0) s_cut = best_cut(s_rounds, s_apart, s_longest, sb.weight);
+        if (tid == 0) s_cut = best_cut(s_walk, s_apart, s_longest);
         __syncthreads();
         for (uint32_t e = tid; e < total && s_cut != 0xFFFFFFFFu; e += blockDim.x) {
             TaskDesc d;

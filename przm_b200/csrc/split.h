@@ -49,10 +49,10 @@ PZ_HD inline uint32_t seg_count(uint32_t n, uint32_t len, uint32_t cut) {
 PZ_HD inline uint32_t seg_apart(uint32_t most, uint32_t symbols, uint32_t off_powers) {
     if (symbols < 2) return 0;
     const float root = sqrtf((float)(4096 - (int)most > 0 ? 4096 - most : 0) / 4096.0f);
-    float share = fmaxf(1.02f - 3.8f * root, 0.0f), slow = fminf(fmaxf(1.25f - 2.0f * root, 0.0f), 0.85f);
+    float share = fmaxf(1.02f - 3.8f * root, 0.0f), slow = fminf(fmaxf(1.35f - 2.0f * root, 0.0f), 0.9f);
     if (off_powers < kOffPowers) {
         const float kept = 0.67f - 0.67f / kOffPowers * (float)off_powers;
-        slow = fmaxf(slow, fminf(4.0f * kept, 0.85f));
+        slow = fmaxf(slow, fminf(4.0f * kept, 0.9f));
         if (off_powers) share = fmaxf(share, kept);
     }
     return (uint32_t)(256.0f * share) | (uint32_t)(256.0f * slow) << 16;
@@ -70,10 +70,11 @@ PZ_HD inline uint32_t seg_off_power(uint32_t f) {
 
 // The cut of a call: tasks of more rounds are split.  The longest task left
 // whole takes 26 ns a round; walking the split ones takes the whole GPU 0.05
-// ns a round, up to 1.85 times that where walkers stay many (weight times:
-// 1 where the call waits for its result, 3 where other batches in flight would
-// use the GPU meanwhile: with ten in flight 256 frames of 1 MiB take 3.1 ms a
-// step whole and 4.2 ms split, with three in flight 64 frames 3.3 and 1.7), and
+// ns a round (weight times: 1 where the call waits for its result, 3 where
+// other batches in flight would use the GPU meanwhile: with ten in flight 256
+// frames of 1 MiB take 3.1 ms a step whole and 4.2 ms split, with three in flight
+// 64 frames 3.3 and 1.7; 64 frames of hexadecimal digits alone 7.5 and 4.2), up to
+// 0.045 more where walkers stay many, and
 // coding them 0.006; the rounds that stay apart are walked again one after another,
 // 27 ns each, task by task side by side, 0.2 ms more where there are many; and 0.2
 // ms pass before a segment can be coded.  The lowest cut counts as a chain of
@@ -97,24 +98,26 @@ PZ_HD inline int seg_cut_below(uint32_t rounds) {  // the highest cut below it, 
     while (i + 1 < kSegSizes && rounds > seg_cut(i + 1)) i++;
     return i;
 }
-PZ_HD inline uint64_t cut_cost(uint64_t longest_whole, uint64_t walk_rounds, uint64_t apart_rounds, uint32_t weight) {
-    if (!walk_rounds) return 520 * longest_whole;
-    const uint64_t apart = 540 * apart_rounds + min64(walk_rounds + walk_rounds / 4, 4000000), counted = 520 * kCutMin;
-    return 520 * longest_whole + weight * walk_rounds + walk_rounds / 8 + (apart > counted ? apart - counted : 0) + 4200000;
+PZ_HD inline uint64_t cut_cost(uint64_t longest_whole, uint64_t walk, uint64_t apart_rounds) {
+    if (!walk) return 520 * longest_whole;
+    const uint64_t apart = 540 * apart_rounds + min64(walk + walk / 4, 4000000), counted = 520 * kCutMin;
+    return 520 * longest_whole + walk + (apart > counted ? apart - counted : 0) + 4200000;
 }
-// A task's rounds as its walk costs them, and those that stay apart.
-PZ_HD inline uint64_t seg_walk_rounds(uint32_t rounds, uint32_t apart) { return rounds + (uint64_t)rounds * (apart >> 16) / 256; }
+// What a task's rounds cost walked and coded, and those of them that stay apart.
+PZ_HD inline uint64_t seg_walk_cost(uint32_t rounds, uint32_t apart, uint32_t weight) {
+    return (uint64_t)rounds * (256 * weight + (apart >> 16) + 32) / 256;
+}
 PZ_HD inline uint32_t seg_apart_rounds(uint32_t rounds, uint32_t apart) { return (uint32_t)((uint64_t)rounds * (apart & 0xFFFFu) / 256); }
-// walk[i]: the sum of seg_walk_rounds of the tasks whose highest cut below is
+// walk[i]: the sum of seg_walk_cost of the tasks whose highest cut below is
 // i; apart[i]: the most seg_apart_rounds of one; longest: the most rounds of
 // one task.  0xFFFFFFFF: nothing is split.
-PZ_HD inline uint32_t best_cut(const unsigned long long* walk, const uint32_t* apart, uint32_t longest, uint32_t weight) {
-    uint64_t best = cut_cost(longest, 0, 0, weight), above = 0;
+PZ_HD inline uint32_t best_cut(const unsigned long long* walk, const uint32_t* apart, uint32_t longest) {
+    uint64_t best = cut_cost(longest, 0, 0), above = 0;
     uint32_t cut = 0xFFFFFFFFu, most = 0;
     for (int i = kSegSizes - 1; i >= 0; i--) {
         above += walk[i];
         most = apart[i] > most ? apart[i] : most;
-        const uint64_t cost = cut_cost(seg_cut(i), above, most, weight);
+        const uint64_t cost = cut_cost(seg_cut(i), above, most);
         if (above && cost < best) {
             best = cost;
             cut = seg_cut(i);

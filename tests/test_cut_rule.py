@@ -27,11 +27,11 @@ extern "C" uint32_t cut(const uint32_t* rounds, const uint32_t* apart, uint32_t 
         const int i = pz::seg_cut_below(rounds[k]);
         longest = rounds[k] > longest ? rounds[k] : longest;
         if (i < 0) continue;
-        walk[i] += pz::seg_walk_rounds(rounds[k], apart[k]);
+        walk[i] += pz::seg_walk_cost(rounds[k], apart[k], weight);
         const uint32_t a = pz::seg_apart_rounds(rounds[k], apart[k]);
         most[i] = a > most[i] ? a : most[i];
     }
-    return pz::best_cut(walk, most, longest, weight);
+    return pz::best_cut(walk, most, longest);
 }
 """
 WHOLE = 0xFFFFFFFF
@@ -81,6 +81,8 @@ def test_models_of_a_bit_and_more_are_not_held_back(rule):
     # 64 streams of 1 MiB, by the probability of their first symbol: whole from where segments take longer
     ([(M, 0.95)] * 64, 1, True), ([(M, 0.99)] * 64, 1, True), ([(M, 0.995)] * 64, 1, False), ([(M, 0.999)] * 64, 1, False),
     ([(M, 0.9999)] * 64, 1, False), ([(M, 0.99)] * 64, 3, False),
+    # 64 frames of hexadecimal digits, other batches beside them
+    ([(M, "hex")] * 64, 3, True),
     # one stream of 4 MiB
     ([(4 * M, 0.99)], 1, True), ([(4 * M, 0.999)], 1, True), ([(4 * M, 0.9999)], 1, False),
     # one stream of 256 KiB
@@ -89,7 +91,7 @@ def test_models_of_a_bit_and_more_are_not_held_back(rule):
     ([(4 * M, 0)] + [(20_000, 0.999)] * 200, 1, True),
 ])
 def test_what_is_split(rule, tasks, weight, split):
-    t = [(r, apart(rule, one(p)) if p else 0) for r, p in tasks]
+    t = [(r, apart(rule, near(16, 2) if p == "hex" else one(p)) if p else 0) for r, p in tasks]
     c = cut(rule, t, weight)
     assert (c != WHOLE) == split
     if split and len(set(t)) > 1:
@@ -112,6 +114,7 @@ TEXT = [205] * 16 + [51] * 16
     (256, M // 4, one(0.97, 15), False), (96, M // 8, one(0.97, 15), False), (64, M, one(0.97, 15), True), (256, M, one(0.97, 15), False),
     (256, M // 4, near(2), False), (96, M // 8, near(2), False), (64, M, near(2), True), (256, M, near(2), False),
     (256, M // 4, near(16), False), (64, M, near(16), True), (256, M, near(16), False),
+    (64, M, near(16, 2), True),
     # exact powers of two: few walkers meet, none is missed
     (256, M // 4, [2048] * 2, False), (200, M, [2048] * 2, True), (1, 4 * M, [2048] * 2, True),
 ])
