@@ -17,7 +17,7 @@
 // (0x80-0xBF), long repeat (0xC0-0xC3), literal runs (0xF0, 0xF3-0xFA), byte
 // runs (0xF1).  A frame that reaches another known opcode is left to
 // k_dec_exec_warp, and so are short frames (exec_short_cap), those of byte runs
-// alone and, in calls of many frames, those of flat command streams.
+// alone and, in calls of many frames, those of few commands (exec_walked).
 //
 // Measured on 128 mixed frames of 1 MiB: 26.0 ms with one warp walking each
 // frame, 1.25 ms so.  A chunk's 16 000 cycles (of 34 000 with its copies, on the
@@ -331,15 +331,32 @@ __device__ void exec_copy(ExecShared<NT>& S, uint8_t* dst, const uint8_t* __rest
 // 3000 of 2000 bytes 72-107, 190-309; 12000 of 200 bytes 10, 300.
 inline uint32_t exec_short_cap(uint32_t nf, uint32_t sms) { return nf <= 2 * sms ? 768u : nf <= 8 * sms ? 1536u : 2304u; }
 
-// flat_to_warps (calls of more than 8 frames an SM): frames of flat streams of
-// short commands are left to k_dec_exec_warp, because one thread finds a
-// chunk's commands here, and two blocks an SM hide less of that than 28 walks
-// (3000 frames of 4000 bytes: 142-254 us walked, 414-604 so; 600 frames: alike
-// or slower).
+// Whether a frame of u bytes is walked sooner than its block comes to it and is
+// done, in a call of turns / 16 frames for every block that the SMs take at
+// once (ns).  Walked: a byte of a flat command stream 170, an opcode of a split
+// one 350, an output byte 3.3 where matches repeat a few bytes, all longer when
+// more than 28 frames an SM want a warp.  In a block: a chunk 11000, one
+// thread's search of a flat stream 60 a byte, an output byte 0.45.  Of split
+// streams only those well below, as opcodes differ most in them, and so in calls
+// of up to 8 frames an SM, where the walk of some after the blocks of others
+// costs most (records, 600 of 3000: 93 in blocks, 131 half walked).  Measured (us,
+// all walked and all in blocks; those left to the walk take 4 ns a frame more):
+// flat streams of few commands, 3000 frames of 3000 bytes 16 and 123, 1300 of
+// 12 000 45 and 125, 600 of 2400 11 and 32; records, 3000 of 2400 82 and 190;
+// hexadecimal digits (split), 3000 of 3000 80 and 108, 1300 of 3000 71 and 50
+// (block); 37 bytes over and over, 200 of 262 144 862 and 126 (block).
+__device__ __forceinline__ bool exec_walked(bool split, uint32_t cl, uint32_t ops, uint32_t u, uint32_t turns) {
+    if (turns <= 16) return false;  // (8 us less at best)
+    uint64_t walk = (split ? 455ull * ops : 170ull * cl) + (split ? 43ull : 33ull) * u / 10;
+    walk += walk * (turns / (14 * 16));
+    if (turns <= 64) walk += 3 * walk / 4;
+    return 16 * walk < turns * (11000 + (split ? 0ull : 60ull * cl) + 9ull * u / 20);
+}
+
 template <uint32_t NT>
 __global__ void __launch_bounds__(NT, 1024 / NT) k_dec_exec(const uint8_t* __restrict__ src, const DecJob* __restrict__ jobs,
                                                          DecInfo* __restrict__ infos, uint8_t* __restrict__ out,
-                                                         bool flat_to_warps) {
+                                                         uint32_t turns) {
     extern __shared__ __align__(16) uint8_t smem_x[];
     ExecShared<NT>& S = *reinterpret_cast<ExecShared<NT>*>(smem_x);
     const uint32_t f = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -360,13 +377,13 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_dec_exec(const uint8_t* __res
     const uint8_t* offs = reinterpret_cast<const uint8_t*>(I.off);
     const uint32_t cl = I.cmd_len, ml = I.meta_len, vl = I.var_len, ll = I.lit_len, ol = I.off_len, bmin = I.bmin;
     const bool split = I.cmd_mode == 1;
-    // flat_to_warps, and frames that are a few byte runs (they begin with one,
-    // and no match has a distance): a chunk and its tiles cost them 9 us and
-    // 1.2 to 2.4 us per 4 KiB, a warp 1.1 us per 4 KiB (300 frames of 65 536
-    // zeros 49.7 us in tiles, 19.6 walked; one of 200 000 alike)
+    // and frames that are a few byte runs (they begin with one, and no match has
+    // a distance): a chunk and its tiles cost them 9 us and 1.2 to 2.4 us per
+    // 4 KiB, a warp 1.1 us per 4 KiB (300 frames of 65 536 zeros 49.7 us in
+    // tiles, 19.6 walked; one of 200 000 alike)
     const bool runs = cl - 2 < 31 && ol == 0 && u <= 131072u &&
                       (cs[0] == 0xF1u || (cs[0] >= 0xF3u && cs[0] <= 0xFAu && cs[1] == 0xF1u));
-    if (!split && (runs || (flat_to_warps && u / 64 <= cl))) {
+    if ((!split && runs) || exec_walked(split, cl, I.cmd_orig, u, turns)) {
         if (tid == 0) infos[f].serial = 1;
         return;
     }

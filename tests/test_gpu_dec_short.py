@@ -131,3 +131,27 @@ def test_ways_to_the_adaptive_bodies(comp, count, way):
     assert st == [0] * count and [o == xs[i].tobytes() for o, i in zip(outs, pick)] == [True] * count
     ks = [n for n, _ in kernels(lambda: decode(comp, frames, caps))]
     assert f"k_dec_adaptive<{way}>" in ks, ks
+
+
+@pytest.mark.parametrize("profile", [0, 1])
+@pytest.mark.parametrize("count,n", [(297, 2400), (600, 6000), (1300, 12_000), (1300, 3000), (4400, 2400)])
+def test_frames_of_few_commands_in_calls_of_many(comp, profile, count, n):
+    # some walked, some by blocks in the same call: rare ones among zeros, a short period, digits, records, text
+    rng = np.random.default_rng(n)
+    xs = []
+    for i in range(5):
+        m = n - 7 * i
+        xs += [(rng.random(m) < 0.003).astype(np.uint8), np.resize(rng.integers(0, 256, 37).astype(np.uint8), m),
+               np.frombuffer(b"0123456789abcdef", np.uint8)[rng.integers(0, 16, m)], W.gen("records", i, m), W.gen("markov", i, m)]
+    fr = [comp.Compress(x, profile)[0] for x in xs]
+    pick = [i % len(xs) for i in range(count)]
+    st, outs = decode(comp, [fr[i] for i in pick], [len(xs[i]) for i in pick])
+    assert st == [0] * count and [o == xs[i].tobytes() for o, i in zip(outs, pick)] == [True] * count
+
+
+def test_rare_ones_are_walked(comp):
+    # 3000 frames of 3000 bytes, each a few matches: 123 us in blocks, 16 walked and 12 for the blocks that leave them
+    x = (np.random.default_rng(1).random(3000) < 0.003).astype(np.uint8)
+    fr = comp.Compress(x, 1)[0]
+    ks = kernels(lambda: decode(comp, [fr] * 3000, [3000] * 3000))
+    assert total(ks, "k_dec_exec") < 3 * total(ks, "k_dec_static"), ks  # (which only finds that there is nothing for it: 19 us)
